@@ -308,7 +308,14 @@ __device__ __forceinline__ double to_unit<double>(uint32_t i) {
 // multiply-add from b in float (b's conversion rounds as v's does, the sum once: within 3.9e-7 of the exact angle,
 // as 2 pi (v - 1/2) computed in steps is).
 __device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, float& z0, float& z1) {
-    const float r = sqrtf(-2.0f * logf(to_unit<float>(a)));
+    // u lies in [2^-33, 1]: told so, the compiler leaves out the logarithm's cases for zero, denormals, infinities and
+    // NaN (22 -> 15 instructions a logarithm, counted over the Phoenix's step loop; the value is logf's)
+    const float u = to_unit<float>(a);
+    __builtin_assume(__float_as_int(u) >= 0x2E800000 && __float_as_int(u) <= 0x3F800000);
+    __builtin_assume(u >= 1.1e-10f);
+    __builtin_assume(u <= 1.0f);
+    __builtin_assume(u != 0.0f);
+    const float r = sqrtf(-2.0f * logf(u));
     float s, c;
     // 2 pi 2^-32 and pi 2^-32 - pi, rounded to float
     __sincosf(fmaf(static_cast<float>(b), 1.46291807926715968e-09f, -3.14159265285070240f), &s, &c);

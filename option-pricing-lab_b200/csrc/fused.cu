@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
     const R* s_root = reinterpret_cast<const R*>(sm + a.off.root);
     const R* s_hes = reinterpret_cast<const R*>(sm + a.off.hes);
     const Pair2<R>* s_tab = GT ? a.tab : reinterpret_cast<const Pair2<R>*>(sm + a.off.table2);
+    const uint32_t tab_s = shared_address<GT || !TABLE>(s_tab);
     const R* s_trig = reinterpret_cast<const R*>(sm + a.off.ln_trig);
     const double* s_disc = reinterpret_cast<const double*>(sm + a.off.obs_disc);
     const int S = a.n_steps;
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
             constexpr bool CHECK = decltype(check)::value, OBS = decltype(observe)::value;
             R z[C * G];
             R za[CA > 0 ? CA * G : 1];
+            R q0 = R(0), q1 = R(0);
 #pragma unroll
             for (int k = 0; k < NB; ++k)
                 normals4<R>(pair, static_cast<uint64_t>(batch) * NB + k, 0u, k0, k1, z[4 * k], z[4 * k + 1],
@@ -240,12 +242,8 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
                         R var0, var1, vp0 = R(0), vp1 = R(0);
                         if (VAR) vp0 = m_max(v0[n], R(0)), vp1 = m_max(v1[n], R(0));
                         if (TABLE) {
-                            int j0, j1;
-                            R f0, f1;
-                            table_cell(ns, a.top, x0[n], j0, f0), table_cell(ns, a.top, x1[n], j1, f1);
-                            const Pair2<R> y0 = GT ? ldg_pair(s_tab + ns.row + j0) : s_tab[ns.row + j0];
-                            const Pair2<R> y1 = GT ? ldg_pair(s_tab + ns.row + j1) : s_tab[ns.row + j1];
-                            const R t0 = y0.a + f0 * y0.b, t1 = y1.a + f1 * y1.b;
+                            R t0, t1;
+                            table_vars<GT>(s_tab, tab_s, ns.org, ns.inv_dx, ns.row, a.top, x0[n], x1[n], t0, t1);
                             var0 = KIND == 1 ? t0 : t0 * vp0, var1 = KIND == 1 ? t1 : t1 * vp1;
                         } else if (VAR) {
                             var0 = vp0, var1 = vp1;
@@ -263,8 +261,7 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
                             x1[n] = lv_advance(x1[n], var1, st.hdt, st.sdt * zm1[n]);
                         } else {
                             const R zd = st.sdt * zc[n];  // sqrt(dt) z, the legs' +-
-                            x0[n] = lv_advance(x0[n], var0, st.hdt, zd);
-                            x1[n] = lv_advance(x1[n], var1, st.hdt, -zd);
+                            lv_advance_legs(x0[n], x1[n], var0, var1, st.hdt, zd);
                         }
                         if (n == 0) w0 = x0[n] + ns.lf, w1 = x1[n] + ns.lf;
                         else w0 = m_min(w0, x0[n] + ns.lf), w1 = m_min(w1, x1[n] + ns.lf);
@@ -272,10 +269,13 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
                     lp0 = w0, lp1 = w1;
                 }
                 if (PRODUCT == OB_PRODUCT_LADDER) {
-                    l0.hi = m_max(l0.hi, lp0), l0.lo = m_min(l0.lo, lp0);
-                    l1.hi = m_max(l1.hi, lp1), l1.lo = m_min(l1.lo, lp1);
+                    l0.hi = run_max(l0.hi, lp0), l0.lo = run_min(l0.lo, lp0);
+                    l1.hi = run_max(l1.hi, lp1), l1.lo = run_min(l1.lo, lp1);
+                } else if (!OBS && G % 2 == 0) {  // no one reads the low within the batch: two steps at a time
+                    if (g % 2) l0.lo = run_min(l0.lo, q0, lp0), l1.lo = run_min(l1.lo, q1, lp1);
+                    else q0 = lp0, q1 = lp1;
                 } else {
-                    l0.lo = m_min(l0.lo, lp0), l1.lo = m_min(l1.lo, lp1);
+                    l0.lo = run_min(l0.lo, lp0), l1.lo = run_min(l1.lo, lp1);
                     const int j = OBS ? s_step[i - 1].obs : -1;
                     if (j >= 0) {
                         leg_observe(a, s_trig, s_disc, l0, lp0, j);

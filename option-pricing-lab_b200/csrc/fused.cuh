@@ -92,6 +92,60 @@ __device__ __forceinline__ double lv_advance(double x, double var, double hdt, d
     return x + fma(sqrt(var), zd, var * hdt);
 }
 
+// Two floats as one 64-bit register pair, for Blackwell's packed single-precision instructions: one issue slot for two
+// multiply-adds, each rounded (and flushed) as the scalar instruction's, so packed and scalar code agree bit for bit.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2_rz(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rz.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// lv_advance of both legs of a pair on the antithetic normal: x0 on sqrt(dt) z, x1 on its negative.
+__device__ __forceinline__ void lv_advance_legs(float& x0, float& x1, float var0, float var1, float hdt, float zd) {
+    const f32x2 drifted = fma2(pack2(var0, var1), pack2(hdt, hdt), pack2(x0, x1));
+    unpack2(fma2(pack2(sqrtf(var0), sqrtf(var1)), pack2(zd, -zd), drifted), x0, x1);
+}
+__device__ __forceinline__ void lv_advance_legs(double& x0, double& x1, double var0, double var1, double hdt,
+                                                double zd) {
+    x0 = lv_advance(x0, var0, hdt, zd), x1 = lv_advance(x1, var1, hdt, -zd);
+}
+
+// The running extremes of a path: m_min(a, b) and m_max(a, b) in one instruction each. A NaN in b gives NaN, as there;
+// a is NaN only once an earlier b was, and a log performance that is NaN once stays NaN.
+__device__ __forceinline__ float run_min(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float run_max(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// run_min over two values in order, one three-input instruction.
+__device__ __forceinline__ float run_min(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ double run_min(double a, double b) { return m_min(a, b); }
+__device__ __forceinline__ double run_max(double a, double b) { return m_max(a, b); }
+__device__ __forceinline__ double run_min(double a, double b, double c) { return m_min(m_min(a, b), c); }
+
 // One table interval: the value at its left point and the increment to the right one, so that an interpolation is
 // one multiply-add (y + w dy, the reference's y_i (1 - w) + y_i+1 w up to rounding).
 template <typename R>
@@ -108,6 +162,50 @@ __device__ __forceinline__ Pair2<float> ldg_pair(const Pair2<float>* p) {
 __device__ __forceinline__ Pair2<double> ldg_pair(const Pair2<double>* p) {
     const double2 v = __ldg(reinterpret_cast<const double2*>(p));
     return {v.x, v.y};
+}
+
+// The local variances of both legs of a pair at x0 and x1 in a step's row of the table: table_cell of each leg and one
+// load and multiply-add each. GLOBAL: tab is in global memory (ldg_pair); else in shared memory, tab_s its shared
+// address. Float: the cell's last three operations packed, and the interval's address straight from the bits of
+// s top + 2^23, one shift-and-add with the offset 2^23's own bits leave (0x4B000000, times 8 modulo 2^32) folded into
+// the row's address. (The shared load has no memory clobber: its address depends on the row read after the barrier
+// that follows the staging, and nothing writes the table after it.)
+template <bool GLOBAL>
+__device__ __forceinline__ void table_vars(const Pair2<float>* tab, uint32_t tab_s, float org, float inv, int row,
+                                           float top, float x0, float x1, float& var0, float& var1) {
+    float s0, s1, b0, b1, f0, f1;
+    asm("fma.rn.ftz.sat.f32 %0, %1, %2, %3;" : "=f"(s0) : "f"(x0), "f"(inv), "f"(org));
+    asm("fma.rn.ftz.sat.f32 %0, %1, %2, %3;" : "=f"(s1) : "f"(x1), "f"(inv), "f"(org));
+    const f32x2 s = pack2(s0, s1), t = pack2(top, top), two23 = pack2(8388608.0f, 8388608.0f);
+    const f32x2 big = fma2_rz(s, t, two23);
+    unpack2(big, b0, b1);
+    unpack2(fma2(s, t, fma2(big, pack2(-1.0f, -1.0f), two23)), f0, f1);  // (2^23 - big is exact)
+    const uint32_t i0 = __float_as_uint(b0), i1 = __float_as_uint(b1);
+    Pair2<float> y0, y1;
+    if (GLOBAL) {
+        y0 = ldg_pair(tab + row + static_cast<int>(i0 - 0x4B000000u));
+        y1 = ldg_pair(tab + row + static_cast<int>(i1 - 0x4B000000u));
+    } else {
+        const uint32_t base = tab_s + 8u * static_cast<uint32_t>(row) - 8u * 0x4B000000u;
+        asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(y0.a), "=f"(y0.b) : "r"(i0 * 8u + base));
+        asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(y1.a), "=f"(y1.b) : "r"(i1 * 8u + base));
+    }
+    var0 = fmaf(f0, y0.b, y0.a), var1 = fmaf(f1, y1.b, y1.a);
+}
+template <bool GLOBAL>
+__device__ __forceinline__ void table_vars(const Pair2<double>* tab, uint32_t, double org, double inv, int row,
+                                           double top, double x0, double x1, double& var0, double& var1) {
+    int j0, j1;
+    double f0, f1;
+    table_cell(org, inv, top, x0, j0, f0), table_cell(org, inv, top, x1, j1, f1);
+    const Pair2<double> y0 = GLOBAL ? ldg_pair(tab + row + j0) : tab[row + j0];
+    const Pair2<double> y1 = GLOBAL ? ldg_pair(tab + row + j1) : tab[row + j1];
+    var0 = y0.a + f0 * y0.b, var1 = y1.a + f1 * y1.b;
+}
+// The shared-memory address of p (0 where the table is left in global memory).
+template <bool GLOBAL>
+__device__ __forceinline__ uint32_t shared_address(const void* p) {
+    return GLOBAL ? 0u : static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
 // A record of whole 16-byte words (StepRec, NameStep) read from global memory through the read-only data cache: the

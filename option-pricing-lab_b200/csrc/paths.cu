@@ -184,6 +184,7 @@ __global__ void __launch_bounds__(lv_block<N>(), N == 1 && sizeof(R) == 4 ? 2 : 
     // per name: v0, kappa, theta, xi, rho, sqrt(1 - rho^2), the constant variance (Black-Scholes)
     const R* s_hes = reinterpret_cast<const R*>(sm + a.off.hes);
     const Pair2<R>* tab = GT ? a.tab : reinterpret_cast<const Pair2<R>*>(sm + a.off.table2);
+    const uint32_t tab_s = shared_address<GT || !TABLE>(tab);
     const int2* s_sched = reinterpret_cast<const int2*>(sm + a.off.sched);  // observations [x, y) at each step end
     const int* s_col = reinterpret_cast<const int*>(sm + a.off.col);
     const R* s_fwd = reinterpret_cast<const R*>(sm + a.off.fwd);
@@ -274,12 +275,8 @@ __global__ void __launch_bounds__(lv_block<N>(), N == 1 && sizeof(R) == 4 ? 2 : 
                     R var0, var1, vp0 = R(0), vp1 = R(0);
                     if (VAR) vp0 = m_max(v0[n], R(0)), vp1 = m_max(v1[n], R(0));
                     if (TABLE) {
-                        int j0, j1;
-                        R f0, f1;
-                        table_cell(ns, a.top, x0[n], j0, f0), table_cell(ns, a.top, x1[n], j1, f1);
-                        const Pair2<R> y0 = GT ? ldg_pair(tab + ns.row + j0) : tab[ns.row + j0];
-                        const Pair2<R> y1 = GT ? ldg_pair(tab + ns.row + j1) : tab[ns.row + j1];
-                        const R t0 = y0.a + f0 * y0.b, t1 = y1.a + f1 * y1.b;
+                        R t0, t1;
+                        table_vars<GT>(tab, tab_s, ns.org, ns.inv_dx, ns.row, a.top, x0[n], x1[n], t0, t1);
                         var0 = KIND == 1 ? t0 : t0 * vp0, var1 = KIND == 1 ? t1 : t1 * vp1;
                     } else if (VAR) {
                         var0 = vp0, var1 = vp1;
@@ -297,8 +294,7 @@ __global__ void __launch_bounds__(lv_block<N>(), N == 1 && sizeof(R) == 4 ? 2 : 
                         x1[n] = lv_advance(x1[n], var1, st.hdt, st.sdt * zm1[n]);
                     } else {
                         const R zd = st.sdt * zc;  // sqrt(dt) z, the legs' +-
-                        x0[n] = lv_advance(x0[n], var0, st.hdt, zd);
-                        x1[n] = lv_advance(x1[n], var1, st.hdt, -zd);
+                        lv_advance_legs(x0[n], x1[n], var0, var1, st.hdt, zd);
                     }
                 }
                 const int2 ob = s_sched[i];

@@ -287,7 +287,7 @@ __device__ __forceinline__ void fix_windows(const ScriptDev<R>& d, const WinMeta
     if constexpr (WF >= 0) {
         if (mask & 1u) {
             const R y = logp(meta.fn[0] >> 2);
-            win.v[0] = WF == 0 ? m_min(win.v[0], y) : m_max(win.v[0], y);
+            win.v[0] = WF == 0 ? run_min(win.v[0], y) : run_max(win.v[0], y);
         }
         return;
     }
@@ -477,6 +477,7 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
     const NameStep<R>* s_ns = reinterpret_cast<const NameStep<R>*>(sm + a.off.name_step);
     const R* s_root = reinterpret_cast<const R*>(sm + a.off.root);
     const Pair2<R>* s_tab = GT ? a.tab : reinterpret_cast<const Pair2<R>*>(sm + a.off.table2);
+    const uint32_t tab_s = shared_address<GT>(s_tab);
     const int2* s_sched = reinterpret_cast<const int2*>(sm + a.off.sched);  // (event, window mask) per step end
     const R* s_lf0 = reinterpret_cast<const R*>(sm + a.off.lf0);
     const int S = d.n_steps;
@@ -570,18 +571,19 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
 #pragma unroll
                 for (int n = 0; n < N; ++n) {
                     const NameStep<R> ns = s_ns[(i - 1) * N + n];
-                    int j0, j1;
-                    R f0, f1;
-                    table_cell(ns, a.top, x0[n], j0, f0), table_cell(ns, a.top, x1[n], j1, f1);
-                    const Pair2<R> p0 = GT ? ldg_pair(s_tab + ns.row + j0) : s_tab[ns.row + j0];
-                    const Pair2<R> p1 = GT ? ldg_pair(s_tab + ns.row + j1) : s_tab[ns.row + j1];
-                    const R v0 = p0.a + f0 * p0.b, v1 = p1.a + f1 * p1.b;
-                    // sqrt(dt) z with the legs' signs (+1, -1 but before a branch), the step's multiply-add written
+                    R v0, v1;
+                    table_vars<GT>(s_tab, tab_s, ns.org, ns.inv_dx, ns.row, a.top, x0[n], x1[n], v0, v1);
+                    // sqrt(dt) z with the legs' signs (+1, -1 but before a branch), the step's multiply-adds written
                     // out: the same arithmetic in every instantiation, so a branch at step 0 is an ordinary run bit
                     // for bit
-                    const R zd = st.sdt * zc[n], z0 = sg0 * zd, z1 = sg1 * zd;
-                    x0[n] = lv_advance(x0[n], v0, st.hdt, z0);
-                    x1[n] = lv_advance(x1[n], v1, st.hdt, z1);
+                    const R zd = st.sdt * zc[n];
+                    if constexpr (BRANCH) {
+                        const R z0 = sg0 * zd, z1 = sg1 * zd;
+                        x0[n] = lv_advance(x0[n], v0, st.hdt, z0);
+                        x1[n] = lv_advance(x1[n], v1, st.hdt, z1);
+                    } else {
+                        lv_advance_legs(x0[n], x1[n], v0, v1, st.hdt, zd);
+                    }
                     y0[n] = x0[n] + ns.lf, y1[n] = x1[n] + ns.lf;
                 }
                 observe(i, events);
