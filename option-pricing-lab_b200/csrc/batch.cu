@@ -184,11 +184,11 @@ __device__ __forceinline__ void rec_init(Rec<R, OB_PRODUCT_AUTOCALL>& r) {
 // Step end i of one leg, with lp the worst log performance and j the observation ending there (-1: none).
 template <typename R>
 __device__ __forceinline__ void rec_step(Rec<R, OB_PRODUCT_LADDER>& r, R lp, int j) {
-    r.last = lp, r.hi = m_max(r.hi, lp), r.lo = m_min(r.lo, lp);
+    r.last = lp, r.hi = run_max(r.hi, lp), r.lo = run_min(r.lo, lp);
 }
 template <typename R>
 __device__ __forceinline__ void rec_step(Rec<R, OB_PRODUCT_AUTOCALL>& r, R lp, int j) {
-    r.low = m_min(r.low, lp);
+    r.low = run_min(r.low, lp);
     if (j >= 0) r.obs[j] = lp;
 }
 
@@ -199,14 +199,14 @@ __device__ __forceinline__ void rec_carry(Rec<R, OB_PRODUCT_LADDER>& r, R lp, R 
     for (int c = 0; c < kBatchMaxCarry; ++c)
         if (c < nc) {
             const R l = lp + d.carry_dt[c] * fi;
-            r.hc[c] = m_max(r.hc[c], l), r.lc[c] = m_min(r.lc[c], l);
+            r.hc[c] = run_max(r.hc[c], l), r.lc[c] = run_min(r.lc[c], l);
         }
 }
 template <typename R>
 __device__ __forceinline__ void rec_carry(Rec<R, OB_PRODUCT_AUTOCALL>& r, R lp, R fi, const BDev<R>& d, int nc) {
 #pragma unroll
     for (int c = 0; c < kBatchMaxCarry; ++c)
-        if (c < nc) r.lowc[c] = m_min(r.lowc[c], lp + d.carry_dt[c] * fi);
+        if (c < nc) r.lowc[c] = run_min(r.lowc[c], lp + d.carry_dt[c] * fi);
 }
 
 template <typename R, int N, bool QE, int PRODUCT>
@@ -280,18 +280,10 @@ __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __res
                             const R org = d.row_org[row], inv = d.row_inv_dx[row];
                             const Pair2<R>* trow = tab + static_cast<long long>(row) * (d.n_x - 1);
                             const R zd = d.sdt * zc;  // sqrt(dt) z, the legs' +-
-#pragma unroll
-                            for (int leg = 0; leg < 2; ++leg) {
-                                R& x = leg ? x1[n] : x0[n];
-                                int j;
-                                R w;
-                                table_cell(org, inv, d.top, x, j, w);
-                                const Pair2<R> p = trow[j];
-                                const R var = p.a + w * p.b;
-                                x = lv_advance(x, var, d.hdt, leg ? -zd : zd);
-                                if (leg) lp1 = m_min(lp1, x + lf);
-                                else lp0 = m_min(lp0, x + lf);
-                            }
+                            R var0, var1;
+                            table_vars<true>(trow, 0u, org, inv, 0, d.top, x0[n], x1[n], var0, var1);
+                            lv_advance_legs(x0[n], x1[n], var0, var1, d.hdt, zd);
+                            lp0 = m_min(lp0, x0[n] + lf), lp1 = m_min(lp1, x1[n] + lf);
                         }
                     }
                     int j = -1;
@@ -366,11 +358,13 @@ BatchFn<R> pick_batch(bool qe, int n) {
 
 }  // namespace
 
+constexpr int kMaxTile = 8192;
+
 // A trade class: the trades sharing one kernel (model, names, product), with its tuned shape.
 struct BClass {
     bool qe = false;
     int n = 1, product = 0;
-    int tile = 8192, block = 256;
+    int tile = kMaxTile, block = 256;  // (default_tiles; ob_batch_tune)
     double untuned_ms = 0.0, tuned_ms = 0.0;  // the autotuner's sample at the shape before tuning and at the kept one
     std::vector<int> trades;
     const void* kernel = nullptr;
@@ -423,6 +417,7 @@ struct Batch {
     template <typename R>
     void build(const ob_batch_request& rq);
     void simulations();
+    void default_tiles();
     // per trade: its base, then under local vol one per vol move, then (2 names or more) one per correlation move
     int sims_of(int i) const {
         const ob_batch_trade& t = trades[i];
@@ -661,8 +656,32 @@ void Batch::simulations() {
     d_sim_outs = arena.put<int>(sim_outs.data(), sim_outs.size());
 }
 
-// Slots and items for per-class tiles. Items of a class go largest trade first, so that the persistent blocks end
-// together. With only_class, the items of that class alone, and with max_sims > 0 of at most that many of its
+// Each class's tile before tuning. An item is one block walking its tile's pairs 256 at a time, so an item of a large
+// tile in a small book is a long serial chain beside an idle GPU (a 32-trade, 8-vol-move book with 2^12 to 2^16 paths
+// a trade: 28 ms at 8192 pairs an item). The tile is the largest multiple of the block, up to kMaxTile, whose
+// item is at most 1 / kItemsPerBlock of the work a resident block gets of the whole book, so that the queues can even
+// out the classes' ends; a book large enough keeps kMaxTile (fewer slots to add). Work in name-steps of a pair; a
+// step of the quadratic-exponential scheme takes about kQeSteps of them.
+void Batch::default_tiles() {
+    constexpr double kItemsPerBlock = 8.0, kQeSteps = 6.0;
+    constexpr int kResident = 4;  // 256-thread blocks an SM
+    auto path = [&](int i) {
+        const ob_batch_trade& t = trades[i];
+        return t.n_steps * (t.model == OB_MODEL_PATHS ? static_cast<double>(t.n_names) : kQeSteps);
+    };
+    double total = 0.0;
+    for (int i = 0; i < n_trades; ++i) total += path(i) * static_cast<double>(trades[i].n_pairs) * sims_of(i);
+    const double most = total / (static_cast<double>(sms) * kResident * kItemsPerBlock);
+    for (BClass& c : classes) {
+        double longest = 1.0;
+        for (int t : c.trades) longest = std::max(longest, path(t));
+        const double pairs = std::min(most / longest, static_cast<double>(kMaxTile));
+        c.tile = std::max(1, static_cast<int>(pairs) / c.block) * c.block;
+    }
+}
+
+// Slots and items for per-class tiles. Items of a class go longest path first (items of a class are equal tiles), so that
+// the persistent blocks end together. With only_class, the items of that class alone, and with max_sims > 0 of at most that many of its
 // simulations, evenly spread over its largest-first order (the autotuner's sample).
 void Batch::layout(BLayout& L, const std::vector<int>& tiles, int only_class, int max_sims) {
     L.arena.release();
@@ -706,8 +725,8 @@ void Batch::layout(BLayout& L, const std::vector<int>& tiles, int only_class, in
         if (only_class >= 0 && static_cast<int>(ci) != only_class) continue;
         std::vector<int> order = classes[ci].trades;
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-            return static_cast<double>(trades[a].n_steps) * trades[a].n_names * trades[a].n_pairs >
-                   static_cast<double>(trades[b].n_steps) * trades[b].n_names * trades[b].n_pairs;
+            return trades[a].n_steps != trades[b].n_steps ? trades[a].n_steps > trades[b].n_steps
+                                                          : trades[a].n_pairs > trades[b].n_pairs;
         });
         std::vector<int4> items;
         for (int t : order) {
@@ -813,6 +832,7 @@ int ob_batch_create(const ob_batch_request* rq, int precision, ob_batch** batch)
             ob::check_cuda(cudaEventCreate(&b->impl.e0), "cudaEventCreate");
             ob::check_cuda(cudaEventCreate(&b->impl.e1), "cudaEventCreate");
             ob::check_cuda(cudaEventCreateWithFlags(&b->impl.fork, cudaEventDisableTiming), "cudaEventCreate");
+            b->impl.default_tiles();
             b->impl.layout(b->impl.main, b->impl.tiles());
         } catch (...) {
             delete b;
