@@ -123,6 +123,52 @@ void release_small_pinned() {
 }
 
 namespace {
+// the kept streams by (device, number)
+struct KeptStreams {
+    std::mutex m;
+    std::map<std::pair<int, int>, cudaStream_t> s;
+    static KeptStreams& get() {
+        static KeptStreams* k = new KeptStreams();
+        return *k;
+    }
+};
+}  // namespace
+
+cudaStream_t kept_stream(int which) {
+    if (which < 0 || which >= kKeptStreams) throw Error(OB_EINVAL, "no such stream");
+    int dev = 0;
+    check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    KeptStreams& k = KeptStreams::get();
+    std::lock_guard<std::mutex> lock(k.m);
+    const auto it = k.s.find({dev, which});
+    if (it != k.s.end()) return it->second;
+    cudaStream_t s = nullptr;
+    check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+    k.s[{dev, which}] = s;
+    return s;
+}
+
+void release_streams() {
+    KeptStreams& k = KeptStreams::get();
+    std::lock_guard<std::mutex> lock(k.m);
+    for (const auto& e : k.s) cudaStreamDestroy(e.second);
+    cudaGetLastError();
+    k.s.clear();
+}
+
+void upload_bytes(void* dst, const void* src, size_t n) {
+    char* slot[2] = {nullptr, nullptr};
+    if (n > kStagedUpload) slot[0] = PinnedStage::get().bytes(0), slot[1] = PinnedStage::get().bytes(1);
+    if (!slot[0] || !slot[1]) {
+        check_cuda(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice), "cudaMemcpy (inputs)");
+        return;
+    }
+    staged_upload(slot, static_cast<char*>(dst), n, PinnedStage::kSlotBytes, [&](char* out, size_t at, size_t count) {
+        std::memcpy(out, static_cast<const char*>(src) + at, count);
+    });
+}
+
+namespace {
 
 // One thread per (pair, block): the Philox outputs and both normal precisions, pair-major.
 __global__ void philox_kernel(uint32_t k0, uint32_t k1, long long first_pair, long long n_pairs, uint32_t tag,
@@ -169,6 +215,7 @@ int ob_release_buffers(void) {
         ob::PinnedStage::get().release();
         ob::clear_launch_caches();
         ob::release_small_pinned();
+        ob::release_streams();
     });
 }
 

@@ -81,17 +81,18 @@ void release_small_pinned();  // (ob_release_buffers)
 
 // ------------------------------------------------------------------------------------------------ device memory
 
-// A non-blocking stream owned by one call, destroyed with it.
-struct Stream {
-    cudaStream_t s = nullptr;
-    Stream() { check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate"); }
-    ~Stream() {
-        if (s) cudaStreamDestroy(s);
-    }
-    Stream(const Stream&) = delete;
-    Stream& operator=(const Stream&) = delete;
-    cudaStream_t get() const { return s; }
-};
+// Non-blocking streams of the current device kept for the calls that need their own (numbered from 0, kKeptStreams of
+// them a device, made at their first use): creating and destroying one costs 0.1 to 10 ms of driver time on a busy host.
+// The library's calls are serialised and finish their work on a kept stream before they return, so one set serves
+// them all.
+constexpr int kKeptStreams = 3;
+cudaStream_t kept_stream(int which);
+void release_streams();  // (ob_release_buffers)
+
+// n bytes of pageable host memory to dst on the device; the copy has finished when it returns. Above kStagedUpload the
+// bytes go through the pinned staging, spread over the host threads (host_copy.cuh).
+constexpr size_t kStagedUpload = size_t(256) << 10;
+void upload_bytes(void* dst, const void* src, size_t n);
 
 // Device buffers that finished calls handed back, for the next call of the process: a one-shot call's cudaMalloc and
 // cudaFree (a few hundred microseconds together, and cudaFree waits for the whole device) become a lookup. At most
@@ -260,7 +261,7 @@ class Upload {
     void commit(DeviceArena& arena) {
         if (bytes_.empty()) return;
         unsigned char* d = arena.alloc<unsigned char>(bytes_.size());
-        check_cuda(cudaMemcpy(d, bytes_.data(), bytes_.size(), cudaMemcpyHostToDevice), "cudaMemcpy (inputs)");
+        upload_bytes(d, bytes_.data(), bytes_.size());
         for (const Fix& f : fixes_) f.set(d + f.off);
     }
 

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "mc.cuh"
+#include "table_upload.cuh"
 
 namespace ob {
 
@@ -585,17 +586,15 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
     const size_t budget = sizeof(R) == 4 ? (110u << 10) : (220u << 10);  // two blocks a SM in float, one in double
     bool table_global = false;
     if (table) {
-        std::vector<Pair2<R>> tab(static_cast<size_t>(rq.n_rows) * (rq.n_x - 1));
-        for (int r = 0; r < rq.n_rows; ++r)
-            for (int k = 0; k + 1 < rq.n_x; ++k) {
-                const double* row = rq.table + static_cast<size_t>(r) * rq.n_x;
-                tab[static_cast<size_t>(r) * (rq.n_x - 1) + k] = {static_cast<R>(row[k]),
-                                                                   static_cast<R>(row[k + 1] - row[k])};
-            }
+        const size_t cells = table_cells(rq.n_rows, rq.n_x);
         const size_t at = (blob.bytes.size() + 15) & ~static_cast<size_t>(15);
-        table_global = at + tab.size() * sizeof(Pair2<R>) + acc_bytes > budget;
-        if (table_global) a.tab = plan.arena.put_raw(tab.data(), tab.size());
-        else a.off.table2 = blob.put(tab);
+        table_global = at + cells * sizeof(Pair2<R>) + acc_bytes > budget;
+        if (table_global) {
+            a.tab = upload_table<R>(plan.arena, rq.table, rq.n_rows, rq.n_x);
+        } else {
+            a.off.table2 = blob.put<Pair2<R>>(nullptr, cells);
+            pack_table<R>(rq.table, rq.n_x, 0, cells, reinterpret_cast<Pair2<R>*>(blob.bytes.data() + a.off.table2));
+        }
     }
     const FusedFn<R> fn = pick(table_global);
     a.smem_blob = static_cast<int>((blob.bytes.size() + 15) & ~static_cast<size_t>(15));

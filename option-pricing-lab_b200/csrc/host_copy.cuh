@@ -13,7 +13,63 @@
 
 #include "common.cuh"
 
+#if defined(__x86_64__)
+#include <cpuid.h>
+#include <emmintrin.h>
+#include <immintrin.h>
+#endif
+
 namespace ob {
+
+// Host memory that the GPU's copy engine reads or overwrites should not sit in the caches of the cores that wrote or
+// read it: on a B200 host a 4.8 MB upload takes 100 us from memory, and 750 us from lines dirty in eight cores' caches;
+// 11 MB of results land in 207 us, in 480 to 1300 us over lines those cores hold. So the threads write the staging
+// past the caches (stream_copy), and give up the lines they have read from it (drop_lines).
+// Copies n bytes to a 16-byte-aligned dst with non-temporal stores (src as aligned as dst).
+inline void stream_copy(void* dst, const void* src, size_t n) {
+#if defined(__x86_64__)
+    const size_t whole = n / 16;
+    const __m128i* s = static_cast<const __m128i*>(src);
+    __m128i* d = static_cast<__m128i*>(dst);
+    for (size_t i = 0; i < whole; ++i) _mm_stream_si128(d + i, _mm_loadu_si128(s + i));
+    std::memcpy(d + whole, s + whole, n - 16 * whole);
+    _mm_sfence();
+#else
+    std::memcpy(dst, src, n);
+#endif
+}
+#if defined(__x86_64__)
+__attribute__((target("clflushopt"))) inline void drop_lines_opt(const char* p, size_t n) {
+    for (size_t i = 0; i < n; i += 64) _mm_clflushopt(const_cast<char*>(p + i));
+    _mm_sfence();
+}
+#endif
+inline void drop_lines(const void* p, size_t n) {
+#if defined(__x86_64__)
+    static const bool have = [] {
+        unsigned a = 0, b = 0, c = 0, d = 0;
+        return __get_cpuid_count(7, 0, &a, &b, &c, &d) && ((b >> 23) & 1u);  // CLFLUSHOPT
+    }();
+    if (have) drop_lines_opt(static_cast<const char*>(p), n);
+#else
+    (void)p, (void)n;
+#endif
+}
+// n values of T widened into out (doubles), written past the caches where out allows it (8-byte aligned memory of which
+// every second double is 16-byte aligned).
+template <typename T>
+inline void widen(double* out, const T* from, long long n) {
+    long long k = 0;
+#if defined(__x86_64__)
+    if (n > 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 8u) out[0] = static_cast<double>(from[0]), k = 1;
+    if ((reinterpret_cast<uintptr_t>(out) & 7u) == 0u) {
+        for (; k + 2 <= n; k += 2)
+            _mm_stream_pd(out + k, _mm_set_pd(static_cast<double>(from[k + 1]), static_cast<double>(from[k])));
+        _mm_sfence();
+    }
+#endif
+    for (; k < n; ++k) out[k] = static_cast<double>(from[k]);
+}
 
 // Two pinned slots of kSlotBytes, allocated at their first use and kept until release() (ob_release_buffers).
 // Portable pinned memory: any device's copies may use it. Null where pinned memory cannot be had (the caller then
@@ -25,7 +81,7 @@ class PinnedStage {
         static PinnedStage* s = new PinnedStage();
         return *s;
     }
-    double* slot(int k) {
+    char* bytes(int k) {
         std::lock_guard<std::mutex> lock(m_);
         if (!base_ && !failed_) {
             if (cudaHostAlloc(&base_, 2 * kSlotBytes, cudaHostAllocPortable) != cudaSuccess) {
@@ -33,8 +89,7 @@ class PinnedStage {
                 base_ = nullptr, failed_ = true;
             }
         }
-        return base_ ? reinterpret_cast<double*>(static_cast<char*>(base_) + static_cast<size_t>(k) * kSlotBytes)
-                     : nullptr;
+        return base_ ? static_cast<char*>(base_) + static_cast<size_t>(k) * kSlotBytes : nullptr;
     }
     void release() {
         std::lock_guard<std::mutex> lock(m_);
@@ -112,5 +167,32 @@ class HostPool {
     int n_ = 0, next_ = 0, done_ = 0;
     unsigned long long gen_ = 0;
 };
+
+// n bytes to dst on the device through two pinned slots of slot_bytes each: make(out, at, count) writes bytes
+// [at, at + count) of the source into out, for blocks of 4 KB at multiples of 4 KB (so a source of records of 8 or 16
+// bytes converts block by block) spread over the host threads; a slot's copy runs while the other is filled. The
+// copies have finished when it returns.
+template <typename Make>
+void staged_upload(char* const (&slot)[2], char* dst, size_t n, size_t slot_bytes, Make make) {
+    constexpr size_t kPiece = size_t(256) << 10, kBlock = 4096;
+    cudaStream_t st = kept_stream(2);
+    int k = 0;
+    for (size_t at = 0; at < n; at += slot_bytes, ++k) {
+        if (k > 1) check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize (inputs)");  // slot k % 2 is free
+        const size_t count = std::min(slot_bytes, n - at);
+        char* out = slot[k % 2];
+        HostPool::get().run(static_cast<int>((count + kPiece - 1) / kPiece), [&](int item) {
+            alignas(64) char block[kBlock];
+            const size_t p0 = static_cast<size_t>(item) * kPiece, p1 = std::min(count, p0 + kPiece);
+            for (size_t q = p0; q < p1; q += kBlock) {
+                const size_t m = std::min(kBlock, p1 - q);
+                make(block, at + q, m);
+                stream_copy(out + q, block, m);
+            }
+        });
+        check_cuda(cudaMemcpyAsync(dst + at, out, count, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync (inputs)");
+    }
+    check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize (inputs)");
+}
 
 }  // namespace ob

@@ -30,7 +30,7 @@
 #include <cstring>
 #include <vector>
 
-#include "common.cuh"
+#include "host_copy.cuh"
 
 namespace ob {
 
@@ -878,28 +878,47 @@ void run_leverage(ob_leverage_request& rq) {
     d.v0 = rq.v0, d.kappa = rq.kappa, d.theta = rq.theta, d.xi = rq.xi, d.rho = rq.rho;
     d.atm_vol = rq.atm_vol, d.bw_scale = rq.bandwidth_scale, d.l_min = rq.l_min, d.l_max = rq.l_max;
     d.q_lo = rq.q_lo, d.q_hi = rq.q_hi;
-    d.dt = arena.put<double>(rq.dt, S);
-    d.t0 = arena.put<double>(rq.t0, S);
-    d.lv_lo = arena.put<double>(rq.lv_lo, S);
-    d.lv_inv_dx = arena.put<double>(rq.lv_inv_dx, S);
-    d.lv_rows = arena.put<double>(rq.lv_rows, static_cast<size_t>(S) * rq.n_lv);
+    // the kernel bandwidth of each step, as RC/src/leverage.cpp:63 computes it
+    const double n_particles = 2.0 * static_cast<double>(rq.n_pairs);
+    std::vector<double> bw(S);
+    for (int i = 0; i < S; ++i)
+        bw[i] = rq.bandwidth_scale * rq.atm_vol * std::sqrt(std::max(rq.t0[i], 0.15)) * std::pow(n_particles, -0.2);
+    const size_t rows_n = static_cast<size_t>(S) * rq.n_lv;
+    double* rows = arena.alloc<double>(rows_n);
+    upload_bytes(rows, rq.lv_rows, rows_n * sizeof(double));
+    d.lv_rows = rows;
+    Upload up;  // the small inputs in one copy
+    up.add<double>(d.dt, rq.dt, S);
+    up.add<double>(d.t0, rq.t0, S);
+    up.add<double>(d.lv_lo, rq.lv_lo, S);
+    up.add<double>(d.lv_inv_dx, rq.lv_inv_dx, S);
+    up.add<double>(d.bw, bw.data(), S);
+    up.commit(arena);
+    const cudaStream_t st = kept_stream(0);
     const int nb = rq.n_bins, nf = rq.n_fine, ll = rq.local_linear;
     d.nfp = (nf + kFinePad - 1) / kFinePad * kFinePad;
     d.nbq = (nb + 1 + 3) / 4 * 4;
     const size_t n_c = static_cast<size_t>(d.nbq);
-    d.fine = arena.alloc<unsigned>(d.nfp);
-    d.cnt = arena.alloc<unsigned>(n_c);
-    d.sv = arena.alloc<unsigned long long>(n_c);
-    d.acc_ll = arena.alloc<double>(3 * static_cast<size_t>(nb));
+    // what a calibration starts from zero, in one block (every part a multiple of 16 bytes): the histogram, the bins
+    // and their v sums, the local-linear moments, the barrier's counter and the status
+    const size_t fine_b = d.nfp * sizeof(unsigned), cnt_b = n_c * sizeof(unsigned), sv_b = n_c * sizeof(unsigned long long);
+    const size_t ll_b = (3 * static_cast<size_t>(nb) * sizeof(double) + 15) / 16 * 16;
+    const size_t zero_b = fine_b + cnt_b + sv_b + ll_b + 4 * sizeof(unsigned);
+    unsigned char* zero = arena.alloc<unsigned char>(zero_b);
+    d.fine = reinterpret_cast<unsigned*>(zero);
+    d.cnt = reinterpret_cast<unsigned*>(zero + fine_b);
+    d.sv = reinterpret_cast<unsigned long long*>(zero + fine_b + cnt_b);
+    d.acc_ll = reinterpret_cast<double*>(zero + fine_b + cnt_b + sv_b);
+    d.bar_count = reinterpret_cast<unsigned*>(zero + fine_b + cnt_b + sv_b + ll_b);
+    d.status = reinterpret_cast<int*>(d.bar_count + 2);
     d.rng = arena.alloc<long long>(4);
-    check_cuda(cudaMemset(d.fine, 0, d.nfp * sizeof(unsigned)), "cudaMemset");
-    check_cuda(cudaMemset(d.cnt, 0, n_c * sizeof(unsigned)), "cudaMemset");
-    check_cuda(cudaMemset(d.sv, 0, n_c * sizeof(unsigned long long)), "cudaMemset");
-    check_cuda(cudaMemset(d.acc_ll, 0, 3 * nb * sizeof(double)), "cudaMemset");
+    check_cuda(cudaMemsetAsync(zero, 0, zero_b, st), "cudaMemset");
     d.x_eval = arena.alloc<double>(rq.n_x);
     d.lev = arena.alloc<double>(rq.n_x);
-    d.x_grids = arena.alloc<double>(static_cast<size_t>(S) * rq.n_x);
-    d.values = arena.alloc<double>(static_cast<size_t>(S) * rq.n_x);
+    // the two output tables side by side: one copy back
+    const size_t out_n = static_cast<size_t>(S) * rq.n_x;
+    d.x_grids = arena.alloc<double>(2 * out_n);
+    d.values = d.x_grids + out_n;
     R* x = arena.alloc<R>(n);
     R* v = arena.alloc<R>(n);
     d.step = arena.alloc<int>(1);
@@ -912,18 +931,7 @@ void run_leverage(ob_leverage_request& rq) {
     // the three-kernel schedule's lev_step blocks (up to 4 an SM) each write their range
     d.part_range = arena.alloc<double>(2 * static_cast<size_t>(4 * sms));
     d.n_steps = S;
-    d.bar_count = arena.alloc<unsigned>(4);
-    d.status = reinterpret_cast<int*>(d.bar_count + 2);
-    check_cuda(cudaMemset(d.bar_count, 0, 4 * sizeof(unsigned)), "cudaMemset");
     d.wait_limit = g_wait_limit;
-    const double n_particles = 2.0 * static_cast<double>(rq.n_pairs);
-    // the kernel bandwidth of each step, as RC/src/leverage.cpp:63 computes it
-    std::vector<double> bw(S);
-    for (int i = 0; i < S; ++i)
-        bw[i] = rq.bandwidth_scale * rq.atm_vol * std::sqrt(std::max(rq.t0[i], 0.15)) * std::pow(n_particles, -0.2);
-    d.bw = arena.put<double>(bw.data(), S);
-    Stream stream;
-    cudaStream_t st = stream.get();
     cudaLaunchAttribute pdl[1];
     pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     pdl[0].val.programmaticStreamSerializationAllowed = 1;
@@ -932,6 +940,30 @@ void run_leverage(ob_leverage_request& rq) {
         c.gridDim = dim3(grid), c.blockDim = dim3(block), c.dynamicSmemBytes = smem, c.stream = st;
         c.attrs = pdl, c.numAttrs = 1;
         return c;
+    };
+    // the output tables and the status through the pinned staging (in one wait), the tables then copied into the
+    // caller's arrays; where it cannot hold them, the tables straight into those
+    double* pin = reinterpret_cast<double*>(PinnedStage::get().bytes(0));
+    if (2 * out_n * sizeof(double) + 16 > PinnedStage::kSlotBytes) pin = nullptr;
+    auto read_back = [&](int* status) {
+        int* const st_to = pin ? reinterpret_cast<int*>(pin + 2 * out_n) : status;
+        if (status)
+            check_cuda(cudaMemcpyAsync(st_to, d.status, sizeof(int), cudaMemcpyDeviceToHost, st), "copy status");
+        if (pin)
+            check_cuda(cudaMemcpyAsync(pin, d.x_grids, 2 * out_n * sizeof(double), cudaMemcpyDeviceToHost, st),
+                       "copy tables");
+        check_cuda(cudaStreamSynchronize(st), "leverage");
+        if (status && pin) *status = *st_to;
+    };
+    auto give_back = [&] {
+        const size_t bytes = out_n * sizeof(double);
+        if (pin) {
+            std::memcpy(rq.x_grids, pin, bytes);
+            std::memcpy(rq.values, pin + out_n, bytes);
+        } else {
+            check_cuda(cudaMemcpy(rq.x_grids, d.x_grids, bytes, cudaMemcpyDeviceToHost), "copy x_grids");
+            check_cuda(cudaMemcpy(rq.values, d.values, bytes, cudaMemcpyDeviceToHost), "copy values");
+        }
     };
     // OPTLAB_B200_LEVERAGE=graphs runs the three-kernel schedule below instead, =unpacked the persistent kernel with a
     // 32-bit fine histogram (to compare them; same results)
@@ -943,28 +975,17 @@ void run_leverage(ob_leverage_request& rq) {
     for (int attempt = 0; !graphs_only && attempt < 2; ++attempt) {
         if (!run_persistent<R>(d, n_particles, bin_smem, sms, st)) break;
         int status = 0;
-        check_cuda(cudaMemcpyAsync(&status, d.status, sizeof status, cudaMemcpyDeviceToHost, st), "copy status");
-        check_cuda(cudaStreamSynchronize(st), "leverage");
+        read_back(&status);
         if (status == kPackOverflow && d.packed) {
             // a fine bin held 2^16 particles or more: the same calibration again, unpacked, from clean buffers
             d.packed = 0;
-            check_cuda(cudaMemset(d.fine, 0, d.nfp * sizeof(unsigned)), "cudaMemset");
-            check_cuda(cudaMemset(d.cnt, 0, n_c * sizeof(unsigned)), "cudaMemset");
-            check_cuda(cudaMemset(d.sv, 0, n_c * sizeof(unsigned long long)), "cudaMemset");
-            check_cuda(cudaMemset(d.acc_ll, 0, 3 * nb * sizeof(double)), "cudaMemset");
-            check_cuda(cudaMemset(d.bar_count, 0, 4 * sizeof(unsigned)), "cudaMemset");
+            check_cuda(cudaMemsetAsync(zero, 0, zero_b, st), "cudaMemset");
             continue;
         }
         if (status == OB_ETIMEOUT)
             throw Error(OB_ETIMEOUT, "leverage: a grid barrier of the calibration gave up waiting for the other blocks");
         if (status != 0) throw Error(OB_ECUDA, "leverage: the calibration kernel reported a failure");
-        check_cuda(cudaMemcpyAsync(rq.x_grids, d.x_grids, static_cast<size_t>(S) * rq.n_x * sizeof(double),
-                                   cudaMemcpyDeviceToHost, st),
-                   "copy x_grids");
-        check_cuda(cudaMemcpyAsync(rq.values, d.values, static_cast<size_t>(S) * rq.n_x * sizeof(double),
-                                   cudaMemcpyDeviceToHost, st),
-                   "copy values");
-        check_cuda(cudaStreamSynchronize(st), "leverage");
+        give_back();
         rq.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
         return;
     }
@@ -984,8 +1005,7 @@ void run_leverage(ob_leverage_request& rq) {
     check_cuda(cudaLaunchKernelEx(&c_reg0, lev_regress, d, n_particles), "lev_regress launch");
     check_cuda(cudaLaunchKernelEx(&c_step0, lev_step<R>, d, x, v), "lev_step launch");
     // the other steps: graphs of kGraphSteps steps, replayed, and one of the remainder
-    Stream capture;
-    const cudaStream_t cs = capture.get();
+    const cudaStream_t cs = kept_stream(1);
     auto on = [&](cudaLaunchConfig_t c) {
         c.stream = cs;
         return c;
@@ -1021,13 +1041,8 @@ void run_leverage(ob_leverage_request& rq) {
         for (int r = 0; r < full; ++r) check_cuda(cudaGraphLaunch(ge, st), "cudaGraphLaunch (leverage)");
     }
     if (tail) check_cuda(cudaGraphLaunch(make_graph(tail), st), "cudaGraphLaunch (leverage)");
-    check_cuda(cudaMemcpyAsync(rq.x_grids, d.x_grids, static_cast<size_t>(S) * rq.n_x * sizeof(double),
-                               cudaMemcpyDeviceToHost, st),
-               "copy x_grids");
-    check_cuda(cudaMemcpyAsync(rq.values, d.values, static_cast<size_t>(S) * rq.n_x * sizeof(double),
-                               cudaMemcpyDeviceToHost, st),
-               "copy values");
-    check_cuda(cudaStreamSynchronize(st), "leverage");
+    read_back(nullptr);
+    give_back();
     rq.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
 }
 

@@ -18,8 +18,7 @@
 #include <cstring>
 #include <vector>
 
-#include "fused.cuh"
-#include "host_copy.cuh"
+#include "table_upload.cuh"
 
 namespace ob {
 
@@ -35,7 +34,7 @@ struct PathsDev {
     const int* win_lo;
     const int* win_hi;
     const R* fwd;  // n x n_obs
-    double* out;
+    R* out;
 };
 
 template <typename R, int N>
@@ -48,10 +47,10 @@ __device__ __forceinline__ void record(const PathsDev<R>& s, long long p, int j,
         if (a >= s.m.n_names) continue;
         const R f = s.fwd[a * s.n_obs + j];
         const R S0 = f * m_exp(st.x[0][a]), S1 = f * m_exp(st.x[1][a]);
-        double* base = s.out + static_cast<long long>(a) * s.n_cols * s.rows;
+        R* base = s.out + static_cast<long long>(a) * s.n_cols * s.rows;
         if (c >= 0) {
-            base[c * s.rows + r0] = static_cast<double>(S0);
-            base[c * s.rows + r1] = static_cast<double>(S1);
+            base[c * s.rows + r0] = S0;
+            base[c * s.rows + r1] = S1;
         }
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
@@ -65,10 +64,10 @@ __device__ __forceinline__ void record(const PathsDev<R>& s, long long p, int j,
             }
             if (j == s.win_hi[w]) {
                 const long long cl = s.n_keep + 2 * w, ch = cl + 1;
-                base[cl * s.rows + r0] = static_cast<double>(lo[0][a][w]);
-                base[ch * s.rows + r0] = static_cast<double>(hi[0][a][w]);
-                base[cl * s.rows + r1] = static_cast<double>(lo[1][a][w]);
-                base[ch * s.rows + r1] = static_cast<double>(hi[1][a][w]);
+                base[cl * s.rows + r0] = lo[0][a][w];
+                base[ch * s.rows + r0] = hi[0][a][w];
+                base[cl * s.rows + r1] = lo[1][a][w];
+                base[ch * s.rows + r1] = hi[1][a][w];
             }
         }
     }
@@ -109,7 +108,7 @@ struct PathsLvArgs {
     long long n_pairs, first_pair, rows;
     uint32_t k0, k1;
     R top;
-    double* out;
+    R* out;
     const Pair2<R>* tab;  // the table in global memory when it does not fit the stage (table_global), else unused
     int table_global;
     int kind, same;  // the names' model kind (0 Black-Scholes, 1 local vol, 2 Heston, 3 SLV); residuals through the root
@@ -127,10 +126,10 @@ __device__ __forceinline__ void lv_record(const PathsLvArgs<R>& a, const int* s_
     for (int n = 0; n < N; ++n) {
         const R f = s_fwd[n * a.n_obs + j];
         const R S0 = f * m_exp(x0[n]), S1 = f * m_exp(x1[n]);
-        double* base = a.out + static_cast<long long>(n) * a.n_cols * a.rows;
+        R* base = a.out + static_cast<long long>(n) * a.n_cols * a.rows;
         if (c >= 0 && active) {
-            base[c * a.rows + p] = static_cast<double>(S0);
-            base[c * a.rows + a.n_pairs + p] = static_cast<double>(S1);
+            base[c * a.rows + p] = S0;
+            base[c * a.rows + a.n_pairs + p] = S1;
         }
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
@@ -143,10 +142,10 @@ __device__ __forceinline__ void lv_record(const PathsLvArgs<R>& a, const int* s_
             }
             if (j == a.win_hi[w] && active) {
                 const long long cl = a.n_keep + 2 * w, ch = cl + 1;
-                base[cl * a.rows + p] = static_cast<double>(lo[0][n][w]);
-                base[ch * a.rows + p] = static_cast<double>(hi[0][n][w]);
-                base[cl * a.rows + a.n_pairs + p] = static_cast<double>(lo[1][n][w]);
-                base[ch * a.rows + a.n_pairs + p] = static_cast<double>(hi[1][n][w]);
+                base[cl * a.rows + p] = lo[0][n][w];
+                base[ch * a.rows + p] = hi[0][n][w];
+                base[cl * a.rows + a.n_pairs + p] = lo[1][n][w];
+                base[ch * a.rows + a.n_pairs + p] = hi[1][n][w];
             }
         }
     }
@@ -362,7 +361,7 @@ bool pack_paths_staged(const ob_paths_request& h, DeviceArena& arena, PathsLvArg
     auto put = [&](const void* src, size_t bytes) {
         const size_t at = (blob.size() + 15) & ~static_cast<size_t>(15);
         blob.resize(at + ((bytes + 15) & ~static_cast<size_t>(15)), 0);
-        if (bytes) std::memcpy(blob.data() + at, src, bytes);
+        if (src && bytes) std::memcpy(blob.data() + at, src, bytes);
         return static_cast<int>(at);
     };
     std::vector<StepRec<R>> steps(S);
@@ -417,18 +416,17 @@ bool pack_paths_staged(const ob_paths_request& h, DeviceArena& arena, PathsLvArg
     std::vector<R> fwd(static_cast<size_t>(n) * h.n_obs);
     for (size_t k = 0; k < fwd.size(); ++k) fwd[k] = static_cast<R>(h.fwd[k]);
     a.off.fwd = put(fwd.data(), fwd.size() * sizeof(R));
-    std::vector<Pair2<R>> tab(table ? static_cast<size_t>(h.n_rows) * (h.n_x - 1) : 0);
-    for (int r = 0; r < (table ? h.n_rows : 0); ++r)
-        for (int k = 0; k + 1 < h.n_x; ++k) {
-            const double y = h.table[static_cast<size_t>(r) * h.n_x + k], y1 = h.table[static_cast<size_t>(r) * h.n_x + k + 1];
-            tab[static_cast<size_t>(r) * (h.n_x - 1) + k] = {static_cast<R>(y), static_cast<R>(y1 - y)};
-        }
     const size_t budget = sizeof(R) == 4 ? (110u << 10) : (200u << 10);
-    const size_t tab_bytes = tab.size() * sizeof(Pair2<R>);
+    const size_t cells = table ? table_cells(h.n_rows, h.n_x) : 0;
     if (blob.size() > budget) return false;
-    a.table_global = ((blob.size() + 15) & ~static_cast<size_t>(15)) + tab_bytes > budget;
-    if (a.table_global) a.tab = arena.put_raw(tab.data(), tab.size());
-    else a.off.table2 = put(tab.data(), tab_bytes);
+    a.table_global = ((blob.size() + 15) & ~static_cast<size_t>(15)) + cells * sizeof(Pair2<R>) > budget;
+    if (a.table_global) {
+        a.tab = upload_table<R>(arena, h.table, h.n_rows, h.n_x);
+    } else {
+        a.off.table2 = put(nullptr, cells * sizeof(Pair2<R>));
+        if (cells)
+            pack_table<R>(h.table, h.n_x, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));
+    }
     a.smem_blob = static_cast<int>(blob.size());
     a.blob = arena.put<unsigned char>(blob.data(), blob.size());
     a.n_steps = S, a.n_obs = h.n_obs, a.n_cols = h.n_cols, a.n_keep = h.n_keep, a.n_win = h.n_windows;
@@ -496,33 +494,6 @@ void run_paths(ob_paths_request& h) {
     }
     DeviceArena arena;
     arena.recycle = true;  // both streams are synchronised before the call returns
-    PathsDev<R> s{};
-    ModelDev<R>& m = s.m;
-    m.n_names = n, m.n_steps = h.n_steps, m.n_x = h.n_x, m.same = h.same, m.mixer = h.mixer;
-    m.has_var = has_var, m.has_slv = has_slv;
-    m.k0 = static_cast<uint32_t>(h.seed), m.k1 = static_cast<uint32_t>(h.seed >> 32);
-    Upload up;  // the inputs in one copy
-    up.add<R>(m.dt, h.dt, h.n_steps);
-    up.add<R>(m.t0, h.t0, h.n_steps);
-    up.add<R>(m.root, h.root, static_cast<size_t>(n) * n);
-    up.add<int>(m.kind, h.kind, n);
-    up.add<R>(m.cvar, h.cvar, n);
-    up.add<R>(m.hes, h.heston, 5 * static_cast<size_t>(n));
-    if (table) {
-        up.add<int>(m.step_row, h.step_row, static_cast<size_t>(n) * h.n_steps);
-        up.add<R>(m.lo, h.row_lo, h.n_rows);
-        up.add<R>(m.inv_dx, h.row_inv_dx, h.n_rows);
-        up.add<R>(m.table, h.table, static_cast<size_t>(h.n_rows) * h.n_x);
-    }
-    if (h.mixer) up.add<R>(m.low_root, h.low_root, static_cast<size_t>(n) * n);
-    for (int k = 0; k < 8; ++k) m.mix[k] = static_cast<R>(h.mix[k]);
-    s.n_obs = h.n_obs, s.n_cols = h.n_cols, s.n_keep = h.n_keep, s.n_win = h.n_windows;
-    up.add<int>(s.obs_step, h.obs_step, h.n_obs);
-    up.add<int>(s.col_of, h.col_of, h.n_obs);
-    up.add<int>(s.win_lo, h.win_lo, h.n_windows);
-    up.add<int>(s.win_hi, h.win_hi, h.n_windows);
-    up.add<R>(s.fwd, h.fwd, static_cast<size_t>(n) * h.n_obs);
-    up.commit(arena);
     PathsLvArgs<R> lv{};
     const void* lv_fn = pack_paths_staged<R>(h, arena, lv)
                             ? pick_paths_staged<R>(n, lv.kind, lv.table_global != 0, h.mixer != 0)
@@ -533,33 +504,63 @@ void run_paths(ob_paths_request& h) {
         allow_smem(lv_fn, lv.smem_blob);
         lv_grid = require_device() * std::max(1, occupancy(lv_fn, lv_block_of(n), lv.smem_blob));
     }
+    PathsDev<R> s{};
+    if (!fast) {  // the generic kernel's inputs, in one copy
+        ModelDev<R>& m = s.m;
+        m.n_names = n, m.n_steps = h.n_steps, m.n_x = h.n_x, m.same = h.same, m.mixer = h.mixer;
+        m.has_var = has_var, m.has_slv = has_slv;
+        m.k0 = static_cast<uint32_t>(h.seed), m.k1 = static_cast<uint32_t>(h.seed >> 32);
+        Upload up;
+        up.add<R>(m.dt, h.dt, h.n_steps);
+        up.add<R>(m.t0, h.t0, h.n_steps);
+        up.add<R>(m.root, h.root, static_cast<size_t>(n) * n);
+        up.add<int>(m.kind, h.kind, n);
+        up.add<R>(m.cvar, h.cvar, n);
+        up.add<R>(m.hes, h.heston, 5 * static_cast<size_t>(n));
+        if (table) {
+            up.add<int>(m.step_row, h.step_row, static_cast<size_t>(n) * h.n_steps);
+            up.add<R>(m.lo, h.row_lo, h.n_rows);
+            up.add<R>(m.inv_dx, h.row_inv_dx, h.n_rows);
+            up.add<R>(m.table, h.table, static_cast<size_t>(h.n_rows) * h.n_x);
+        }
+        if (h.mixer) up.add<R>(m.low_root, h.low_root, static_cast<size_t>(n) * n);
+        for (int k = 0; k < 8; ++k) m.mix[k] = static_cast<R>(h.mix[k]);
+        s.n_obs = h.n_obs, s.n_cols = h.n_cols, s.n_keep = h.n_keep, s.n_win = h.n_windows;
+        up.add<int>(s.obs_step, h.obs_step, h.n_obs);
+        up.add<int>(s.col_of, h.col_of, h.n_obs);
+        up.add<int>(s.win_lo, h.win_lo, h.n_windows);
+        up.add<int>(s.win_hi, h.win_hi, h.n_windows);
+        up.add<R>(s.fwd, h.fwd, static_cast<size_t>(n) * h.n_obs);
+        up.commit(arena);
+    }
 
     // Chunks of pairs, on two streams: the kernel of one chunk runs while the previous chunk's columns are copied to
-    // the host. Large outputs go in four chunks at least; each chunk's output (two buffers) within an eighth of the
-    // free memory, at most 2 GB. The caller's array is not pinned (pinning 117 MB took 12.5 ms on a B200 host, longer
-    // than the pageable copy itself, 6.7 ms; pinned, 2.2 ms): a chunk is copied into the library's pinned staging
-    // (PinnedStage, at most a slot a chunk), and host threads spread it into the caller's array while the next chunk
-    // runs; without the staging, straight into the caller's array.
+    // the host. A chunk's columns come back in the paths' own type (a float's double is the same value: half the bytes
+    // over the link) into the library's pinned staging (PinnedStage, at most a slot a chunk; host memory of this call
+    // where pinned memory cannot be had), and host threads widen and spread them into the caller's array while the
+    // next chunk runs. Large outputs go in four chunks at least. (The caller's array is not pinned: pinning 117 MB
+    // took 12.5 ms on a B200 host, longer than the pageable copy itself, 6.7 ms; pinned, 2.2 ms.)
     const long long cols = static_cast<long long>(n) * h.n_cols;
-    size_t free_mem = 0, total_mem = 0;
-    check_cuda(cudaMemGetInfo(&free_mem, &total_mem), "cudaMemGetInfo");
-    const long long budget = std::min<long long>(static_cast<long long>(free_mem) / 8, 2LL << 30);
-    const long long row_bytes = cols * 2 * 8;  // one pair's output
-    double* stage[2] = {nullptr, nullptr};
-    if (cols > 0 && row_bytes <= static_cast<long long>(PinnedStage::kSlotBytes)) {
-        stage[0] = PinnedStage::get().slot(0), stage[1] = PinnedStage::get().slot(1);
-        if (!stage[0] || !stage[1]) stage[0] = stage[1] = nullptr;
-    }
+    const long long row_bytes = cols * 2 * static_cast<long long>(sizeof(R));  // one pair's output
+    constexpr long long kSlot = static_cast<long long>(PinnedStage::kSlotBytes);
     long long chunk = h.n_pairs;
     if (cols > 0) {
-        chunk = std::min(chunk, std::max<long long>(1024, budget / row_bytes));
-        if (row_bytes * h.n_pairs >= (32LL << 20)) chunk = std::min(chunk, (h.n_pairs + 3) / 4);
-        if (stage[0]) chunk = std::min(chunk, static_cast<long long>(PinnedStage::kSlotBytes) / row_bytes);
+        if (row_bytes * h.n_pairs >= kSlot / 8 * static_cast<long long>(sizeof(R))) chunk = (h.n_pairs + 3) / 4;
+        chunk = std::min(chunk, std::max<long long>(kSlot / row_bytes, 1024));
     }
-    double* dbuf[2] = {arena.alloc<double>(std::max<long long>(1, cols * 2 * chunk)),
-                       chunk < h.n_pairs ? arena.alloc<double>(std::max<long long>(1, cols * 2 * chunk)) : nullptr};
-    Stream s0, s1;
-    const cudaStream_t sts[2] = {s0.get(), s1.get()};
+    R* stage[2] = {nullptr, nullptr};
+    std::vector<R> own[2];
+    if (cols > 0) {
+        char* slot[2] = {PinnedStage::get().bytes(0), PinnedStage::get().bytes(1)};
+        const bool pinned = slot[0] && slot[1] && row_bytes * chunk <= kSlot;
+        for (int k = 0; k < 2; ++k) {
+            if (!pinned && (k == 0 || chunk < h.n_pairs)) own[k].resize(static_cast<size_t>(cols * 2 * chunk));
+            stage[k] = pinned ? reinterpret_cast<R*>(slot[k]) : own[k].data();
+        }
+    }
+    R* dbuf[2] = {arena.alloc<R>(std::max<long long>(1, cols * 2 * chunk)),
+                  chunk < h.n_pairs ? arena.alloc<R>(std::max<long long>(1, cols * 2 * chunk)) : nullptr};
+    const cudaStream_t sts[2] = {kept_stream(0), kept_stream(1)};
     std::vector<cudaEvent_t> evs;
     auto event = [&]() {
         cudaEvent_t e;
@@ -575,10 +576,10 @@ void run_paths(ob_paths_request& h) {
     } done{evs};
     const long long n_chunks = (h.n_pairs + chunk - 1) / chunk;
     std::vector<cudaEvent_t> k0(n_chunks), k1(n_chunks), staged(n_chunks);
-    // with the staging: chunk c's columns into slot c % 2 on its stream (after its kernel) ...
+    // chunk c's columns into slot c % 2 on its stream (after its kernel) ...
     auto stage_chunk = [&](long long c) {
         const long long mcount = std::min(chunk, h.n_pairs - c * chunk);
-        check_cuda(cudaMemcpyAsync(stage[c % 2], dbuf[c % 2], static_cast<size_t>(cols * 2 * mcount) * sizeof(double),
+        check_cuda(cudaMemcpyAsync(stage[c % 2], dbuf[c % 2], static_cast<size_t>(cols * 2 * mcount) * sizeof(R),
                                    cudaMemcpyDeviceToHost, sts[c % 2]),
                    "cudaMemcpyAsync (columns)");
         staged[c] = event();
@@ -591,37 +592,22 @@ void run_paths(ob_paths_request& h) {
         const long long c0 = c * chunk, mcount = std::min(chunk, h.n_pairs - c0);
         constexpr long long kPiece = 1 << 16;
         const long long pieces = (mcount + kPiece - 1) / kPiece;
-        const double* src = stage[c % 2];
+        const R* src = stage[c % 2];
         double* out = h.out;
         const long long P = h.n_pairs;
         HostPool::get().run(static_cast<int>(cols * 2 * pieces), [&](int item) {
             const long long col = item / (2 * pieces), leg = (item / pieces) % 2, q = item % pieces;
             const long long r0 = q * kPiece, r1 = std::min(mcount, r0 + kPiece);
-            std::memcpy(out + col * 2 * P + leg * P + c0 + r0, src + col * 2 * mcount + leg * mcount + r0,
-                        static_cast<size_t>(r1 - r0) * sizeof(double));
+            const R* from = src + col * 2 * mcount + leg * mcount + r0;
+            double* to = out + col * 2 * P + leg * P + c0 + r0;
+            widen(to, from, r1 - r0);
+            drop_lines(from, static_cast<size_t>(r1 - r0) * sizeof(R));
         });
-    };
-    auto copy_back = [&](long long c) {
-        if (cols <= 0) return;
-        if (stage[0]) {
-            spread_chunk(c);
-            return;
-        }
-        const long long c0 = c * chunk, mcount = std::min(chunk, h.n_pairs - c0);
-        const double* src = dbuf[c % 2];
-        const size_t width = static_cast<size_t>(mcount) * sizeof(double);
-        const size_t spitch = static_cast<size_t>(2 * mcount) * sizeof(double);
-        const size_t dpitch = static_cast<size_t>(2 * h.n_pairs) * sizeof(double);
-        check_cuda(cudaMemcpy2DAsync(h.out + c0, dpitch, src, spitch, width, cols, cudaMemcpyDeviceToHost, sts[c % 2]),
-                   "cudaMemcpy2D (leg 0)");
-        check_cuda(cudaMemcpy2DAsync(h.out + h.n_pairs + c0, dpitch, src + mcount, spitch, width, cols,
-                                     cudaMemcpyDeviceToHost, sts[c % 2]),
-                   "cudaMemcpy2D (leg 1)");
     };
     for (long long c = 0; c < n_chunks; ++c) {
         const long long c0 = c * chunk, mcount = std::min(chunk, h.n_pairs - c0);
         const cudaStream_t st = sts[c % 2];
-        double* out = dbuf[c % 2];
+        R* out = dbuf[c % 2];
         PathsDev<R> part = s;
         part.n_pairs = mcount, part.first_pair = h.first_pair + c0, part.rows = 2 * mcount, part.out = out;
         const int block = 256;
@@ -643,10 +629,10 @@ void run_paths(ob_paths_request& h) {
         else paths_kernel<R, 8><<<grid, block, 0, st>>>(part);
         check_cuda(cudaGetLastError(), "paths_kernel launch");
         check_cuda(cudaEventRecord(k1[c], st), "cudaEventRecord");
-        if (cols > 0 && stage[0]) stage_chunk(c);
-        if (c > 0) copy_back(c - 1);  // the host waits for it while chunk c runs on the other stream
+        if (cols > 0) stage_chunk(c);
+        if (cols > 0 && c > 0) spread_chunk(c - 1);  // the host waits for it while chunk c runs on the other stream
     }
-    copy_back(n_chunks - 1);
+    if (cols > 0) spread_chunk(n_chunks - 1);
     check_cuda(cudaStreamSynchronize(sts[0]), "paths");
     check_cuda(cudaStreamSynchronize(sts[1]), "paths");
     float kernel_ms = 0.0f;

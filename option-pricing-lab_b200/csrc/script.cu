@@ -23,6 +23,7 @@
 
 #include "exercise.cuh"
 #include "mc.cuh"
+#include "table_upload.cuh"
 
 namespace ob {
 
@@ -559,7 +560,7 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
                 const StepRec<R> st = s_step[i - 1];
                 const bool before = BRANCH && i <= d.branch_step;
                 const R* zs = before ? &zo[g * C] : &z[g * C];
-                const R sg0 = before ? osign : R(1), sg1 = before ? osign : R(-1);  // the legs' signs
+                [[maybe_unused]] const R sg0 = before ? osign : R(1), sg1 = before ? osign : R(-1);  // the legs' signs
                 R zc[N];
 #pragma unroll
                 for (int n = 0; n < N; ++n) {
@@ -683,7 +684,7 @@ bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, Device
     auto put = [&](const void* src, size_t bytes) {
         const size_t at = (blob.size() + 15) & ~static_cast<size_t>(15);
         blob.resize(at + ((bytes + 15) & ~static_cast<size_t>(15)), 0);
-        if (bytes) std::memcpy(blob.data() + at, src, bytes);
+        if (src && bytes) std::memcpy(blob.data() + at, src, bytes);
         return static_cast<int>(at);
     };
     std::vector<StepRec<R>> steps(S);
@@ -711,18 +712,17 @@ bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, Device
     a.off.root = put(root.data(), root.size() * sizeof(R));
     a.off.lf0 = put(lf0.data(), lf0.size() * sizeof(R));
     a.off.sched = put(sched.data(), sched.size() * sizeof(int2));
-    std::vector<Pair2<R>> tab(static_cast<size_t>(q.n_rows) * (q.n_x - 1));
-    for (int r = 0; r < q.n_rows; ++r)
-        for (int k = 0; k + 1 < q.n_x; ++k) {
-            const double* row = q.table + static_cast<size_t>(r) * q.n_x;
-            tab[static_cast<size_t>(r) * (q.n_x - 1) + k] = {static_cast<R>(row[k]), static_cast<R>(row[k + 1] - row[k])};
-        }
+    const size_t cells = table_cells(q.n_rows, q.n_x);
     const size_t budget = sizeof(R) == 4 ? (110u << 10) : (220u << 10);
     if (blob.size() > budget) return false;
-    a.table_global = ((blob.size() + 15) & ~static_cast<size_t>(15)) + tab.size() * sizeof(Pair2<R>) > budget;
+    a.table_global = ((blob.size() + 15) & ~static_cast<size_t>(15)) + cells * sizeof(Pair2<R>) > budget;
     if (a.table_global && (rq.branch || rq.n_calls > 0 || rq.n_windows > 2)) return false;
-    if (a.table_global) a.tab = arena.put_raw(tab.data(), tab.size());
-    else a.off.table2 = put(tab.data(), tab.size() * sizeof(Pair2<R>));
+    if (a.table_global) {
+        a.tab = upload_table<R>(arena, q.table, q.n_rows, q.n_x);
+    } else {
+        a.off.table2 = put(nullptr, cells * sizeof(Pair2<R>));
+        pack_table<R>(q.table, q.n_x, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));
+    }
     a.smem_blob = static_cast<int>((blob.size() + 15) & ~static_cast<size_t>(15));
     unsigned char* dblob = arena.alloc<unsigned char>(std::max<size_t>(16, blob.size()));
     check_cuda(cudaMemcpy(dblob, blob.data(), blob.size(), cudaMemcpyHostToDevice), "copy blob");
@@ -873,16 +873,36 @@ void run_script(const ob_script_request& rq, ob_script_result& res, const Record
     ScriptDev<R> d{};
     d.model = mq.model, d.n_names = n, d.n_steps = S;
     for (int a = 0; a < n; ++a) d.spot0[a] = static_cast<R>(mq.spot[a]);
+    std::vector<int> event_at(S + 1, -1);
+    for (int k = 0; k < rq.n_events; ++k) event_at[rq.event_step[k]] = k;
+    std::vector<unsigned> fix_mask(S + 1, 0u);
+    std::vector<int> nfix(std::max(1, rq.n_windows), 0);
+    for (int w = 0; w < rq.n_windows; ++w) {
+        for (int k = rq.win_fix0[w]; k < rq.win_fix0[w + 1]; ++k) fix_mask[rq.fix_step[k]] |= 1u << w;
+        nfix[w] = rq.win_fix0[w + 1] - rq.win_fix0[w];
+    }
+    // per step end (event, window mask); a step end without an event holds minus the number of steps to the next
+    // one (past the last, more than any batch)
+    std::vector<int2> sched(S + 1);
+    for (int i = S, next = S + (1 << 20); i >= 0; --i) {
+        if (event_at[i] >= 0) next = i;
+        sched[i] = make_int2(event_at[i] >= 0 ? event_at[i] : i - next, static_cast<int>(fix_mask[i]));
+    }
+    LvArgs<R> lv{};
+    const bool fast = pack_lv<R>(rq, sched, arena, lv);
+    if (rq.branch && !fast) invalid("a branched run needs the staged local-vol kernel (its tables too large)");
     Upload up;
     ModelDev<R>& m = d.m;
     m.n_names = n, m.n_steps = S, m.n_x = mq.n_x, m.same = mq.same, m.mixer = mq.mixer;
-    up.add<R>(m.dt, mq.dt, S);
-    up.add<R>(m.t0, mq.t0, S);
+    if (!fast) {  // the generic kernel's inputs (the staged kernel reads its blob)
+        up.add<R>(m.dt, mq.dt, S);
+        up.add<R>(m.t0, mq.t0, S);
+    }
     if (mq.mixer) {  // local correlation: the generic interpreter kernel runs it (pack_lv declines)
         up.add<R>(m.low_root, mq.low_root, static_cast<size_t>(n) * n);
         for (int k = 0; k < 8; ++k) m.mix[k] = static_cast<R>(mq.mix[k]);
     }
-    if (mq.model == OB_MODEL_PATHS) {
+    if (mq.model == OB_MODEL_PATHS && !fast) {
         bool table = false;
         for (int a = 0; a < n; ++a) {
             m.has_var |= mq.kind[a] == 2 || mq.kind[a] == 3;
@@ -900,7 +920,7 @@ void run_script(const ob_script_request& rq, ob_script_result& res, const Record
             up.add<R>(m.table, mq.table, static_cast<size_t>(mq.n_rows) * mq.n_x);
         }
         up.add<R>(d.lf, mq.log_fwd, static_cast<size_t>(n) * (S + 1));
-    } else {
+    } else if (mq.model != OB_MODEL_PATHS) {
         d.qe = make_qe_consts<R>(mq.heston, mq.r, mq.q, mq.dt[0]);
     }
     std::vector<int4> code(static_cast<size_t>(rq.n_code));  // (the caller's ints need not be 16-byte aligned)
@@ -908,18 +928,10 @@ void run_script(const ob_script_request& rq, ob_script_result& res, const Record
     up.add<int4>(d.code, code.data(), code.size());
     up.add<double>(d.consts, rq.consts, rq.n_const);
     d.n_const = rq.n_const, d.n_regs = rq.n_regs;
-    std::vector<int> event_at(S + 1, -1);
-    for (int k = 0; k < rq.n_events; ++k) event_at[rq.event_step[k]] = k;
-    up.add<int>(d.event_at, event_at.data(), event_at.size());
+    if (!fast) up.add<int>(d.event_at, event_at.data(), event_at.size());
     up.add<int>(d.event_code, rq.event_code, rq.n_events + 1);
     up.add<double>(d.event_disc, rq.event_discount, rq.n_events);
-    std::vector<unsigned> fix_mask(S + 1, 0u);
-    std::vector<int> nfix(std::max(1, rq.n_windows), 0);
-    for (int w = 0; w < rq.n_windows; ++w) {
-        for (int k = rq.win_fix0[w]; k < rq.win_fix0[w + 1]; ++k) fix_mask[rq.fix_step[k]] |= 1u << w;
-        nfix[w] = rq.win_fix0[w + 1] - rq.win_fix0[w];
-    }
-    up.add<unsigned>(d.fix_mask, fix_mask.data(), fix_mask.size());
+    if (!fast) up.add<unsigned>(d.fix_mask, fix_mask.data(), fix_mask.size());
     d.n_windows = rq.n_windows;
     if (rq.n_windows) {
         up.add<int>(d.win_name, rq.win_name, rq.n_windows);
@@ -964,16 +976,6 @@ void run_script(const ob_script_request& rq, ob_script_result& res, const Record
     up.commit(arena);
     d.bad = outs;
 
-    // per step end (event, window mask); a step end without an event holds minus the number of steps to the next
-    // one (past the last, more than any batch)
-    std::vector<int2> sched(S + 1);
-    for (int i = S, next = S + (1 << 20); i >= 0; --i) {
-        if (event_at[i] >= 0) next = i;
-        sched[i] = make_int2(event_at[i] >= 0 ? event_at[i] : i - next, static_cast<int>(fix_mask[i]));
-    }
-    LvArgs<R> lv{};
-    const bool fast = pack_lv<R>(rq, sched, arena, lv);
-    if (rq.branch && !fast) invalid("a branched run needs the staged local-vol kernel (its tables too large)");
     const void* fn = fast ? reinterpret_cast<const void*>(
                                 pick_lv<R>(n, rq.n_windows, rq.n_windows ? rq.win_func[0] : -1, rq.branch != 0, rq.n_calls > 0,
                                           lv.table_global != 0))

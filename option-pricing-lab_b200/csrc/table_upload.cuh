@@ -1,0 +1,46 @@
+// A table of n_rows x n_x doubles as its (y_i, y_i+1 - y_i) intervals in R: into a host array (the staged blobs), or into
+// global memory for tables beyond the stage, converted by the host threads straight into the pinned staging (the 801
+// points of each of 504 steps, 3.2 MB of intervals: 0.59 ms as one thread's conversion and a pageable copy).
+#pragma once
+
+#include "fused.cuh"
+#include "host_copy.cuh"
+
+namespace ob {
+
+inline size_t table_cells(int n_rows, int n_x) {
+    return static_cast<size_t>(n_rows) * static_cast<size_t>(n_x - 1);
+}
+
+// Intervals [first, first + count) into out.
+template <typename R>
+inline void pack_table(const double* table, int n_x, size_t first, size_t count, Pair2<R>* out) {
+    const size_t w = static_cast<size_t>(n_x - 1);
+    size_t row = first / w, k = first - row * w;
+    for (size_t done = 0; done < count; ++row, k = 0) {
+        const double* y = table + row * static_cast<size_t>(n_x);
+        const size_t end = std::min(w, k + (count - done));
+        for (; k < end; ++k, ++done) out[done] = {static_cast<R>(y[k]), static_cast<R>(y[k + 1] - y[k])};
+    }
+}
+
+template <typename R>
+inline Pair2<R>* upload_table(DeviceArena& arena, const double* table, int n_rows, int n_x) {
+    const size_t cells = table_cells(n_rows, n_x);
+    Pair2<R>* d = arena.alloc<Pair2<R>>(cells);
+    char* slot[2] = {PinnedStage::get().bytes(0), PinnedStage::get().bytes(1)};
+    if (!slot[0] || !slot[1]) {
+        std::vector<Pair2<R>> tab(cells);
+        pack_table<R>(table, n_x, 0, cells, tab.data());
+        check_cuda(cudaMemcpy(d, tab.data(), cells * sizeof(Pair2<R>), cudaMemcpyHostToDevice), "cudaMemcpy (table)");
+        return d;
+    }
+    staged_upload(slot, reinterpret_cast<char*>(d), cells * sizeof(Pair2<R>), PinnedStage::kSlotBytes,
+                  [&](char* out, size_t at, size_t count) {
+                      pack_table<R>(table, n_x, at / sizeof(Pair2<R>), count / sizeof(Pair2<R>),
+                                    reinterpret_cast<Pair2<R>*>(out));
+                  });
+    return d;
+}
+
+}  // namespace ob
