@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "mc.cuh"
+#include "qe64.cuh"
 #include "table_upload.cuh"
 
 namespace ob {
@@ -365,29 +366,75 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
         R x = R(0), v = a.qe.v0, lp = R(0);
         Leg<R> l;
         leg_init<R, PRODUCT>(l);
-        for (int i0 = 1, m = 0; i0 <= S; i0 += 4, ++m) {
-            R z[4], e[8];
-            normals4<R>(pair, static_cast<uint64_t>(2 * m + odd), 0u, k0, k1, z[0], z[1], z[2], z[3]);
+        auto keep = [&](int i) {  // the leg's books at step end i
+            lp = x;
+            if (PRODUCT == OB_PRODUCT_LADDER) {
+                l.hi = run_max(l.hi, lp), l.lo = run_min(l.lo, lp);
+            } else {
+                l.lo = run_min(l.lo, lp);
+                const int j = s_step[i - 1].obs;
+                if (j >= 0) leg_observe(a, s_trig, s_disc, l, lp, j);
+            }
+        };
+        // the lane's own block of the two of batch m, and both lanes' normals of its four steps
+        auto swap = [&](const R (&z)[4], R (&e)[8]) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const R o = __shfl_xor_sync(kFull, z[k], 1);
                 e[k] = odd ? o : z[k];      // block 2m: steps i0, i0 + 1
                 e[4 + k] = odd ? z[k] : o;  // block 2m + 1: steps i0 + 2, i0 + 3
             }
-            // one copy of the (long, FP64) step in the loop body: the four steps rotate the normals through e[0..1]
+        };
+        if constexpr (sizeof(R) == 8) {
+            // the steps of a batch and the next batch's draws and tails in one straight line: they do not wait for
+            // each other
+            const Qe64Tables& t = *reinterpret_cast<const Qe64Tables*>(sm + a.off.qe_tables);
+            R e[8], tail[4];
+            auto draw = [&](int m) {
+                uint32_t c[4] = {static_cast<uint32_t>(pair), static_cast<uint32_t>(pair >> 32),
+                                 static_cast<uint32_t>(2 * m + odd), 0u};
+                philox4x32_10(c[0], c[1], c[2], c[3], k0, k1);
+                R z[4];
+                box_muller64(t, c[0], c[1], z[0], z[1]);
+                box_muller64(t, c[2], c[3], z[2], z[3]);
+                swap(z, e);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) e[2 * g] *= sgn, e[2 * g + 1] *= sgn, tail[g] = tail64(t, e[2 * g]);
+            };
+            draw(0);
+            int i = 1, m = 0;
+            for (; i + 3 <= S; i += 4) {
+                R ce[8], ct[4];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) ce[k] = e[k];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) ct[k] = tail[k];
+                draw(++m);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    qe64_step(a.qe, t, x, v, ce[2 * g], ce[2 * g + 1], ct[g]);
+                    keep(i + g);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < 3; ++g)
+                if (i + g <= S) {
+                    qe64_step(a.qe, t, x, v, e[2 * g], e[2 * g + 1], tail[g]);
+                    keep(i + g);
+                }
+        } else {
+            for (int i0 = 1, m = 0; i0 <= S; i0 += 4, ++m) {
+                R z[4], e[8];
+                normals4<R>(pair, static_cast<uint64_t>(2 * m + odd), 0u, k0, k1, z[0], z[1], z[2], z[3]);
+                swap(z, e);
+                // one copy of the step in the loop body: the four steps rotate the normals through e[0..1]
 #pragma unroll 1
-            for (int g = 0; g < 4; ++g) {
-                const int i = i0 + g;
-                if (i > S) break;
-                qe_step_warp(a.qe, x, v, sgn * e[0], sgn * e[1]);  // (all 32 lanes step together)
-                e[0] = e[2], e[1] = e[3], e[2] = e[4], e[3] = e[5], e[4] = e[6], e[5] = e[7];
-                lp = x;
-                if (PRODUCT == OB_PRODUCT_LADDER) {
-                    l.hi = m_max(l.hi, lp), l.lo = m_min(l.lo, lp);
-                } else {
-                    l.lo = m_min(l.lo, lp);
-                    const int j = s_step[i - 1].obs;
-                    if (j >= 0) leg_observe(a, s_trig, s_disc, l, lp, j);
+                for (int g = 0; g < 4; ++g) {
+                    const int i = i0 + g;
+                    if (i > S) break;
+                    qe_step_warp(a.qe, x, v, sgn * e[0], sgn * e[1]);  // (all 32 lanes step together)
+                    e[0] = e[2], e[1] = e[3], e[2] = e[4], e[3] = e[5], e[4] = e[6], e[5] = e[7];
+                    keep(i);
                 }
             }
         }
@@ -521,6 +568,7 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
     const bool table = kind == 1 || kind == 3;
     if (kind == 4) {
         a.qe = make_qe_consts<R>(rq.heston, rq.r, rq.q, rq.dt[0]);
+        if (sizeof(R) == 8) a.off.qe_tables = blob.put(&qe64_tables(), 1);
     } else {
         std::vector<NameStep<R>> ns(static_cast<size_t>(S) * n);
         for (int i = 1; i <= S; ++i)

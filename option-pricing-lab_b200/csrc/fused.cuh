@@ -233,6 +233,7 @@ struct alignas(16) StepRec {
 struct FusedOffsets {
     int step, name_step, root, hes, table2, ln_trig, obs_disc, leg_type, leg_strike, leg_barrier, ln_level;
     int mix_den, low_root;  // local correlation: per step sigma sqrt(max(t0, 1/12)); the aligned low root
+    int qe_tables;          // Heston QE in double: Qe64Tables
 };
 
 template <typename R>
