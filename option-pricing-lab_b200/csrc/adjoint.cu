@@ -749,11 +749,10 @@ void AdjPlan::build(const ob_adjoint_request& r) {
                    "cudaFuncSetAttribute");
     }
     tab_n = rq.n_rows * rq.n_x;
-    int per_f = 0, per_b = 0;
-    check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_f, kfs, block_f, smem), "occupancy");
+    int per_b = 0;
     check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_b, kb, block_b, smem_b), "occupancy");
-    grid_f = static_cast<int>(std::max<long long>(
-        1, std::min<long long>((P + block_f - 1) / block_f, static_cast<long long>(sms) * std::max(1, per_f))));
+    const LaunchShape f = launch_shape(kfs, smem, sms, P, block_f);
+    block_f = f.block, grid_f = f.grid;
     const long long pairs_b = dense ? block_b / 2 : block_b;  // the dense backward takes one leg a thread
     grid_b = static_cast<int>(std::max<long long>(
         1, std::min<long long>((P + pairs_b - 1) / pairs_b, static_cast<long long>(sms) * std::max(1, per_b))));

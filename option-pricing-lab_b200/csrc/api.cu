@@ -91,6 +91,25 @@ void allow_smem(const void* kernel, size_t smem) {
     have = smem;
 }
 
+LaunchShape launch_shape(const void* kernel, size_t smem, int sms, long long units, int max_block) {
+    constexpr double kIssueWarps = 24.0;
+    const long long chunks = (units + 31) / 32;
+    auto grid_of = [&](int b) {
+        const long long full = static_cast<long long>(sms) * std::max(1, occupancy(kernel, b, smem));
+        return std::max<long long>(1, std::min<long long>((units + b - 1) / b, full));
+    };
+    double best = -1.0;
+    int best_block = max_block;
+    for (int b = max_block; b >= 64; b -= 32) {
+        const long long grid = grid_of(b), warps = grid * (b / 32), rounds = (chunks + warps - 1) / warps;
+        const double fill = static_cast<double>(chunks) / static_cast<double>(rounds * warps);
+        const double per_sm = static_cast<double>(warps) / sms;
+        const double score = fill * std::min(1.0, per_sm / kIssueWarps) * std::min(1.0, static_cast<double>(grid) / sms);
+        if (score > best * 1.0001) best = score, best_block = b;
+    }
+    return {best_block, static_cast<int>(grid_of(best_block))};
+}
+
 void clear_launch_caches() {
     LaunchCaches& c = LaunchCaches::get();
     std::lock_guard<std::mutex> lock(c.m);

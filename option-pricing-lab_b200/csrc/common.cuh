@@ -70,6 +70,18 @@ int occupancy(const void* kernel, int block, size_t smem);
 // Raises kernel's dynamic shared-memory limit on the current device to at least smem bytes (once per kernel and
 // size: the attribute is a maximum, so a larger setting serves smaller launches).
 void allow_smem(const void* kernel, size_t smem);
+// Block size and grid of a launch whose warps each take chunks of 32 threads' units grid-stride, every chunk the same
+// length (a whole path): the run lasts ceil(chunks / resident warps) rounds, so among the multiples of 32 from max_block
+// down to 64 the block is taken that keeps that ceiling close to the exact quotient, with enough warps on each SM to keep
+// its schedulers issuing (24; fewer count as proportionally slower) and as many SMs as can be at work. 2^19 pairs of the
+// fused Phoenix: 448-thread blocks run 3.95 of 4 rounds where 512 leave a fourth round 46 % full (1.39 against
+// 1.52 ms); 2^18 pairs of the script kernel run two full rounds at 448 where 512 leave the second three quarters full
+// (877 -> 801 us a call); 2^16 pairs of the adjoint's forward run on 147 SMs at 448 where 1024 reached 64 (Greeks
+// 4.16 -> 3.58 ms). smem: dynamic shared memory at any block size.
+struct LaunchShape {
+    int block, grid;
+};
+LaunchShape launch_shape(const void* kernel, size_t smem, int sms, long long units, int max_block);
 // Forgets both (ob_release_buffers: after a device reset the kernels' attributes are gone).
 void clear_launch_caches();
 

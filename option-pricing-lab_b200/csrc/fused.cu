@@ -653,14 +653,12 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
     a.blob = d;
     const void* k = reinterpret_cast<const void*>(fn);
     allow_smem(k, smem);
-    const int per_sm = occupancy(k, block, smem);
-    if (per_sm < 1) return false;
+    if (occupancy(k, block, smem) < 1) return false;
     plan.fused = true;
     plan.threads_per_pair = kind == 4 ? 2 : 1;
     plan.kernel = k;
     plan.block = block;
     plan.smem_bytes = smem;
-    plan.blocks_per_sm = per_sm;
     plan.n_out = a.n_out;
     plan.fused_args<R>() = a;
     return true;

@@ -418,7 +418,6 @@ void McPlan::build(const ob_mc_request& rq) {
     smem_bytes = static_cast<size_t>(a.smem_blob) + acc_bytes;
     kernel = reinterpret_cast<const void*>(pick<R>(rq.model, rq.product, n));
     allow_smem(kernel, smem_bytes);
-    blocks_per_sm = std::max(1, occupancy(kernel, block, smem_bytes));
 }
 
 template void McPlan::build<float>(const ob_mc_request&);
@@ -444,53 +443,10 @@ McPlan::~McPlan() {
     if (e1) cudaEventDestroy(e1);
 }
 
-// Block size and grid of a run. Among the plan's block and its halves down to 64 threads, the shape that keeps the
-// most warps resident on the most SMs: a small batch (2^15 pairs of the QE ladder) then spreads over every SM in
-// small blocks, while a large one keeps 512-thread blocks. The grid fills each SM once with resident blocks and the
-// pairs are handed out grid-stride.
-int McPlan::occupancy_at(int blk) {
-    if (blk == block) return blocks_per_sm;
-    for (int k = 0; k < 16; ++k)
-        if (occ_block[k] == blk) return occ_blocks[k];
-    const int per_sm = std::max(1, occupancy(kernel, blk, smem_bytes));
-    for (int k = 0; k < 16; ++k)
-        if (!occ_block[k]) {
-            occ_block[k] = blk, occ_blocks[k] = per_sm;
-            break;
-        }
-    return per_sm;
-}
-
-// Block size and grid of a launch. A warp works through its pairs in chunks of 32 lanes, every chunk the whole path,
-// so the run lasts ceil(chunks / resident warps) rounds: the block size is chosen (multiples of 32 up to the plan's
-// block) to keep that ceiling close to the exact quotient, with enough warps on each SM to keep its schedulers
-// issuing (kIssueWarps; fewer count as proportionally slower).
-int McPlan::launch_shape(long long n_pairs, int& blk) {
-    constexpr double kIssueWarps = 24.0;
-    const long long units = n_pairs * threads_per_pair;
-    const long long chunks = (units + 31) / 32;
-    double best = -1.0;
-    int best_blk = block;
-    for (int b = block; b >= 64; b -= 32) {
-        const long long need = (units + b - 1) / b;
-        const long long grid = std::min<long long>(need, static_cast<long long>(sms) * occupancy_at(b));
-        const long long warps = grid * (b / 32);
-        const long long rounds = (chunks + warps - 1) / warps;
-        const double fill = static_cast<double>(chunks) / static_cast<double>(rounds * warps);
-        const double per_sm = static_cast<double>(warps) / sms;
-        const double score = fill * std::min(1.0, per_sm / kIssueWarps) * std::min(1.0, static_cast<double>(grid) / sms);
-        if (score > best * 1.0001) best = score, best_blk = b;
-    }
-    blk = best_blk;
-    const long long need = (units + blk - 1) / blk;
-    const long long full = static_cast<long long>(sms) * occupancy_at(blk) * grid_waves;
-    return static_cast<int>(std::max<long long>(1, std::min<long long>({need, full, max_blocks})));
-}
-
 void McPlan::run(long long n_pairs, long long first_pair, unsigned long long seed, cudaStream_t st) {
     if (n_pairs < 1 || first_pair < 0) invalid("n_pairs must be >= 1 and first_pair >= 0");
-    int blk = block;
-    const int grid = launch_shape(n_pairs, blk);
+    const LaunchShape shape = launch_shape(kernel, smem_bytes, sms, n_pairs * threads_per_pair, block);
+    const int grid = std::min(shape.grid, max_blocks), blk = shape.block;
     const uint32_t k0 = static_cast<uint32_t>(seed), k1 = static_cast<uint32_t>(seed >> 32);
     if (!timing) check_cuda(cudaEventRecord(e0, st), "cudaEventRecord"), timing = true;
     using FusedF = void (*)(FusedArgs<float>, long long, long long, uint32_t, uint32_t, double*);

@@ -484,7 +484,7 @@ const void* pick_paths_staged(int n, int kind, bool table_global, bool mixer) {
 template <typename R>
 void run_paths(ob_paths_request& h) {
     const auto t_start = std::chrono::steady_clock::now();
-    require_device();
+    const int sms = require_device();
     const int n = h.n_names;
     bool table = false, has_var = false, has_slv = false;
     for (int a = 0; a < n; ++a) {
@@ -499,11 +499,7 @@ void run_paths(ob_paths_request& h) {
                             ? pick_paths_staged<R>(n, lv.kind, lv.table_global != 0, h.mixer != 0)
                             : nullptr;
     const bool fast = lv_fn != nullptr;
-    int lv_grid = 0;
-    if (fast) {
-        allow_smem(lv_fn, lv.smem_blob);
-        lv_grid = require_device() * std::max(1, occupancy(lv_fn, lv_block_of(n), lv.smem_blob));
-    }
+    if (fast) allow_smem(lv_fn, lv.smem_blob);
     PathsDev<R> s{};
     if (!fast) {  // the generic kernel's inputs, in one copy
         ModelDev<R>& m = s.m;
@@ -619,9 +615,7 @@ void run_paths(ob_paths_request& h) {
         if (fast) {
             PathsLvArgs<R> la = lv;
             la.n_pairs = mcount, la.first_pair = h.first_pair + c0, la.rows = 2 * mcount, la.out = out;
-            const int lb = lv_block_of(n);
-            const unsigned g = static_cast<unsigned>(std::max<long long>(
-                1, std::min<long long>(lv_grid, (mcount + lb - 1) / lb)));
+            const auto [lb, g] = launch_shape(lv_fn, la.smem_blob, sms, mcount, lv_block_of(n));
             reinterpret_cast<void (*)(PathsLvArgs<R>)>(const_cast<void*>(lv_fn))<<<g, lb, la.smem_blob, st>>>(la);
         } else if (n <= 1) paths_kernel<R, 1><<<grid, block, 0, st>>>(part);
         else if (n <= 2) paths_kernel<R, 2><<<grid, block, 0, st>>>(part);

@@ -980,12 +980,9 @@ void run_script(const ob_script_request& rq, ob_script_result& res, const Record
                                 pick_lv<R>(n, rq.n_windows, rq.n_windows ? rq.win_func[0] : -1, rq.branch != 0, rq.n_calls > 0,
                                           lv.table_global != 0))
                           : reinterpret_cast<const void*>(pick_script<R>(mq.model, n, rq.n_windows));
-    const int block = fast ? 512 : 128;
     const size_t smem = fast ? static_cast<size_t>(lv.smem_blob) : 0;
     if (fast) allow_smem(fn, smem);
-    const int per_sm = occupancy(fn, block, smem);
-    const long long need = (mq.n_pairs + block - 1) / block;
-    const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(need, 1LL * sms * std::max(1, per_sm))));
+    const auto [block, grid] = launch_shape(fn, smem, sms, mq.n_pairs, fast ? 512 : 128);
     double* partial = arena.alloc<double>(2 * static_cast<size_t>(grid));
     double* sums = reinterpret_cast<double*>(outs + 4);
     cudaEvent_t e0, e1;
