@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __res
                             const Pair2<R>* trow = tab + static_cast<long long>(row) * (d.n_x - 1);
                             const R zd = d.sdt * zc;  // sqrt(dt) z, the legs' +-
                             R var0, var1;
-                            table_vars<true>(trow, 0u, org, inv, 0, d.top, x0[n], x1[n], var0, var1);
+                            table_vars<kTabGlobal>(trow, nullptr, 0u, org, inv, 0, d.top, x0[n], x1[n], var0, var1);
                             lv_advance_legs(x0[n], x1[n], var0, var1, d.hdt, zd);
                             lp0 = m_min(lp0, x0[n] + lf), lp1 = m_min(lp1, x1[n] + lf);
                         }

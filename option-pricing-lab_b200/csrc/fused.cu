@@ -86,7 +86,7 @@ constexpr int min_blocks() {
 }
 
 // KIND: 1 local vol (table), 2 Heston (Euler), 3 SLV (table x Heston, residuals on the aux stream), 4 Heston QE-M.
-// GT: the table is read from global memory (a.tab) instead of the stage.
+// TM: where the table is read (kTabStaged, kTabGlobal, kTabStreamed).
 // Blocks of 512 an SM the register budget allows: two in float (64 registers), one in double; one for the mixer's
 // 4- and 5-name baskets in float too, whose two legs' normals would spill at 64.
 template <typename R, int N, bool MIX>
@@ -94,9 +94,17 @@ constexpr int fused_min_blocks() {
     return MIX && N >= 4 ? 1 : min_blocks<R>();
 }
 
+// Steps per batch of whole Philox blocks. One local-vol name draws two blocks a batch (8 steps), whose two independent
+// multiply chains interleave (1.317 -> 1.300 ms for the 2^20-path Phoenix; one SLV name would draw four and spill in
+// FP64).
+constexpr int batch_steps(int n, int kind, bool mix) {
+    const int c = kind == 4 ? 2 : kind == 2 ? 2 * n : n + (mix ? 1 : 0);
+    return c == 1 && kind == 1 ? 8 : 4 / gcd4(c);
+}
+
 // MIX (local vol, 2 to 5 names): the local-correlation mixer, one more normal a step after the names'.
-template <typename R, int N, int KIND, int PRODUCT, bool GT = false, bool MIX = false>
-__global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
+template <typename R, int N, int KIND, int PRODUCT, int TM = kTabStaged, bool MIX = false>
+__global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM == kTabStreamed ? 1 : fused_min_blocks<R, N, MIX>())
     fused_kernel(FusedArgs<R> a, long long n_pairs, long long first_pair, uint32_t k0, uint32_t k1,
                  double* __restrict__ partial) {
     constexpr bool QE = KIND == 4;
@@ -105,10 +113,7 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
     static_assert(!MIX || (KIND == 1 && N >= 2), "the mixer runs local-vol baskets");
     constexpr int C = QE ? 2 : (KIND == 2 ? 2 * N : N + (MIX ? 1 : 0));  // normals per step, stream 0
     constexpr int CA = KIND == 3 ? N : 0;                // normals per step, aux stream
-    // steps per batch of whole Philox blocks; one local-vol name draws two blocks a batch (8 steps), whose two
-    // independent multiply chains interleave (1.317 -> 1.300 ms for the 2^20-path Phoenix; one SLV name would draw four
-    // and spill in FP64)
-    constexpr int G = C == 1 && KIND == 1 ? 8 : 4 / gcd4(C);
+    constexpr int G = batch_steps(N, KIND, MIX);
     constexpr int NB = C * G / 4, NBA = CA * G / 4;
 
     extern __shared__ __align__(16) unsigned char sm[];
@@ -119,15 +124,18 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
     }
     const int n_warps = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_acc = 2 * a.n_out;
-    double* wacc = reinterpret_cast<double*>(sm + a.smem_blob);
+    double* wacc = reinterpret_cast<double*>(sm + a.smem_acc);
     for (int t = threadIdx.x; t < n_warps * n_acc; t += blockDim.x) wacc[t] = 0.0;
     __syncthreads();
     const StepRec<R>* s_step = reinterpret_cast<const StepRec<R>*>(sm + a.off.step);
     const NameStep<R>* s_ns = reinterpret_cast<const NameStep<R>*>(sm + a.off.name_step);
     const R* s_root = reinterpret_cast<const R*>(sm + a.off.root);
     const R* s_hes = reinterpret_cast<const R*>(sm + a.off.hes);
-    const Pair2<R>* s_tab = GT ? a.tab : reinterpret_cast<const Pair2<R>*>(sm + a.off.table2);
-    const uint32_t tab_s = shared_address<GT || !TABLE>(s_tab);
+    const Pair2<R>* s_tab = TM == kTabStaged ? reinterpret_cast<const Pair2<R>*>(sm + a.off.table2) : a.tab;
+    const uint32_t tab_s = TM == kTabStreamed ? static_cast<uint32_t>(a.rs.off)
+                                              : shared_address<TABLE && TM == kTabStaged>(s_tab);
+    RowStream<R, N, G> rows(a.rs, a.tab, s_ns, sm, a.n_steps);
+    if (TM == kTabStreamed) rows.first();
     const R* s_trig = reinterpret_cast<const R*>(sm + a.off.ln_trig);
     const double* s_disc = reinterpret_cast<const double*>(sm + a.off.obs_disc);
     const int S = a.n_steps;
@@ -138,8 +146,9 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
     for (int k = 0; k < (kRootRegs ? N * N : 0); ++k) rt[k] = s_root[k];
 
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long base = static_cast<long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); base < n_pairs;
-         base += stride) {
+    for (long long block0 = static_cast<long long>(blockIdx.x) * blockDim.x; block0 < n_pairs; block0 += stride) {
+        const long long base = block0 + (threadIdx.x & ~31);
+        if (TM != kTabStreamed && base >= n_pairs) break;  // (a streaming block's warps keep together)
         const bool active = base + lane < n_pairs;
         const uint64_t pair = static_cast<uint64_t>(first_pair + (active ? base + lane : n_pairs - 1));
         R x0[N], x1[N], v0[N], v1[N];
@@ -156,6 +165,7 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
         // without an observation run without testing each step for one (OBS false).
         auto run_batch = [&](int i0, int batch, auto check, auto observe) {
             constexpr bool CHECK = decltype(check)::value, OBS = decltype(observe)::value;
+            if (TM == kTabStreamed && rows.opens(batch)) rows.turn(batch, block0 + stride < n_pairs);
             R z[C * G];
             R za[CA > 0 ? CA * G : 1];
             R q0 = R(0), q1 = R(0);
@@ -245,7 +255,8 @@ __global__ void __launch_bounds__(512, (fused_min_blocks<R, N, MIX>()))
                         if (VAR) vp0 = m_max(v0[n], R(0)), vp1 = m_max(v1[n], R(0));
                         if (TABLE) {
                             R t0, t1;
-                            table_vars<GT>(s_tab, tab_s, ns.org, ns.inv_dx, ns.row, a.top, x0[n], x1[n], t0, t1);
+                            table_vars<TM>(s_tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i, n) : ns.row,
+                                           a.top, x0[n], x1[n], t0, t1);
                             var0 = KIND == 1 ? t0 : t0 * vp0, var1 = KIND == 1 ? t1 : t1 * vp1;
                         } else if (VAR) {
                             var0 = vp0, var1 = vp1;
@@ -342,7 +353,7 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
     }
     const int n_warps = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_acc = 2 * a.n_out;
-    double* wacc = reinterpret_cast<double*>(sm + a.smem_blob);
+    double* wacc = reinterpret_cast<double*>(sm + a.smem_acc);
     for (int t = threadIdx.x; t < n_warps * n_acc; t += blockDim.x) wacc[t] = 0.0;
     __syncthreads();
     const StepRec<R>* s_step = reinterpret_cast<const StepRec<R>*>(sm + a.off.step);
@@ -457,38 +468,47 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
 template <typename R>
 using FusedFn = void (*)(FusedArgs<R>, long long, long long, uint32_t, uint32_t, double*);
 
-template <typename R, int KIND, int PRODUCT, bool GT>
+template <typename R, int KIND, int PRODUCT, int TM>
 FusedFn<R> pick_n(int n) {
-    if (n == 1) return fused_kernel<R, 1, KIND, PRODUCT, GT>;
-    if (n == 2) return fused_kernel<R, 2, KIND, PRODUCT, GT>;
-    if (n == 3) return fused_kernel<R, 3, KIND, PRODUCT, GT>;
-    if constexpr (KIND == 1 || KIND == 0) {
-        if (n == 4) return fused_kernel<R, 4, KIND, PRODUCT, GT>;
-        if (n == 5) return fused_kernel<R, 5, KIND, PRODUCT, GT>;
+    if (n == 1) return fused_kernel<R, 1, KIND, PRODUCT, TM>;
+    if (n == 2) return fused_kernel<R, 2, KIND, PRODUCT, TM>;
+    if (n == 3) return fused_kernel<R, 3, KIND, PRODUCT, TM>;
+    if constexpr ((KIND == 1 || KIND == 0) && TM != kTabStreamed) {
+        if (n == 4) return fused_kernel<R, 4, KIND, PRODUCT, TM>;
+        if (n == 5) return fused_kernel<R, 5, KIND, PRODUCT, TM>;
     }
     return nullptr;
 }
 
 // Local-vol baskets of 2 to 5 names with the local-correlation mixer.
-template <typename R, int PRODUCT, bool GT>
+template <typename R, int PRODUCT, int TM>
 FusedFn<R> pick_mix(int n) {
     switch (n) {
-        case 2: return fused_kernel<R, 2, 1, PRODUCT, GT, true>;
-        case 3: return fused_kernel<R, 3, 1, PRODUCT, GT, true>;
-        case 4: return fused_kernel<R, 4, 1, PRODUCT, GT, true>;
-        case 5: return fused_kernel<R, 5, 1, PRODUCT, GT, true>;
+        case 2: return fused_kernel<R, 2, 1, PRODUCT, TM, true>;
+        case 3: return fused_kernel<R, 3, 1, PRODUCT, TM, true>;
+        case 4: return fused_kernel<R, 4, 1, PRODUCT, TM, true>;
+        case 5: return fused_kernel<R, 5, 1, PRODUCT, TM, true>;
         default: return nullptr;
     }
 }
 
-// table_global: the kinds with a table (local vol, SLV) read it from global memory.
+// tm: where the kinds with a table (local vol, SLV) read it; rows are streamed for one to three local-vol names in
+// float (in double the arithmetic bounds the step, not the table's reads).
 template <typename R, int PRODUCT>
-FusedFn<R> pick_fused(int kind, int n, bool table_global) {
+FusedFn<R> pick_fused(int kind, int n, int tm, bool mix) {
+    if (tm == kTabStreamed) {
+        if constexpr (sizeof(R) == 4)
+            if (kind == 1 && !mix) return pick_n<R, 1, PRODUCT, kTabStreamed>(n);
+        return nullptr;
+    }
+    const bool global = tm == kTabGlobal;
+    if (mix)
+        return kind != 1 ? nullptr : global ? pick_mix<R, PRODUCT, kTabGlobal>(n) : pick_mix<R, PRODUCT, kTabStaged>(n);
     switch (kind) {
-        case 0: return table_global ? nullptr : pick_n<R, 0, PRODUCT, false>(n);
-        case 1: return table_global ? pick_n<R, 1, PRODUCT, true>(n) : pick_n<R, 1, PRODUCT, false>(n);
-        case 2: return pick_n<R, 2, PRODUCT, false>(n);
-        case 3: return table_global ? pick_n<R, 3, PRODUCT, true>(n) : pick_n<R, 3, PRODUCT, false>(n);
+        case 0: return global ? nullptr : pick_n<R, 0, PRODUCT, kTabStaged>(n);
+        case 1: return global ? pick_n<R, 1, PRODUCT, kTabGlobal>(n) : pick_n<R, 1, PRODUCT, kTabStaged>(n);
+        case 2: return pick_n<R, 2, PRODUCT, kTabStaged>(n);
+        case 3: return global ? pick_n<R, 3, PRODUCT, kTabGlobal>(n) : pick_n<R, 3, PRODUCT, kTabStaged>(n);
         case 4: return n == 1 ? qe_pair_kernel<R, PRODUCT> : nullptr;
         default: return nullptr;
     }
@@ -528,16 +548,11 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
             if (rq.kind[a] != kind) return false;
     }
     if (rq.mixer && kind != 1) return false;  // the mixer beside other kinds: the generic kernel
-    auto pick = [&](bool table_global) -> FusedFn<R> {
-        const bool ladder = rq.product == OB_PRODUCT_LADDER;
-        if (rq.mixer)
-            return ladder ? (table_global ? pick_mix<R, OB_PRODUCT_LADDER, true>(n) : pick_mix<R, OB_PRODUCT_LADDER, false>(n))
-                          : (table_global ? pick_mix<R, OB_PRODUCT_AUTOCALL, true>(n)
-                                          : pick_mix<R, OB_PRODUCT_AUTOCALL, false>(n));
-        return ladder ? pick_fused<R, OB_PRODUCT_LADDER>(kind, n, table_global)
-                      : pick_fused<R, OB_PRODUCT_AUTOCALL>(kind, n, table_global);
+    auto pick = [&](int tm) -> FusedFn<R> {
+        return rq.product == OB_PRODUCT_LADDER ? pick_fused<R, OB_PRODUCT_LADDER>(kind, n, tm, rq.mixer != 0)
+                                               : pick_fused<R, OB_PRODUCT_AUTOCALL>(kind, n, tm, rq.mixer != 0);
     };
-    if (!pick(false)) return false;
+    if (!pick(kTabStaged)) return false;
     FusedArgs<R> a{};
     a.n_steps = S, a.n_x = rq.n_x, a.same = rq.same;
     a.n_obs = rq.product == OB_PRODUCT_AUTOCALL ? rq.n_obs : 0;
@@ -579,7 +594,7 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
                 if (table) {
                     const int row = rq.step_row[static_cast<size_t>(k) * S + (i - 1)];
                     set_cell_row(r, rq.row_lo[row], rq.row_inv_dx[row], a.top);
-                    r.row = row * (rq.n_x - 1);
+                    r.row = row;  // (the row's first cell, once it is known where the table goes)
                 }
             }
         a.off.name_step = blob.put(ns);
@@ -629,25 +644,37 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
         a.ln_ki = rq.ki_barrier > 0 ? static_cast<R>(std::log(rq.ki_barrier)) : R(-1e30);
         a.coupon = rq.coupon, a.put_strike = rq.put_strike, a.memory = rq.memory, a.ki_daily = rq.ki_daily;
     }
-    const int block = 512;
-    const size_t acc_bytes = static_cast<size_t>(block / 32) * 2 * a.n_out * sizeof(double);
+    int block = 512;
+    auto acc_bytes = [&](int b) { return static_cast<size_t>(b / 32) * 2 * a.n_out * sizeof(double); };
     const size_t budget = sizeof(R) == 4 ? (110u << 10) : (220u << 10);  // two blocks a SM in float, one in double
-    bool table_global = false;
+    auto aligned = [&] { return (blob.bytes.size() + 15) & ~static_cast<size_t>(15); };
+    int tm = kTabStaged;
+    size_t end = 0;  // of the blob and the ring
     if (table) {
-        const size_t cells = table_cells(rq.n_rows, rq.n_x);
-        const size_t at = (blob.bytes.size() + 15) & ~static_cast<size_t>(15);
-        table_global = at + cells * sizeof(Pair2<R>) + acc_bytes > budget;
-        if (table_global) {
+        const size_t cells = static_cast<size_t>(rq.n_rows) * (rq.n_x - 1);
+        if (aligned() + cells * sizeof(Pair2<R>) + acc_bytes(block) > budget) {
+            constexpr size_t kStreamBudget = 220u << 10;  // one block an SM
+            const int G = batch_steps(n, kind, false);
+            tm = pick(kTabStreamed) && streams_rows(n, rq.n_pairs, plan.sms) &&
+                         plan_row_stream<R>(a.rs, rq.n_x, n, G, aligned(), kStreamBudget - acc_bytes(1024))
+                     ? kTabStreamed
+                     : kTabGlobal;
+            if (tm == kTabStreamed) block = 1024, end = a.rs.off + row_stream_bytes(a.rs, n, G);
             a.tab = upload_table<R>(plan.arena, rq.table, rq.n_rows, rq.n_x);
         } else {
             a.off.table2 = blob.put<Pair2<R>>(nullptr, cells);
-            pack_table<R>(rq.table, rq.n_x, 0, cells, reinterpret_cast<Pair2<R>*>(blob.bytes.data() + a.off.table2));
+            pack_table<R>(rq.table, rq.n_x, rq.n_x - 1, 0, cells,
+                          reinterpret_cast<Pair2<R>*>(blob.bytes.data() + a.off.table2));
         }
+        NameStep<R>* ns = reinterpret_cast<NameStep<R>*>(blob.bytes.data() + a.off.name_step);
+        for (size_t k = 0; k < static_cast<size_t>(S) * n; ++k)
+            ns[k].row *= tm == kTabStaged ? rq.n_x - 1 : table_pitch<R>(rq.n_x);
     }
-    const FusedFn<R> fn = pick(table_global);
-    a.smem_blob = static_cast<int>((blob.bytes.size() + 15) & ~static_cast<size_t>(15));
-    const size_t smem = a.smem_blob + acc_bytes;
-    if (smem > budget) return false;
+    const FusedFn<R> fn = pick(tm);
+    a.smem_blob = static_cast<int>(aligned());
+    if (static_cast<size_t>(a.smem_blob) + acc_bytes(512) > budget) return false;
+    a.smem_acc = static_cast<int>(std::max(aligned(), end));
+    const size_t smem = a.smem_acc + acc_bytes(block);
     unsigned char* d = plan.arena.alloc<unsigned char>(std::max<size_t>(16, blob.bytes.size()));
     check_cuda(cudaMemcpy(d, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice), "copy blob");
     a.blob = d;

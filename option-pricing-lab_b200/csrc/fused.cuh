@@ -164,15 +164,20 @@ __device__ __forceinline__ Pair2<double> ldg_pair(const Pair2<double>* p) {
     return {v.x, v.y};
 }
 
+// Where a kernel reads its table: the stage, global memory, or rows streamed through a ring in shared memory.
+constexpr int kTabStaged = 0, kTabGlobal = 1, kTabStreamed = 2;
+
 // The local variances of both legs of a pair at x0 and x1 in a step's row of the table: table_cell of each leg and one
-// load and multiply-add each. GLOBAL: tab is in global memory (ldg_pair); else in shared memory, tab_s its shared
-// address. Float: the cell's last three operations packed, and the interval's address straight from the bits of
-// s top + 2^23, one shift-and-add with the offset 2^23's own bits leave (0x4B000000, times 8 modulo 2^32) folded into
-// the row's address. (The shared load has no memory clobber: its address depends on the row read after the barrier
-// that follows the staging, and nothing writes the table after it.)
-template <bool GLOBAL>
-__device__ __forceinline__ void table_vars(const Pair2<float>* tab, uint32_t tab_s, float org, float inv, int row,
-                                           float top, float x0, float x1, float& var0, float& var1) {
+// load and multiply-add each. MODE kTabStaged: the table is staged in shared memory, at shared address tab_s; kTabGlobal: in global memory
+// (ldg_pair); kTabStreamed: the row is in a ring in the dynamic shared memory sm, tab_s its offset there. Float: the cell's last three
+// operations packed, and the interval's address straight from the bits of s top + 2^23, one shift-and-add with the offset
+// 2^23's own bits leave (0x4B000000, times 8 modulo 2^32) folded into the row's address. (The staged load has no memory
+// clobber: its address depends on the row read after the barrier that follows the staging, and nothing writes the table
+// after it. A ring is rewritten, so its loads are plain ones, which no barrier lets pass.)
+template <int MODE>
+__device__ __forceinline__ void table_vars(const Pair2<float>* tab, const unsigned char* sm, uint32_t tab_s, float org,
+                                           float inv, int row, float top, float x0, float x1, float& var0,
+                                           float& var1) {
     float s0, s1, b0, b1, f0, f1;
     asm("fma.rn.ftz.sat.f32 %0, %1, %2, %3;" : "=f"(s0) : "f"(x0), "f"(inv), "f"(org));
     asm("fma.rn.ftz.sat.f32 %0, %1, %2, %3;" : "=f"(s1) : "f"(x1), "f"(inv), "f"(org));
@@ -182,30 +187,37 @@ __device__ __forceinline__ void table_vars(const Pair2<float>* tab, uint32_t tab
     unpack2(fma2(s, t, fma2(big, pack2(-1.0f, -1.0f), two23)), f0, f1);  // (2^23 - big is exact)
     const uint32_t i0 = __float_as_uint(b0), i1 = __float_as_uint(b1);
     Pair2<float> y0, y1;
-    if (GLOBAL) {
+    if (MODE == kTabGlobal) {
         y0 = ldg_pair(tab + row + static_cast<int>(i0 - 0x4B000000u));
         y1 = ldg_pair(tab + row + static_cast<int>(i1 - 0x4B000000u));
     } else {
         const uint32_t base = tab_s + 8u * static_cast<uint32_t>(row) - 8u * 0x4B000000u;
-        asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(y0.a), "=f"(y0.b) : "r"(i0 * 8u + base));
-        asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(y1.a), "=f"(y1.b) : "r"(i1 * 8u + base));
+        if (MODE == kTabStaged) {
+            asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(y0.a), "=f"(y0.b) : "r"(i0 * 8u + base));
+            asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(y1.a), "=f"(y1.b) : "r"(i1 * 8u + base));
+        } else {
+            y0 = *reinterpret_cast<const Pair2<float>*>(sm + (i0 * 8u + base));
+            y1 = *reinterpret_cast<const Pair2<float>*>(sm + (i1 * 8u + base));
+        }
     }
     var0 = fmaf(f0, y0.b, y0.a), var1 = fmaf(f1, y1.b, y1.a);
 }
-template <bool GLOBAL>
-__device__ __forceinline__ void table_vars(const Pair2<double>* tab, uint32_t, double org, double inv, int row,
-                                           double top, double x0, double x1, double& var0, double& var1) {
+template <int MODE>
+__device__ __forceinline__ void table_vars(const Pair2<double>* tab, const unsigned char* sm, uint32_t tab_s,
+                                           double org, double inv, int row, double top, double x0, double x1,
+                                           double& var0, double& var1) {
     int j0, j1;
     double f0, f1;
     table_cell(org, inv, top, x0, j0, f0), table_cell(org, inv, top, x1, j1, f1);
-    const Pair2<double> y0 = GLOBAL ? ldg_pair(tab + row + j0) : tab[row + j0];
-    const Pair2<double> y1 = GLOBAL ? ldg_pair(tab + row + j1) : tab[row + j1];
+    if (MODE == kTabStreamed) tab = reinterpret_cast<const Pair2<double>*>(sm + tab_s);
+    const Pair2<double> y0 = MODE == kTabGlobal ? ldg_pair(tab + row + j0) : tab[row + j0];
+    const Pair2<double> y1 = MODE == kTabGlobal ? ldg_pair(tab + row + j1) : tab[row + j1];
     var0 = y0.a + f0 * y0.b, var1 = y1.a + f1 * y1.b;
 }
-// The shared-memory address of p (0 where the table is left in global memory).
-template <bool GLOBAL>
+// The shared-memory address of p (0 unless the table is staged there).
+template <bool STAGED>
 __device__ __forceinline__ uint32_t shared_address(const void* p) {
-    return GLOBAL ? 0u : static_cast<uint32_t>(__cvta_generic_to_shared(p));
+    return STAGED ? static_cast<uint32_t>(__cvta_generic_to_shared(p)) : 0u;
 }
 
 // A record of whole 16-byte words (StepRec, NameStep) read from global memory through the read-only data cache: the
@@ -229,6 +241,15 @@ struct alignas(16) StepRec {
     int obs;
 };
 
+// A ring of streamed rows (row_stream.cuh).
+struct RowStreamArgs {
+    int batches;  // batches of steps a stage
+    int pitch;    // intervals from one row to the next, a whole number of 16-byte words
+    int chunks;   // 16-byte words a row
+    unsigned inv; // 2^32 / chunks, rounded up: c / chunks = c inv >> 32 for the c of a stage
+    int off;      // the ring's offset in shared memory (two stages)
+};
+
 // Byte offsets inside the staged blob.
 struct FusedOffsets {
     int step, name_step, root, hes, table2, ln_trig, obs_disc, leg_type, leg_strike, leg_barrier, ln_level;
@@ -241,6 +262,7 @@ struct FusedArgs {
     FusedOffsets off;
     const unsigned char* blob;
     int smem_blob;
+    int smem_acc;  // the warps' sums, after the blob and the ring
     int n_steps, n_obs, n_out, n_legs, n_x, same;
     R top;  // n_x - 1 - 1e-4, the clamp of the table interpolation
     QeConsts<R> qe;
@@ -249,7 +271,8 @@ struct FusedArgs {
     int has_coupon, memory, ki_daily;
     R ln_cb, ln_ki;
     double coupon, put_strike;
-    const Pair2<R>* tab;  // the table in global memory when it does not fit the stage (kernels with GT), else unused
+    const Pair2<R>* tab;  // the table in global memory (kTabGlobal, kTabStreamed), else unused
+    RowStreamArgs rs;     // kTabStreamed
     // local correlation (kernels with MIX): w0 + level, down, up, sign, cos, sin of the mixer (paths.hpp:219-237)
     R mix_base, mix_down, mix_up, mix_sign, mix_cos, mix_sin;
 };

@@ -109,8 +109,10 @@ struct PathsLvArgs {
     uint32_t k0, k1;
     R top;
     R* out;
-    const Pair2<R>* tab;  // the table in global memory when it does not fit the stage (table_global), else unused
-    int table_global;
+    const Pair2<R>* tab;  // the table in global memory (kTabGlobal, kTabStreamed), else unused
+    int tm;               // where the table is read
+    RowStreamArgs rs;     // kTabStreamed
+    int smem;             // bytes of dynamic shared memory
     int kind, same;  // the names' model kind (0 Black-Scholes, 1 local vol, 2 Heston, 3 SLV); residuals through the root
     int mixer;       // local correlation (kernels with MIX): w0 + level, down, up, sign, cos, sin of the mixer
     R mix_base, mix_down, mix_up, mix_sign, mix_cos, mix_sin;
@@ -152,23 +154,30 @@ __device__ __forceinline__ void lv_record(const PathsLvArgs<R>& a, const int* s_
 }
 
 // 512-thread blocks for one or two names, 256 for more (registers); one float name fits two blocks an SM (32 warps).
-template <int N>
+// A block that streams its rows (one name) has an SM to itself.
+template <int N, int TM>
 constexpr int lv_block() {
-    return N <= 2 ? 512 : 256;
+    return TM == kTabStreamed ? 1024 : N <= 2 ? 512 : 256;
+}
+
+// Steps per batch of whole Philox blocks.
+constexpr int paths_batch_steps(int n, int kind, bool mix) {
+    const int c = kind == 2 ? 2 * n : n + (mix ? 1 : 0);
+    return c % 4 == 0 ? 1 : (c % 2 == 0 ? 2 : 4);
 }
 
 // KIND: 0 Black-Scholes (constant variance), 1 local vol (table), 2 Heston (Euler), 3 SLV (table x Heston, residuals
-// on the aux stream). GT: the table is read from global memory (a.tab) instead of the stage. MIX (Black-Scholes or
+// on the aux stream). TM: where the table is read (kTabStaged, kTabGlobal, kTabStreamed). MIX (Black-Scholes or
 // local vol, 2 to 5 names): the local-correlation mixer, one more normal a step after the names'.
-template <typename R, int N, int KIND, bool GT, bool MIX = false>
-__global__ void __launch_bounds__(lv_block<N>(), N == 1 && sizeof(R) == 4 ? 2 : 1)
+template <typename R, int N, int KIND, int TM, bool MIX = false>
+__global__ void __launch_bounds__(lv_block<N, TM>(), TM != kTabStreamed && N == 1 && sizeof(R) == 4 ? 2 : 1)
     paths_staged_kernel(PathsLvArgs<R> a) {
     constexpr bool VAR = KIND == 2 || KIND == 3;
     constexpr bool TABLE = KIND == 1 || KIND == 3;
     static_assert(!MIX || (KIND <= 1 && N >= 2), "the staged mixer runs Black-Scholes and local-vol baskets");
     constexpr int C = KIND == 2 ? 2 * N : N + (MIX ? 1 : 0);  // normals per step, stream 0
     constexpr int CA = KIND == 3 ? N : 0;     // normals per step, aux stream
-    constexpr int G = C % 4 == 0 ? 1 : (C % 2 == 0 ? 2 : 4);  // steps per batch of whole Philox blocks
+    constexpr int G = paths_batch_steps(N, KIND, MIX);
     constexpr int NB = C * G / 4, NBA = CA * G / 4;
     extern __shared__ __align__(16) unsigned char sm[];
     {
@@ -182,16 +191,20 @@ __global__ void __launch_bounds__(lv_block<N>(), N == 1 && sizeof(R) == 4 ? 2 : 
     const R* s_root = reinterpret_cast<const R*>(sm + a.off.root);
     // per name: v0, kappa, theta, xi, rho, sqrt(1 - rho^2), the constant variance (Black-Scholes)
     const R* s_hes = reinterpret_cast<const R*>(sm + a.off.hes);
-    const Pair2<R>* tab = GT ? a.tab : reinterpret_cast<const Pair2<R>*>(sm + a.off.table2);
-    const uint32_t tab_s = shared_address<GT || !TABLE>(tab);
+    const Pair2<R>* tab = TM == kTabStaged ? reinterpret_cast<const Pair2<R>*>(sm + a.off.table2) : a.tab;
+    const uint32_t tab_s = TM == kTabStreamed ? static_cast<uint32_t>(a.rs.off)
+                                              : shared_address<TABLE && TM == kTabStaged>(tab);
+    RowStream<R, N, G> rows(a.rs, a.tab, s_ns, sm, a.n_steps);
+    if (TM == kTabStreamed) rows.first();
     const int2* s_sched = reinterpret_cast<const int2*>(sm + a.off.sched);  // observations [x, y) at each step end
     const int* s_col = reinterpret_cast<const int*>(sm + a.off.col);
     const R* s_fwd = reinterpret_cast<const R*>(sm + a.off.fwd);
     const int S = a.n_steps;
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long base = static_cast<long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); base < a.n_pairs;
-         base += stride) {
+    for (long long block0 = static_cast<long long>(blockIdx.x) * blockDim.x; block0 < a.n_pairs; block0 += stride) {
         const int lane = threadIdx.x & 31;
+        const long long base = block0 + (threadIdx.x & ~31);
+        if (TM != kTabStreamed && base >= a.n_pairs) break;  // (a streaming block's warps keep together)
         const bool active = base + lane < a.n_pairs;
         const long long p = active ? base + lane : a.n_pairs - 1;
         const uint64_t pair = static_cast<uint64_t>(a.first_pair + p);
@@ -205,6 +218,7 @@ __global__ void __launch_bounds__(lv_block<N>(), N == 1 && sizeof(R) == 4 ? 2 : 
         }
         for (int j = s_sched[0].x; j < s_sched[0].y; ++j) lv_record<R, N>(a, s_col, s_fwd, j, p, active, x0, x1, lo, hi);
         for (int i0 = 1, b = 0; i0 <= S; i0 += G, ++b) {
+            if (TM == kTabStreamed && rows.opens(b)) rows.turn(b, block0 + stride < a.n_pairs);
             R z[C * G];
             R za[CA > 0 ? CA * G : 1];
 #pragma unroll
@@ -275,7 +289,8 @@ __global__ void __launch_bounds__(lv_block<N>(), N == 1 && sizeof(R) == 4 ? 2 : 
                     if (VAR) vp0 = m_max(v0[n], R(0)), vp1 = m_max(v1[n], R(0));
                     if (TABLE) {
                         R t0, t1;
-                        table_vars<GT>(tab, tab_s, ns.org, ns.inv_dx, ns.row, a.top, x0[n], x1[n], t0, t1);
+                        table_vars<TM>(tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i, n) : ns.row,
+                                       a.top, x0[n], x1[n], t0, t1);
                         var0 = KIND == 1 ? t0 : t0 * vp0, var1 = KIND == 1 ? t1 : t1 * vp1;
                     } else if (VAR) {
                         var0 = vp0, var1 = vp1;
@@ -343,13 +358,20 @@ void check_request(const ob_paths_request& c) {
         if (c.win_lo[w] < 0 || c.win_hi[w] < c.win_lo[w] || c.win_hi[w] >= c.n_obs) invalid("bad window");
 }
 
+// The requests whose rows may be streamed: one local-vol name in float (two names measured no faster: 290 to 310 us at
+// 2^15 pairs, 368 to 323 at 2^16).
+template <typename R>
+constexpr bool streams_paths(int n, int kind, bool mixer) {
+    return sizeof(R) == 4 && kind == 1 && n == 1 && !mixer;
+}
+
 // The staged blob of paths_staged_kernel, or false when the request is not for it (names of different kinds, a
 // mixer, more than five Black-Scholes / local-vol or three Heston / SLV names, or a blob beyond the shared-memory
 // budget: 110 KB in float, 200 KB in double, without the table). The table goes into the stage when it fits beside
 // the rest, else into global memory: a plan's per-step rows (801 points for each of the 756 steps of three daily
 // years, 4.8 MB in float) stay in L2 and are read through the read-only cache.
 template <typename R>
-bool pack_paths_staged(const ob_paths_request& h, DeviceArena& arena, PathsLvArgs<R>& a) {
+bool pack_paths_staged(const ob_paths_request& h, long long chunk, int sms, DeviceArena& arena, PathsLvArgs<R>& a) {
     const int n = h.n_names, S = h.n_steps, kind = h.kind[0];
     if (S < 1 || kind < 0 || kind > 3 || n > (kind <= 1 ? 5 : 3)) return false;
     if (h.mixer && (kind > 1 || n < 2)) return false;  // the mixer beside Heston or SLV names: the generic kernel
@@ -380,7 +402,7 @@ bool pack_paths_staged(const ob_paths_request& h, DeviceArena& arena, PathsLvArg
             if (!table) continue;
             const int row = h.step_row[static_cast<size_t>(k) * S + i];
             set_cell_row(r, h.row_lo[row], h.row_inv_dx[row], a.top);
-            r.row = row * (h.n_x - 1);
+            r.row = row;  // (the row's first cell, once it is known where the table goes)
         }
     a.off.name_step = put(ns.data(), ns.size() * sizeof(NameStep<R>));
     std::vector<R> root(static_cast<size_t>(n) * n);
@@ -416,18 +438,31 @@ bool pack_paths_staged(const ob_paths_request& h, DeviceArena& arena, PathsLvArg
     std::vector<R> fwd(static_cast<size_t>(n) * h.n_obs);
     for (size_t k = 0; k < fwd.size(); ++k) fwd[k] = static_cast<R>(h.fwd[k]);
     a.off.fwd = put(fwd.data(), fwd.size() * sizeof(R));
+    // two blocks an SM for one float name, else one (a table that one block an SM still holds is staged for those too)
     const size_t budget = sizeof(R) == 4 ? (110u << 10) : (200u << 10);
-    const size_t cells = table ? table_cells(h.n_rows, h.n_x) : 0;
+    const size_t cells = table ? static_cast<size_t>(h.n_rows) * (h.n_x - 1) : 0;
     if (blob.size() > budget) return false;
-    a.table_global = ((blob.size() + 15) & ~static_cast<size_t>(15)) + cells * sizeof(Pair2<R>) > budget;
-    if (a.table_global) {
+    const size_t at = (blob.size() + 15) & ~static_cast<size_t>(15);
+    a.tm = at + cells * sizeof(Pair2<R>) > (n == 1 ? budget : size_t(200) << 10) ? kTabGlobal : kTabStaged;
+    if (a.tm == kTabGlobal) {
+        const int G = paths_batch_steps(n, kind, false);
+        if (streams_paths<R>(n, kind, h.mixer != 0) && streams_rows(n, chunk, sms) &&
+            plan_row_stream<R>(a.rs, h.n_x, n, G, at, 220u << 10)) {
+            a.tm = kTabStreamed;
+            a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
+        }
         a.tab = upload_table<R>(arena, h.table, h.n_rows, h.n_x);
-    } else {
+    } else if (cells) {
         a.off.table2 = put(nullptr, cells * sizeof(Pair2<R>));
-        if (cells)
-            pack_table<R>(h.table, h.n_x, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));
+        pack_table<R>(h.table, h.n_x, h.n_x - 1, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));
+    }
+    if (table) {
+        NameStep<R>* step_ns = reinterpret_cast<NameStep<R>*>(blob.data() + a.off.name_step);
+        for (size_t k = 0; k < static_cast<size_t>(S) * n; ++k)
+            step_ns[k].row *= a.tm == kTabStaged ? h.n_x - 1 : table_pitch<R>(h.n_x);
     }
     a.smem_blob = static_cast<int>(blob.size());
+    if (a.tm != kTabStreamed) a.smem = a.smem_blob;
     a.blob = arena.put<unsigned char>(blob.data(), blob.size());
     a.n_steps = S, a.n_obs = h.n_obs, a.n_cols = h.n_cols, a.n_keep = h.n_keep, a.n_win = h.n_windows;
     for (int w = 0; w < 2; ++w) {
@@ -438,45 +473,52 @@ bool pack_paths_staged(const ob_paths_request& h, DeviceArena& arena, PathsLvArg
     return true;
 }
 
-inline int lv_block_of(int n) { return n <= 2 ? lv_block<1>() : lv_block<3>(); }
+inline int lv_block_of(int n, int tm) {
+    return tm == kTabStreamed ? lv_block<1, kTabStreamed>() : n <= 2 ? lv_block<1, kTabStaged>() : lv_block<3, kTabStaged>();
+}
 
-template <typename R, int KIND, bool GT>
+template <typename R, int KIND, int TM>
 const void* pick_paths_n(int n) {
     switch (n) {
-        case 1: return reinterpret_cast<const void*>(paths_staged_kernel<R, 1, KIND, GT>);
-        case 2: return reinterpret_cast<const void*>(paths_staged_kernel<R, 2, KIND, GT>);
-        case 3: return reinterpret_cast<const void*>(paths_staged_kernel<R, 3, KIND, GT>);
+        case 1: return reinterpret_cast<const void*>(paths_staged_kernel<R, 1, KIND, TM>);
+        case 2: return reinterpret_cast<const void*>(paths_staged_kernel<R, 2, KIND, TM>);
+        case 3: return reinterpret_cast<const void*>(paths_staged_kernel<R, 3, KIND, TM>);
     }
     if constexpr (KIND <= 1) {
-        if (n == 4) return reinterpret_cast<const void*>(paths_staged_kernel<R, 4, KIND, GT>);
-        if (n == 5) return reinterpret_cast<const void*>(paths_staged_kernel<R, 5, KIND, GT>);
+        if (n == 4) return reinterpret_cast<const void*>(paths_staged_kernel<R, 4, KIND, TM>);
+        if (n == 5) return reinterpret_cast<const void*>(paths_staged_kernel<R, 5, KIND, TM>);
     }
     return nullptr;
 }
 
-template <typename R, int KIND, bool GT>
+template <typename R, int KIND, int TM>
 const void* pick_paths_mix(int n) {
     switch (n) {
-        case 2: return reinterpret_cast<const void*>(paths_staged_kernel<R, 2, KIND, GT, true>);
-        case 3: return reinterpret_cast<const void*>(paths_staged_kernel<R, 3, KIND, GT, true>);
-        case 4: return reinterpret_cast<const void*>(paths_staged_kernel<R, 4, KIND, GT, true>);
-        case 5: return reinterpret_cast<const void*>(paths_staged_kernel<R, 5, KIND, GT, true>);
+        case 2: return reinterpret_cast<const void*>(paths_staged_kernel<R, 2, KIND, TM, true>);
+        case 3: return reinterpret_cast<const void*>(paths_staged_kernel<R, 3, KIND, TM, true>);
+        case 4: return reinterpret_cast<const void*>(paths_staged_kernel<R, 4, KIND, TM, true>);
+        case 5: return reinterpret_cast<const void*>(paths_staged_kernel<R, 5, KIND, TM, true>);
         default: return nullptr;
     }
 }
 
 template <typename R>
-const void* pick_paths_staged(int n, int kind, bool table_global, bool mixer) {
+const void* pick_paths_staged(int n, int kind, int tm, bool mixer) {
+    const bool global = tm == kTabGlobal;
+    if (tm == kTabStreamed) {
+        if constexpr (sizeof(R) == 4) return reinterpret_cast<const void*>(paths_staged_kernel<R, 1, 1, kTabStreamed>);
+        return nullptr;
+    }
     if (mixer) {
-        if (kind == 0) return pick_paths_mix<R, 0, false>(n);
-        if (kind == 1) return table_global ? pick_paths_mix<R, 1, true>(n) : pick_paths_mix<R, 1, false>(n);
+        if (kind == 0) return pick_paths_mix<R, 0, kTabStaged>(n);
+        if (kind == 1) return global ? pick_paths_mix<R, 1, kTabGlobal>(n) : pick_paths_mix<R, 1, kTabStaged>(n);
         return nullptr;
     }
     switch (kind) {
-        case 0: return pick_paths_n<R, 0, false>(n);
-        case 1: return table_global ? pick_paths_n<R, 1, true>(n) : pick_paths_n<R, 1, false>(n);
-        case 2: return pick_paths_n<R, 2, false>(n);
-        case 3: return table_global ? pick_paths_n<R, 3, true>(n) : pick_paths_n<R, 3, false>(n);
+        case 0: return pick_paths_n<R, 0, kTabStaged>(n);
+        case 1: return global ? pick_paths_n<R, 1, kTabGlobal>(n) : pick_paths_n<R, 1, kTabStaged>(n);
+        case 2: return pick_paths_n<R, 2, kTabStaged>(n);
+        case 3: return global ? pick_paths_n<R, 3, kTabGlobal>(n) : pick_paths_n<R, 3, kTabStaged>(n);
         default: return nullptr;
     }
 }
@@ -494,12 +536,26 @@ void run_paths(ob_paths_request& h) {
     }
     DeviceArena arena;
     arena.recycle = true;  // both streams are synchronised before the call returns
+    // Chunks of pairs, on two streams: the kernel of one chunk runs while the previous chunk's columns are copied to
+    // the host. A chunk's columns come back in the paths' own type (a float's double is the same value: half the bytes
+    // over the link) into the library's pinned staging (PinnedStage, at most a slot a chunk; host memory of this call
+    // where pinned memory cannot be had), and host threads widen and spread them into the caller's array while the
+    // next chunk runs. Large outputs go in four chunks at least. (The caller's array is not pinned: pinning 117 MB
+    // took 12.5 ms on a B200 host, longer than the pageable copy itself, 6.7 ms; pinned, 2.2 ms.)
+    const long long cols = static_cast<long long>(n) * h.n_cols;
+    const long long row_bytes = cols * 2 * static_cast<long long>(sizeof(R));  // one pair's output
+    constexpr long long kSlot = static_cast<long long>(PinnedStage::kSlotBytes);
+    long long chunk = h.n_pairs;
+    if (cols > 0) {
+        if (row_bytes * h.n_pairs >= kSlot / 8 * static_cast<long long>(sizeof(R))) chunk = (h.n_pairs + 3) / 4;
+        chunk = std::min(chunk, std::max<long long>(kSlot / row_bytes, 1024));
+    }
     PathsLvArgs<R> lv{};
-    const void* lv_fn = pack_paths_staged<R>(h, arena, lv)
-                            ? pick_paths_staged<R>(n, lv.kind, lv.table_global != 0, h.mixer != 0)
+    const void* lv_fn = pack_paths_staged<R>(h, chunk, sms, arena, lv)
+                            ? pick_paths_staged<R>(n, lv.kind, lv.tm, h.mixer != 0)
                             : nullptr;
     const bool fast = lv_fn != nullptr;
-    if (fast) allow_smem(lv_fn, lv.smem_blob);
+    if (fast) allow_smem(lv_fn, lv.smem);
     PathsDev<R> s{};
     if (!fast) {  // the generic kernel's inputs, in one copy
         ModelDev<R>& m = s.m;
@@ -530,20 +586,6 @@ void run_paths(ob_paths_request& h) {
         up.commit(arena);
     }
 
-    // Chunks of pairs, on two streams: the kernel of one chunk runs while the previous chunk's columns are copied to
-    // the host. A chunk's columns come back in the paths' own type (a float's double is the same value: half the bytes
-    // over the link) into the library's pinned staging (PinnedStage, at most a slot a chunk; host memory of this call
-    // where pinned memory cannot be had), and host threads widen and spread them into the caller's array while the
-    // next chunk runs. Large outputs go in four chunks at least. (The caller's array is not pinned: pinning 117 MB
-    // took 12.5 ms on a B200 host, longer than the pageable copy itself, 6.7 ms; pinned, 2.2 ms.)
-    const long long cols = static_cast<long long>(n) * h.n_cols;
-    const long long row_bytes = cols * 2 * static_cast<long long>(sizeof(R));  // one pair's output
-    constexpr long long kSlot = static_cast<long long>(PinnedStage::kSlotBytes);
-    long long chunk = h.n_pairs;
-    if (cols > 0) {
-        if (row_bytes * h.n_pairs >= kSlot / 8 * static_cast<long long>(sizeof(R))) chunk = (h.n_pairs + 3) / 4;
-        chunk = std::min(chunk, std::max<long long>(kSlot / row_bytes, 1024));
-    }
     R* stage[2] = {nullptr, nullptr};
     std::vector<R> own[2];
     if (cols > 0) {
@@ -615,8 +657,8 @@ void run_paths(ob_paths_request& h) {
         if (fast) {
             PathsLvArgs<R> la = lv;
             la.n_pairs = mcount, la.first_pair = h.first_pair + c0, la.rows = 2 * mcount, la.out = out;
-            const auto [lb, g] = launch_shape(lv_fn, la.smem_blob, sms, mcount, lv_block_of(n));
-            reinterpret_cast<void (*)(PathsLvArgs<R>)>(const_cast<void*>(lv_fn))<<<g, lb, la.smem_blob, st>>>(la);
+            const auto [lb, g] = launch_shape(lv_fn, la.smem, sms, mcount, lv_block_of(n, la.tm));
+            reinterpret_cast<void (*)(PathsLvArgs<R>)>(const_cast<void*>(lv_fn))<<<g, lb, la.smem, st>>>(la);
         } else if (n <= 1) paths_kernel<R, 1><<<grid, block, 0, st>>>(part);
         else if (n <= 2) paths_kernel<R, 2><<<grid, block, 0, st>>>(part);
         else if (n <= 4) paths_kernel<R, 4><<<grid, block, 0, st>>>(part);

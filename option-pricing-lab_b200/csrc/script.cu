@@ -445,15 +445,17 @@ struct LvArgs {
     const unsigned char* blob;
     int smem_blob;
     R top;
-    const Pair2<R>* tab;  // the table in global memory when it does not fit the stage (kernels with GT), else unused
-    int table_global;
+    const Pair2<R>* tab;  // the table in global memory (kTabGlobal, kTabStreamed), else unused
+    int tm;               // where the table is read
+    RowStreamArgs rs;     // kTabStreamed
+    int smem;             // bytes of dynamic shared memory
 };
 
 // BRANCH: the pairs continue the paths of an outer simulation after step end d.branch_step (one leg per outer path:
 // before the branch both legs take the outer path's normals, the outer antithetic leg's with the sign flipped).
-// GT: the table is read from global memory (a.tab) instead of the stage.
-template <typename R, int N, int NW, bool BRANCH, bool CALLS, bool GT = false, int WF = -1>
-__global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
+// TM: where the table is read (kTabStaged, kTabGlobal, kTabStreamed).
+template <typename R, int N, int NW, bool BRANCH, bool CALLS, int TM = kTabStaged, int WF = -1>
+__global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM != kTabStreamed && sizeof(R) == 4 ? 2 : 1)
     script_lv_kernel(ScriptDev<R> d, LvArgs<R> a, long long n_pairs, uint32_t k0, uint32_t k1,
                      double* __restrict__ partial) {
     constexpr int C = N;
@@ -465,20 +467,22 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
     constexpr int G = kLean ? 8 : (C % 4 == 0 ? 1 : (C % 2 == 0 ? 2 : 4));
     constexpr int NB = C * G / 4;
     extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ double wacc[16][2];
+    __shared__ double wacc[32][2];
     {
         const int4* src = reinterpret_cast<const int4*>(a.blob);
         int4* dst = reinterpret_cast<int4*>(sm);
         for (int t = threadIdx.x; t < a.smem_blob / 16; t += blockDim.x) dst[t] = src[t];
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-    if (threadIdx.x < 32) (&wacc[0][0])[threadIdx.x] = 0.0;
+    if (threadIdx.x < 64) (&wacc[0][0])[threadIdx.x] = 0.0;
     __syncthreads();
     const StepRec<R>* s_step = reinterpret_cast<const StepRec<R>*>(sm + a.off.step);
     const NameStep<R>* s_ns = reinterpret_cast<const NameStep<R>*>(sm + a.off.name_step);
     const R* s_root = reinterpret_cast<const R*>(sm + a.off.root);
-    const Pair2<R>* s_tab = GT ? a.tab : reinterpret_cast<const Pair2<R>*>(sm + a.off.table2);
-    const uint32_t tab_s = shared_address<GT>(s_tab);
+    const Pair2<R>* s_tab = TM == kTabStaged ? reinterpret_cast<const Pair2<R>*>(sm + a.off.table2) : a.tab;
+    const uint32_t tab_s = TM == kTabStreamed ? static_cast<uint32_t>(a.rs.off) : shared_address<TM == kTabStaged>(s_tab);
+    RowStream<R, N, G> rows(a.rs, a.tab, s_ns, sm, d.n_steps);
+    if (TM == kTabStreamed) rows.first();
     const int2* s_sched = reinterpret_cast<const int2*>(sm + a.off.sched);  // (event, window mask) per step end
     const R* s_lf0 = reinterpret_cast<const R*>(sm + a.off.lf0);
     const int S = d.n_steps;
@@ -489,8 +493,9 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
 #pragma unroll
     for (int k = 0; k < (kRootRegs ? N * N : 0); ++k) rt[k] = s_root[k];
     const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    for (long long base = static_cast<long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31); base < n_pairs;
-         base += stride) {
+    for (long long block0 = static_cast<long long>(blockIdx.x) * blockDim.x; block0 < n_pairs; block0 += stride) {
+        const long long base = block0 + (threadIdx.x & ~31);
+        if (TM != kTabStreamed && base >= n_pairs) break;  // (a streaming block's warps keep together)
         const bool active = base + lane < n_pairs;
         const uint64_t pair = static_cast<uint64_t>(active ? base + lane : n_pairs - 1);
         uint64_t opair = 0;
@@ -536,6 +541,7 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
         // One batch of G steps from step i0; only the tail batch (CHECK) may stop inside.
         auto run_batch = [&](int i0, int b, auto check, auto events) {
             constexpr bool CHECK = decltype(check)::value;
+            if (TM == kTabStreamed && rows.opens(b)) rows.turn(b, block0 + stride < n_pairs);
             R z[C * G];
             const bool own = !BRANCH || i0 + G - 1 > d.branch_step;  // a step of the batch draws its own normals
             if (own) {
@@ -573,7 +579,8 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
                 for (int n = 0; n < N; ++n) {
                     const NameStep<R> ns = s_ns[(i - 1) * N + n];
                     R v0, v1;
-                    table_vars<GT>(s_tab, tab_s, ns.org, ns.inv_dx, ns.row, a.top, x0[n], x1[n], v0, v1);
+                    table_vars<TM>(s_tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i, n) : ns.row,
+                                   a.top, x0[n], x1[n], v0, v1);
                     // sqrt(dt) z with the legs' signs (+1, -1 but before a branch), the step's multiply-adds written
                     // out: the same arithmetic in every instantiation, so a branch at step 0 is an ordinary run bit
                     // for bit
@@ -631,14 +638,14 @@ __global__ void __launch_bounds__(512, sizeof(R) == 4 ? 2 : 1)
 template <typename R>
 using ScriptLvFn = void (*)(ScriptDev<R>, LvArgs<R>, long long, uint32_t, uint32_t, double*);
 
-template <typename R, int NW, bool CALLS, bool GT = false>
+template <typename R, int NW, bool CALLS, int TM = kTabStaged>
 ScriptLvFn<R> pick_lv_calls(int n) {
     switch (n) {
-        case 1: return script_lv_kernel<R, 1, NW, false, CALLS, GT>;
-        case 2: return script_lv_kernel<R, 2, NW, false, CALLS, GT>;
-        case 3: return script_lv_kernel<R, 3, NW, false, CALLS, GT>;
-        case 4: return script_lv_kernel<R, 4, NW, false, CALLS, GT>;
-        case 5: return script_lv_kernel<R, 5, NW, false, CALLS, GT>;
+        case 1: return script_lv_kernel<R, 1, NW, false, CALLS, TM>;
+        case 2: return script_lv_kernel<R, 2, NW, false, CALLS, TM>;
+        case 3: return script_lv_kernel<R, 3, NW, false, CALLS, TM>;
+        case 4: return script_lv_kernel<R, 4, NW, false, CALLS, TM>;
+        case 5: return script_lv_kernel<R, 5, NW, false, CALLS, TM>;
         default: return nullptr;
     }
 }
@@ -651,20 +658,35 @@ ScriptLvFn<R> pick_lv_nw(int n, bool branch, bool calls) {
 
 // Kernels for one window (a knock-in barrier: its state alone stays in registers under the 64-register cap of two
 // blocks an SM, where a second window's spills it to local memory, 3.11 -> 2.67 ms for the 3-year daily-window
-// Phoenix), up to 2 and up to 8. A table in global memory (table_global) only comes with up to 2 windows, no call and
-// no branch (pack_lv checks).
+// Phoenix), up to 2 and up to 8. A table in global memory only comes with up to 2 windows, no call and no branch
+// (pack_lv checks); its rows are streamed for one name in float with at most one window (streams_script).
 // One name whose one window is a lowest or a highest (a knock-in or knock-out barrier of a single-name note), no call
 // and no branch: the window's function is compiled in (fix_windows, WF).
-template <typename R, bool GT>
+template <typename R, int TM>
 ScriptLvFn<R> pick_lv_single_window(int win_func) {
-    return win_func == 0 ? script_lv_kernel<R, 1, 1, false, false, GT, 0> : script_lv_kernel<R, 1, 1, false, false, GT, 1>;
+    return win_func == 0 ? script_lv_kernel<R, 1, 1, false, false, TM, 0> : script_lv_kernel<R, 1, 1, false, false, TM, 1>;
 }
 
 template <typename R>
-ScriptLvFn<R> pick_lv(int n, int n_windows, int win_func0, bool branch, bool calls, bool table_global) {
-    if (n == 1 && n_windows == 1 && !branch && !calls && (win_func0 == 0 || win_func0 == 1))
-        return table_global ? pick_lv_single_window<R, true>(win_func0) : pick_lv_single_window<R, false>(win_func0);
-    if (table_global) return n_windows <= 1 ? pick_lv_calls<R, 1, false, true>(n) : pick_lv_calls<R, 2, false, true>(n);
+constexpr bool streams_script(int n, int n_windows) {
+    return sizeof(R) == 4 && n == 1 && n_windows <= 1;
+}
+
+template <typename R>
+ScriptLvFn<R> pick_lv(int n, int n_windows, int win_func0, bool branch, bool calls, int tm) {
+    const bool single = n == 1 && n_windows == 1 && !branch && !calls && (win_func0 == 0 || win_func0 == 1);
+    if (tm == kTabStreamed) {
+        if constexpr (sizeof(R) == 4) {
+            if (single) return pick_lv_single_window<R, kTabStreamed>(win_func0);
+            return script_lv_kernel<R, 1, 1, false, false, kTabStreamed>;
+        }
+        return nullptr;
+    }
+    if (single)
+        return tm == kTabGlobal ? pick_lv_single_window<R, kTabGlobal>(win_func0)
+                                : pick_lv_single_window<R, kTabStaged>(win_func0);
+    if (tm == kTabGlobal)
+        return n_windows <= 1 ? pick_lv_calls<R, 1, false, kTabGlobal>(n) : pick_lv_calls<R, 2, false, kTabGlobal>(n);
     if (n_windows <= 1 && !branch && !calls) return pick_lv_calls<R, 1, false>(n);
     return n_windows <= 2 ? pick_lv_nw<R, 2>(n, branch, calls) : pick_lv_nw<R, kMaxWindows>(n, branch, calls);
 }
@@ -674,7 +696,7 @@ ScriptLvFn<R> pick_lv(int n, int n_windows, int win_func0, bool branch, bool cal
 // goes into the stage when it fits beside the rest, else into global memory (L2-resident, read through the read-only
 // cache) for scripts with up to two windows, no call and no branch.
 template <typename R>
-bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, DeviceArena& arena, LvArgs<R>& a) {
+bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, int sms, DeviceArena& arena, LvArgs<R>& a) {
     const ob_mc_request& q = rq.model;
     const int n = q.n_names, S = q.n_steps;
     if (q.model != OB_MODEL_PATHS || n > 5 || q.mixer) return false;
@@ -703,7 +725,7 @@ bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, Device
             const int row = q.step_row[static_cast<size_t>(k) * S + (i - 1)];
             r.lf = static_cast<R>(q.log_fwd[static_cast<size_t>(k) * (S + 1) + i]);
             set_cell_row(r, q.row_lo[row], q.row_inv_dx[row], a.top);
-            r.row = row * (q.n_x - 1);
+            r.row = row;  // (the row's first cell, once it is known where the table goes)
         }
     a.off.name_step = put(ns.data(), ns.size() * sizeof(NameStep<R>));
     std::vector<R> root(static_cast<size_t>(n) * n), lf0(n);
@@ -712,18 +734,29 @@ bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, Device
     a.off.root = put(root.data(), root.size() * sizeof(R));
     a.off.lf0 = put(lf0.data(), lf0.size() * sizeof(R));
     a.off.sched = put(sched.data(), sched.size() * sizeof(int2));
-    const size_t cells = table_cells(q.n_rows, q.n_x);
+    const size_t cells = static_cast<size_t>(q.n_rows) * (q.n_x - 1);
     const size_t budget = sizeof(R) == 4 ? (110u << 10) : (220u << 10);
     if (blob.size() > budget) return false;
-    a.table_global = ((blob.size() + 15) & ~static_cast<size_t>(15)) + cells * sizeof(Pair2<R>) > budget;
-    if (a.table_global && (rq.branch || rq.n_calls > 0 || rq.n_windows > 2)) return false;
-    if (a.table_global) {
+    const size_t at = (blob.size() + 15) & ~static_cast<size_t>(15);
+    a.tm = at + cells * sizeof(Pair2<R>) > budget ? kTabGlobal : kTabStaged;
+    if (a.tm == kTabGlobal && (rq.branch || rq.n_calls > 0 || rq.n_windows > 2)) return false;
+    if (a.tm == kTabGlobal) {
+        constexpr int G = 8;  // (kLean)
+        if (streams_script<R>(n, rq.n_windows) && streams_rows(n, q.n_pairs, sms) &&
+            plan_row_stream<R>(a.rs, q.n_x, n, G, at, 220u << 10)) {
+            a.tm = kTabStreamed;
+            a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
+        }
         a.tab = upload_table<R>(arena, q.table, q.n_rows, q.n_x);
     } else {
         a.off.table2 = put(nullptr, cells * sizeof(Pair2<R>));
-        pack_table<R>(q.table, q.n_x, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));
+        pack_table<R>(q.table, q.n_x, q.n_x - 1, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));
     }
+    NameStep<R>* step_ns = reinterpret_cast<NameStep<R>*>(blob.data() + a.off.name_step);
+    for (size_t k = 0; k < static_cast<size_t>(S) * n; ++k)
+        step_ns[k].row *= a.tm == kTabStaged ? q.n_x - 1 : table_pitch<R>(q.n_x);
     a.smem_blob = static_cast<int>((blob.size() + 15) & ~static_cast<size_t>(15));
+    if (a.tm != kTabStreamed) a.smem = a.smem_blob;
     unsigned char* dblob = arena.alloc<unsigned char>(std::max<size_t>(16, blob.size()));
     check_cuda(cudaMemcpy(dblob, blob.data(), blob.size(), cudaMemcpyHostToDevice), "copy blob");
     a.blob = dblob;
@@ -889,7 +922,7 @@ void run_script(const ob_script_request& rq, ob_script_result& res, const Record
         sched[i] = make_int2(event_at[i] >= 0 ? event_at[i] : i - next, static_cast<int>(fix_mask[i]));
     }
     LvArgs<R> lv{};
-    const bool fast = pack_lv<R>(rq, sched, arena, lv);
+    const bool fast = pack_lv<R>(rq, sched, sms, arena, lv);
     if (rq.branch && !fast) invalid("a branched run needs the staged local-vol kernel (its tables too large)");
     Upload up;
     ModelDev<R>& m = d.m;
@@ -978,11 +1011,11 @@ void run_script(const ob_script_request& rq, ob_script_result& res, const Record
 
     const void* fn = fast ? reinterpret_cast<const void*>(
                                 pick_lv<R>(n, rq.n_windows, rq.n_windows ? rq.win_func[0] : -1, rq.branch != 0, rq.n_calls > 0,
-                                          lv.table_global != 0))
+                                          lv.tm))
                           : reinterpret_cast<const void*>(pick_script<R>(mq.model, n, rq.n_windows));
-    const size_t smem = fast ? static_cast<size_t>(lv.smem_blob) : 0;
+    const size_t smem = fast ? static_cast<size_t>(lv.smem) : 0;
     if (fast) allow_smem(fn, smem);
-    const auto [block, grid] = launch_shape(fn, smem, sms, mq.n_pairs, fast ? 512 : 128);
+    const auto [block, grid] = launch_shape(fn, smem, sms, mq.n_pairs, !fast ? 128 : lv.tm == kTabStreamed ? 1024 : 512);
     double* partial = arena.alloc<double>(2 * static_cast<size_t>(grid));
     double* sums = reinterpret_cast<double*>(outs + 4);
     cudaEvent_t e0, e1;

@@ -3,8 +3,8 @@
 // points of each of 504 steps, 3.2 MB of intervals: 0.59 ms as one thread's conversion and a pageable copy).
 #pragma once
 
-#include "fused.cuh"
 #include "host_copy.cuh"
+#include "row_stream.cuh"
 
 namespace ob {
 
@@ -12,32 +12,35 @@ inline size_t table_cells(int n_rows, int n_x) {
     return static_cast<size_t>(n_rows) * static_cast<size_t>(n_x - 1);
 }
 
-// Intervals [first, first + count) into out.
+// Cells [first, first + count) into out, of rows of n_x - 1 intervals padded to `pitch` cells (the padding zero).
 template <typename R>
-inline void pack_table(const double* table, int n_x, size_t first, size_t count, Pair2<R>* out) {
-    const size_t w = static_cast<size_t>(n_x - 1);
-    size_t row = first / w, k = first - row * w;
+inline void pack_table(const double* table, int n_x, int pitch, size_t first, size_t count, Pair2<R>* out) {
+    const size_t w = static_cast<size_t>(n_x - 1), full = static_cast<size_t>(pitch);
+    size_t row = first / full, k = first - row * full;
     for (size_t done = 0; done < count; ++row, k = 0) {
         const double* y = table + row * static_cast<size_t>(n_x);
-        const size_t end = std::min(w, k + (count - done));
-        for (; k < end; ++k, ++done) out[done] = {static_cast<R>(y[k]), static_cast<R>(y[k + 1] - y[k])};
+        const size_t end = std::min(full, k + (count - done)), real = std::min(w, end);
+        for (; k < real; ++k, ++done) out[done] = {static_cast<R>(y[k]), static_cast<R>(y[k + 1] - y[k])};
+        for (; k < end; ++k, ++done) out[done] = {R(0), R(0)};
     }
 }
 
+// The table in global memory, its rows table_pitch cells apart.
 template <typename R>
 inline Pair2<R>* upload_table(DeviceArena& arena, const double* table, int n_rows, int n_x) {
-    const size_t cells = table_cells(n_rows, n_x);
+    const int pitch = table_pitch<R>(n_x);
+    const size_t cells = static_cast<size_t>(n_rows) * static_cast<size_t>(pitch);
     Pair2<R>* d = arena.alloc<Pair2<R>>(cells);
     char* slot[2] = {PinnedStage::get().bytes(0), PinnedStage::get().bytes(1)};
     if (!slot[0] || !slot[1]) {
         std::vector<Pair2<R>> tab(cells);
-        pack_table<R>(table, n_x, 0, cells, tab.data());
+        pack_table<R>(table, n_x, pitch, 0, cells, tab.data());
         check_cuda(cudaMemcpy(d, tab.data(), cells * sizeof(Pair2<R>), cudaMemcpyHostToDevice), "cudaMemcpy (table)");
         return d;
     }
     staged_upload(slot, reinterpret_cast<char*>(d), cells * sizeof(Pair2<R>), PinnedStage::kSlotBytes,
                   [&](char* out, size_t at, size_t count) {
-                      pack_table<R>(table, n_x, at / sizeof(Pair2<R>), count / sizeof(Pair2<R>),
+                      pack_table<R>(table, n_x, pitch, at / sizeof(Pair2<R>), count / sizeof(Pair2<R>),
                                     reinterpret_cast<Pair2<R>*>(out));
                   });
     return d;
