@@ -381,7 +381,7 @@ int ob_cpu_threads(void);
 int ob_device_info(int device, ob_device* out);
 /* No counterpart in the reference (it allocates and frees per call). The one-shot calls (ob_price, ob_mc_price,
    ob_paths, ob_script_price, ob_leverage, ob_philox_normals) keep their device buffers for the next call, at most
-   512 MB over all devices, with 64 MB of pinned host memory through which large inputs and outputs pass (the result
+   512 MB over all devices, with 64 MB of pinned host memory (at most) through which large inputs and outputs pass (the result
    reads 16 KB more) and up to three streams a device; this frees them and forgets the kernels' occupancy answers and shared-memory limits the
    plans cached. Call it before cudaDeviceReset or before destroying a context the library has used: cached buffers
    and attributes belong to the context that made them. */

@@ -176,15 +176,10 @@ void release_streams() {
 }
 
 void upload_bytes(void* dst, const void* src, size_t n) {
-    char* slot[2] = {nullptr, nullptr};
-    if (n > kStagedUpload) slot[0] = PinnedStage::get().bytes(0), slot[1] = PinnedStage::get().bytes(1);
-    if (!slot[0] || !slot[1]) {
-        check_cuda(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice), "cudaMemcpy (inputs)");
-        return;
-    }
-    staged_upload(slot, static_cast<char*>(dst), n, PinnedStage::kSlotBytes, [&](char* out, size_t at, size_t count) {
+    const bool staged = staged_upload(static_cast<char*>(dst), n, [&](char* out, size_t at, size_t count) {
         std::memcpy(out, static_cast<const char*>(src) + at, count);
     });
+    if (!staged) check_cuda(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice), "cudaMemcpy (inputs)");
 }
 
 namespace {

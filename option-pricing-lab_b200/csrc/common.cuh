@@ -101,9 +101,9 @@ constexpr int kKeptStreams = 3;
 cudaStream_t kept_stream(int which);
 void release_streams();  // (ob_release_buffers)
 
-// n bytes of pageable host memory to dst on the device; the copy has finished when it returns. Above kStagedUpload the
-// bytes go through the pinned staging, spread over the host threads (host_copy.cuh).
-constexpr size_t kStagedUpload = size_t(256) << 10;
+// n bytes of pageable host memory to dst on the device; the copy has finished when it returns. From kStagedUpload the
+// bytes go through the pinned staging, spread over the host threads (staged_upload in host_copy.cuh).
+constexpr size_t kStagedUpload = size_t(512) << 10;
 void upload_bytes(void* dst, const void* src, size_t n);
 
 // Device buffers that finished calls handed back, for the next call of the process: a one-shot call's cudaMalloc and

@@ -71,36 +71,46 @@ inline void widen(double* out, const T* from, long long n) {
     for (; k < n; ++k) out[k] = static_cast<double>(from[k]);
 }
 
-// Two pinned slots of kSlotBytes, allocated at their first use and kept until release() (ob_release_buffers).
-// Portable pinned memory: any device's copies may use it. Null where pinned memory cannot be had (the caller then
-// copies into its pageable array directly).
+// Two pinned slots, allocated at their first use and kept until release() (ob_release_buffers): of kSmallBytes while
+// that is enough, else of kSlotBytes (pinning costs 0.4 ms a megabyte, so a process that only uploads a table does not pay
+// for the path engine's). Portable pinned memory: any device's copies may use it. The library's calls are serialised and
+// finish their copies before they return, so a larger pair may replace the smaller one at the next call.
 class PinnedStage {
   public:
-    static constexpr size_t kSlotBytes = size_t(32) << 20;
+    static constexpr size_t kSmallBytes = size_t(4) << 20, kSlotBytes = size_t(32) << 20;
     static PinnedStage& get() {
         static PinnedStage* s = new PinnedStage();
         return *s;
     }
-    char* bytes(int k) {
+    // Both slots with room for `need` bytes each (at most kSlotBytes); false where pinned memory cannot be had (the
+    // caller then copies from or into pageable memory).
+    bool slots(size_t need, char* (&out)[2]) {
         std::lock_guard<std::mutex> lock(m_);
-        if (!base_ && !failed_) {
-            if (cudaHostAlloc(&base_, 2 * kSlotBytes, cudaHostAllocPortable) != cudaSuccess) {
+        const size_t want = need <= kSmallBytes ? kSmallBytes : kSlotBytes;
+        if (need > kSlotBytes) return false;
+        if (size_ < want && !failed_) {
+            if (base_) cudaFreeHost(base_);
+            base_ = nullptr, size_ = want;
+            if (cudaHostAlloc(&base_, 2 * want, cudaHostAllocPortable) != cudaSuccess) {
                 cudaGetLastError();
-                base_ = nullptr, failed_ = true;
+                base_ = nullptr, size_ = 0, failed_ = true;
             }
         }
-        return base_ ? static_cast<char*>(base_) + static_cast<size_t>(k) * kSlotBytes : nullptr;
+        if (!base_ || size_ < want) return false;
+        out[0] = static_cast<char*>(base_), out[1] = static_cast<char*>(base_) + size_;
+        return true;
     }
     void release() {
         std::lock_guard<std::mutex> lock(m_);
         if (base_) cudaFreeHost(base_);
         cudaGetLastError();
-        base_ = nullptr, failed_ = false;
+        base_ = nullptr, size_ = 0, failed_ = false;
     }
 
   private:
     std::mutex m_;
     void* base_ = nullptr;
+    size_t size_ = 0;
     bool failed_ = false;
 };
 
@@ -168,12 +178,16 @@ class HostPool {
     unsigned long long gen_ = 0;
 };
 
-// n bytes to dst on the device through two pinned slots of slot_bytes each: make(out, at, count) writes bytes
-// [at, at + count) of the source into out, for blocks of 4 KB at multiples of 4 KB (so a source of records of 8 or 16
-// bytes converts block by block) spread over the host threads; a slot's copy runs while the other is filled. The
-// copies have finished when it returns.
+// n bytes to dst on the device through the two pinned slots: make(out, at, count) writes bytes [at, at + count) of the
+// source into out, for blocks of 4 KB at multiples of 4 KB (so a source of records of 8 or 16 bytes converts block by
+// block) spread over the host threads; a slot's copy runs while the other is filled. The copies have finished when it
+// returns. False (nothing done) below kStagedUpload bytes, where one pageable copy is as fast, and without pinned memory.
 template <typename Make>
-void staged_upload(char* const (&slot)[2], char* dst, size_t n, size_t slot_bytes, Make make) {
+bool staged_upload(char* dst, size_t n, Make make) {
+    if (n < kStagedUpload) return false;
+    const size_t slot_bytes = n <= 4 * PinnedStage::kSmallBytes ? PinnedStage::kSmallBytes : PinnedStage::kSlotBytes;
+    char* slot[2];
+    if (!PinnedStage::get().slots(slot_bytes, slot)) return false;
     constexpr size_t kPiece = size_t(256) << 10, kBlock = 4096;
     cudaStream_t st = kept_stream(2);
     int k = 0;
@@ -193,6 +207,7 @@ void staged_upload(char* const (&slot)[2], char* dst, size_t n, size_t slot_byte
         check_cuda(cudaMemcpyAsync(dst + at, out, count, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync (inputs)");
     }
     check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize (inputs)");
+    return true;
 }
 
 }  // namespace ob

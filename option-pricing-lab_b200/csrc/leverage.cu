@@ -337,26 +337,26 @@ __global__ void __launch_bounds__(512) lev_bin(LevDev d, const R* __restrict__ x
     if (threadIdx.x == 0) bulk_wait_all();
 }
 
-// Exclusive prefix of x over the block and the block's total (any block size that is a multiple of 32, up to 1024).
-// Without `reuse` the caller guarantees a barrier before s_warp is written again, and the last one is left out.
-__device__ unsigned long long block_scan(unsigned long long x, unsigned long long* s_warp, unsigned long long& total,
-                                         bool reuse = true) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    unsigned long long inc = x;
+// Exclusive prefix of x over the block of NT threads and the block's total. The caller guarantees a barrier before
+// s_warp is written again.
+template <int NT, typename U>
+__device__ __forceinline__ U block_scan(U x, U* s_warp, U& total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    U inc = x;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xffffffffu, inc, off);
+        const U y = __shfl_up_sync(0xffffffffu, inc, off);
         if (lane >= off) inc += y;
     }
     if (lane == 31) s_warp[warp] = inc;
     __syncthreads();
-    unsigned long long before = 0, tot = 0;
-    for (int w = 0; w < nw; ++w) {
-        const unsigned long long c = s_warp[w];
-        before += w < warp ? c : 0ull;
+    U before = 0, tot = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+        const U c = s_warp[w];
+        before += w < warp ? c : U(0);
         tot += c;
     }
-    if (reuse) __syncthreads();
     total = tot;
     return before + inc - x;
 }
@@ -378,8 +378,8 @@ __device__ __forceinline__ double interp_uniform(double x, double a, double b, c
 // the runs' totals finds, for each quantile, the first run that reaches it, and that run's thread finds its bin.
 struct RegressShared {
     unsigned long long warp[32];
-    int best[2];
     double q[2];
+    double loc;  // the local variance at the block's grid point
     double red[5][32];
     double bw, lv_lo, lv_hi;  // the step's kernel bandwidth and local-variance row bounds (regress_stage)
 };
@@ -411,11 +411,14 @@ __device__ void regress_stage(const LevDev& d, int i, RegressShared& sh, double*
     }
 }
 
-// `more`: the block regresses another grid point after this one (its shared memory must be free again).
+// `more`: the block (of NT threads) regresses another grid point after this one (its shared memory must be free again).
+// U: the particle counts' type (a persistent block's shared memory bounds the particles far below 2^32).
+template <int NT, typename U>
 __device__ void regress_phase(const LevDev& d, double n_particles, int g, int i, double lo, double hi,
                               RegressShared& sh, unsigned* s_fine, double* s_row, bool more) {
-    const int nx = d.n_x, nb = d.n_bins, nf = d.n_fine, t = threadIdx.x, nt = blockDim.x;
-    const int lane = t & 31, warp = t >> 5, nw = nt >> 5;
+    constexpr int nt = NT, nw = NT / 32;
+    const int nx = d.n_x, nb = d.n_bins, nf = d.n_fine, t = threadIdx.x;
+    const int lane = t & 31, warp = t >> 5;
     const double* row = d.lv_rows + static_cast<long long>(i) * d.n_lv;
     double x0, cond = d.v0;
     unsigned long long all_v = 0;
@@ -438,7 +441,7 @@ __device__ void regress_phase(const LevDev& d, double n_particles, int g, int i,
         const int seg = (pk ? d.nfp / 2 : d.nfp) / nt, n4 = seg / 4, seg_b = pk ? 2 * seg : seg;
         const uint4* __restrict__ src = reinterpret_cast<const uint4*>(d.fine + static_cast<long long>(t) * seg);
         uint4* dst = reinterpret_cast<uint4*>(s_fine + t * seg);
-        unsigned long long mine = 0;
+        U mine = 0;
         for (int m0 = 0; m0 < n4; m0 += 4) {
             uint4 f[4];  // the loads issued together, then the stores
 #pragma unroll
@@ -449,32 +452,28 @@ __device__ void regress_phase(const LevDev& d, double n_particles, int g, int i,
                 const unsigned w4[4] = {f[u].x, f[u].y, f[u].z, f[u].w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    mine += pk ? (w4[j] & 0xffffu) + (w4[j] >> 16) : static_cast<unsigned long long>(w4[j]);
+                    mine += pk ? (w4[j] & 0xffffu) + (w4[j] >> 16) : w4[j];
             }
         }
-        if (t < 2) sh.best[t] = nt;
-        unsigned long long total_u;
-        // (its barrier publishes sh.best; the next write of sh.warp is in the next regression, barriers later)
-        const unsigned long long before = block_scan(mine, sh.warp, total_u, false);
+        if (t < 2) sh.q[t] = hi;  // (no run reaches the quantile's target)
+        U total_u;
+        // (its barrier publishes sh.q; the next write of sh.warp is in the next regression, barriers later)
+        const U before = block_scan<NT>(mine, reinterpret_cast<U*>(sh.warp), total_u);
         // every particle is in one fine bin: a packed count that passed 2^16 - 1 shows here
-        if (pk && t == 0 && total_u != static_cast<unsigned long long>(n_particles)) atomicCAS(d.status, 0, kPackOverflow);
+        if (pk && t == 0 && total_u != static_cast<U>(n_particles)) atomicCAS(d.status, 0, kPackOverflow);
         const double total = static_cast<double>(total_u);
         const double q2[2] = {d.q_lo, d.q_hi};
-        // counts are integers: (count) >= q total exactly when (count) >= ceil(q total)
-        const unsigned long long need[2] = {static_cast<unsigned long long>(ceil(q2[0] * total)),
-                                            static_cast<unsigned long long>(ceil(q2[1] * total))};
-        // the first run with a count whose end reaches the target holds the quantile's bin
-#pragma unroll
-        for (int qi = 0; qi < 2; ++qi)
-            if (mine > 0 && before + mine >= need[qi]) atomicMin(&sh.best[qi], t);
-        __syncthreads();
         const double width = (hi - lo) / static_cast<double>(nf);
+        // The first run with a count whose end reaches the target holds the quantile's bin: one thread at most, which
+        // finds the bin in the run it has just written. Counts are integers: (count) >= q total exactly when (count) >=
+        // ceil(q total).
 #pragma unroll
         for (int qi = 0; qi < 2; ++qi) {
-            const int w = sh.best[qi];
-            if (t == w) {
+            const double target = q2[qi] * total;
+            const U need = static_cast<U>(ceil(target));
+            if (mine > 0 && before + mine >= need && (before < need || before == 0)) {
                 const uint4* run = reinterpret_cast<const uint4*>(s_fine + t * seg);
-                unsigned long long cum = before, before_kb = 0;
+                U cum = before, before_kb = 0;
                 int kb = -1;
                 unsigned c_kb = 0u;
                 for (int m = 0; m < n4 && kb < 0; ++m) {
@@ -486,17 +485,13 @@ __device__ void regress_phase(const LevDev& d, double n_particles, int g, int i,
                         if (!pk && (u & 1)) continue;
                         const unsigned c = pk ? ((u & 1) ? w4[u >> 1] >> 16 : w4[u >> 1] & 0xffffu) : w4[u >> 1];
                         const int bin = t * seg_b + (pk ? 8 * m + u : 4 * m + (u >> 1));
-                        if (kb < 0 && c > 0 && cum + c >= need[qi]) kb = bin, c_kb = c, before_kb = cum;
+                        if (kb < 0 && c > 0 && cum + c >= need) kb = bin, c_kb = c, before_kb = cum;
                         cum += c;
                     }
                 }
-                const double target = q2[qi] * total;
-                sh.q[qi] = kb < 0 ? hi
-                                  : lo + (static_cast<double>(kb) +
-                                          (target - static_cast<double>(before_kb)) / static_cast<double>(c_kb)) *
-                                             width;
-            } else if (w >= nt && t == 0) {
-                sh.q[qi] = hi;
+                if (kb >= 0)
+                    sh.q[qi] = lo + (static_cast<double>(kb) +
+                                     (target - static_cast<double>(before_kb)) / static_cast<double>(c_kb)) * width;
             }
         }
         __syncthreads();
@@ -523,11 +518,19 @@ __device__ void regress_phase(const LevDev& d, double n_particles, int g, int i,
             r[q] = warp_sum(r[q]);
             if (lane == 0) sh.red[q][warp] = r[q];
         }
+        // beside the sums, one thread of the last warp reads the local variance at the grid point
+        if (t == nt - 1) sh.loc = interp_uniform(x0, sh.lv_lo, sh.lv_hi, s_row ? s_row : row, d.n_lv);
         __syncthreads();
         // the warps' sums added by warp 0 (thread 0 uses them)
         if (warp == 0)
 #pragma unroll
-            for (int q = 0; q < 5; ++q) r[q] = q < nq ? warp_sum(lane < nw ? sh.red[q][lane] : 0.0) : 0.0;
+            for (int q = 0; q < 5; ++q) {
+                if (q >= nq) break;
+                r[q] = lane < nw ? sh.red[q][lane] : 0.0;
+                // warp_sum's tree without its first level, whose upper half holds zeros
+#pragma unroll
+                for (int off = nw / 2; off > 0; off >>= 1) r[q] += __shfl_down_sync(0xffffffffu, r[q], off);
+            }
         const double S0 = r[0], T0 = r[1], Ax = r[2], Axx = r[3], Axv = r[4];
         const double nw_e = S0 > 1e-8 ? T0 / (S0 > 1e-300 ? S0 : 1e-300)
                                       : static_cast<double>(static_cast<long long>(all_v)) / kFix / n_particles;
@@ -541,7 +544,7 @@ __device__ void regress_phase(const LevDev& d, double n_particles, int g, int i,
         }
     }
     if (t == 0) {
-        const double loc = interp_uniform(x0, sh.lv_lo, sh.lv_hi, s_row ? s_row : row, d.n_lv);
+        const double loc = i == 0 ? interp_uniform(x0, sh.lv_lo, sh.lv_hi, s_row ? s_row : row, d.n_lv) : sh.loc;
         double L = sqrt(loc / (cond > 1e-8 ? cond : 1e-8));
         L = L > d.l_min ? L : d.l_min;
         L = L < d.l_max ? L : d.l_max;
@@ -567,7 +570,7 @@ __global__ void __launch_bounds__(256) lev_regress(LevDev d, double n_particles)
     double lo = 0.0, hi = 0.0;
     if (i > 0) range_of(d, lo, hi, s_mn, s_mx);  // (its barriers also order the staging)
     else __syncthreads();
-    regress_phase(d, n_particles, blockIdx.x, i, lo, hi, sh, s_fine, s_row, false);
+    regress_phase<256, unsigned long long>(d, n_particles, blockIdx.x, i, lo, hi, sh, s_fine, s_row, false);
 }
 
 // The normals of this thread's pairs at step i (Philox counter (pair, i + 1, 0, 0)): z0 at p, z1 at n + p.
@@ -577,6 +580,23 @@ __device__ void step_normals(const LevDev& d, const Particles<R>& pt, int i, R* 
         R z0, z1, z2, z3;
         normals4<R>(static_cast<uint64_t>(pt.first + p), static_cast<uint64_t>(i + 1), 0u, d.k0, d.k1, z0, z1, z2, z3);
         s_z[p] = z0, s_z[pt.n + p] = z1;
+    }
+}
+
+// The warp's min and max in lane 0: floats as integers in their order, one reduction instruction each.
+__device__ __forceinline__ void warp_extremes(float& mn, float& mx) {
+    auto key = [](float x) {
+        const int b = __float_as_int(x);
+        return b >= 0 ? b : b ^ 0x7fffffff;
+    };
+    auto back = [](int k) { return __int_as_float(k >= 0 ? k : k ^ 0x7fffffff); };
+    mn = back(__reduce_min_sync(0xffffffffu, key(mn))), mx = back(__reduce_max_sync(0xffffffffu, key(mx)));
+}
+__device__ __forceinline__ void warp_extremes(double& mn, double& mx) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        mn = m_min(mn, __shfl_down_sync(0xffffffffu, mn, off));
+        mx = m_max(mx, __shfl_down_sync(0xffffffffu, mx, off));
     }
 }
 
@@ -649,22 +669,14 @@ __device__ void step_phase(const LevDev& d, const Particles<R>& pt, int i, R* s_
             mn = m_min(mn, xn), mx = m_max(mx, xn);
         }
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        mn = m_min(mn, __shfl_down_sync(0xffffffffu, mn, off));
-        mx = m_max(mx, __shfl_down_sync(0xffffffffu, mx, off));
-    }
+    warp_extremes(mn, mx);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (lane == 0) s_min[warp] = mn, s_max[warp] = mx;
     __syncthreads();
     if (warp == 0) {
         // the warps' extremes, by warp 0
         mn = lane < nw ? s_min[lane] : s_min[0], mx = lane < nw ? s_max[lane] : s_max[0];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            mn = m_min(mn, __shfl_down_sync(0xffffffffu, mn, off));
-            mx = m_max(mx, __shfl_down_sync(0xffffffffu, mx, off));
-        }
+        warp_extremes(mn, mx);
     }
     if (threadIdx.x == 0) {
         if constexpr (SH) {
@@ -784,18 +796,19 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
     for (int i = 0; i < d.n_steps; ++i) {
         double lo = 0.0, hi = 0.0;
         if (i > 0) {
-            // the range's keys are loaded first; the step's normals are computed while they arrive
             const long long* r = d.rng + 2 * ((i - 1) & 1);
             const long long k_lo = __ldcg(r), k_hi = __ldcg(r + 1);
-            if (s_z) step_normals(d, pt, i, s_z);
             lo = from_order_key(k_lo), hi = from_order_key(k_hi);
             bin_phase<R, true>(d, pt, b, lo, hi);
             grid_arrive(d, arrived);
-            if (regresses) regress_stage(d, i, rs, s_row);  // (while thread 0 waits for the bulk reductions)
+            // while thread 0 waits for the bulk reductions and then for the other blocks': the regression's inputs and
+            // the step's normals
+            if (regresses) regress_stage(d, i, rs, s_row);
+            if (s_z) step_normals(d, pt, i, s_z);
             if (!grid_wait(d, arrived)) return;
         }
         for (int g = blockIdx.x; g < d.n_x; g += gridDim.x)
-            regress_phase(d, n_particles, g, i, lo, hi, rs, b.fine, s_row, g + static_cast<int>(gridDim.x) < d.n_x);
+            regress_phase<kPersistentThreads, unsigned>(d, n_particles, g, i, lo, hi, rs, b.fine, s_row, g + static_cast<int>(gridDim.x) < d.n_x);
         grid_arrive(d, arrived);
         bin_clear_shared(d, b);
         if (i == 0 && s_z) step_normals(d, pt, 0, s_z);
@@ -943,8 +956,8 @@ void run_leverage(ob_leverage_request& rq) {
     };
     // the output tables and the status through the pinned staging (in one wait), the tables then copied into the
     // caller's arrays; where it cannot hold them, the tables straight into those
-    double* pin = reinterpret_cast<double*>(PinnedStage::get().bytes(0));
-    if (2 * out_n * sizeof(double) + 16 > PinnedStage::kSlotBytes) pin = nullptr;
+    char* slot[2];
+    double* pin = PinnedStage::get().slots(2 * out_n * sizeof(double) + 16, slot) ? reinterpret_cast<double*>(slot[0]) : nullptr;
     auto read_back = [&](int* status) {
         int* const st_to = pin ? reinterpret_cast<int*>(pin + 2 * out_n) : status;
         if (status)

@@ -589,8 +589,8 @@ void run_paths(ob_paths_request& h) {
     R* stage[2] = {nullptr, nullptr};
     std::vector<R> own[2];
     if (cols > 0) {
-        char* slot[2] = {PinnedStage::get().bytes(0), PinnedStage::get().bytes(1)};
-        const bool pinned = slot[0] && slot[1] && row_bytes * chunk <= kSlot;
+        char* slot[2];
+        const bool pinned = PinnedStage::get().slots(static_cast<size_t>(row_bytes * chunk), slot);
         for (int k = 0; k < 2; ++k) {
             if (!pinned && (k == 0 || chunk < h.n_pairs)) own[k].resize(static_cast<size_t>(cols * 2 * chunk));
             stage[k] = pinned ? reinterpret_cast<R*>(slot[k]) : own[k].data();

@@ -31,18 +31,16 @@ inline Pair2<R>* upload_table(DeviceArena& arena, const double* table, int n_row
     const int pitch = table_pitch<R>(n_x);
     const size_t cells = static_cast<size_t>(n_rows) * static_cast<size_t>(pitch);
     Pair2<R>* d = arena.alloc<Pair2<R>>(cells);
-    char* slot[2] = {PinnedStage::get().bytes(0), PinnedStage::get().bytes(1)};
-    if (!slot[0] || !slot[1]) {
+    const bool staged = staged_upload(reinterpret_cast<char*>(d), cells * sizeof(Pair2<R>),
+                                      [&](char* out, size_t at, size_t count) {
+                                          pack_table<R>(table, n_x, pitch, at / sizeof(Pair2<R>),
+                                                        count / sizeof(Pair2<R>), reinterpret_cast<Pair2<R>*>(out));
+                                      });
+    if (!staged) {
         std::vector<Pair2<R>> tab(cells);
         pack_table<R>(table, n_x, pitch, 0, cells, tab.data());
         check_cuda(cudaMemcpy(d, tab.data(), cells * sizeof(Pair2<R>), cudaMemcpyHostToDevice), "cudaMemcpy (table)");
-        return d;
     }
-    staged_upload(slot, reinterpret_cast<char*>(d), cells * sizeof(Pair2<R>), PinnedStage::kSlotBytes,
-                  [&](char* out, size_t at, size_t count) {
-                      pack_table<R>(table, n_x, pitch, at / sizeof(Pair2<R>), count / sizeof(Pair2<R>),
-                                    reinterpret_cast<Pair2<R>*>(out));
-                  });
     return d;
 }
 
