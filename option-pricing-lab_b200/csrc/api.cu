@@ -92,22 +92,18 @@ void allow_smem(const void* kernel, size_t smem) {
 }
 
 LaunchShape launch_shape(const void* kernel, size_t smem, int sms, long long units, int max_block) {
-    constexpr double kIssueWarps = 24.0;
+    constexpr long long kLatencyWarps = 12;
     const long long chunks = (units + 31) / 32;
-    auto grid_of = [&](int b) {
-        const long long full = static_cast<long long>(sms) * std::max(1, occupancy(kernel, b, smem));
-        return std::max<long long>(1, std::min<long long>((units + b - 1) / b, full));
-    };
-    double best = -1.0;
-    int best_block = max_block;
+    LaunchShape best{max_block, 1};
+    long long least = -1;
     for (int b = max_block; b >= 64; b -= 32) {
-        const long long grid = grid_of(b), warps = grid * (b / 32), rounds = (chunks + warps - 1) / warps;
-        const double fill = static_cast<double>(chunks) / static_cast<double>(rounds * warps);
-        const double per_sm = static_cast<double>(warps) / sms;
-        const double score = fill * std::min(1.0, per_sm / kIssueWarps) * std::min(1.0, static_cast<double>(grid) / sms);
-        if (score > best * 1.0001) best = score, best_block = b;
+        const long long full = static_cast<long long>(sms) * std::max(1, occupancy(kernel, b, smem));
+        const long long grid = std::max<long long>(1, std::min<long long>((units + b - 1) / b, full));
+        const long long warps = grid * (b / 32), rounds = (chunks + warps - 1) / warps;
+        const long long cost = rounds * (kLatencyWarps + (grid + sms - 1) / sms * (b / 32));
+        if (least < 0 || cost < least) least = cost, best = {b, static_cast<int>(grid)};
     }
-    return {best_block, static_cast<int>(grid_of(best_block))};
+    return best;
 }
 
 void clear_launch_caches() {

@@ -71,13 +71,12 @@ int occupancy(const void* kernel, int block, size_t smem);
 // size: the attribute is a maximum, so a larger setting serves smaller launches).
 void allow_smem(const void* kernel, size_t smem);
 // Block size and grid of a launch whose warps each take chunks of 32 threads' units grid-stride, every chunk the same
-// length (a whole path): the run lasts ceil(chunks / resident warps) rounds, so among the multiples of 32 from max_block
-// down to 64 the block is taken that keeps that ceiling close to the exact quotient, with enough warps on each SM to keep
-// its schedulers issuing (24; fewer count as proportionally slower) and as many SMs as can be at work. 2^19 pairs of the
-// fused Phoenix: 448-thread blocks run 3.95 of 4 rounds where 512 leave a fourth round 46 % full (1.39 against
-// 1.52 ms); 2^18 pairs of the script kernel run two full rounds at 448 where 512 leave the second three quarters full
-// (877 -> 801 us a call); 2^16 pairs of the adjoint's forward run on 147 SMs at 448 where 1024 reached 64 (Greeks
-// 4.16 -> 3.58 ms). smem: dynamic shared memory at any block size.
+// length (a whole path). The launch lasts `rounds` = ceil(chunks / resident warps) walks, each as long as the fullest SM
+// makes it: a walk with w warps on an SM takes about as long as kLatencyWarps + w warps' issue (the 504-step Phoenix: 61 us
+// at 2 warps, 174 us at 28 to 32). Among the multiples of 32 from max_block down to 64 the block with the least
+// rounds (kLatencyWarps + w) is taken. 2^19 pairs of the fused Phoenix: 448-thread blocks run 3.95 of 4 rounds where 512
+// leave a fourth round 46 % full (1.39 against 1.52 ms); 2^16 pairs: 147 blocks of 448, one an SM, where 158 of 416 put
+// two on ten SMs (159 us). smem: dynamic shared memory at any block size.
 struct LaunchShape {
     int block, grid;
 };

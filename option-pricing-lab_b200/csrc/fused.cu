@@ -117,11 +117,7 @@ __global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM == kTabStr
     constexpr int NB = C * G / 4, NBA = CA * G / 4;
 
     extern __shared__ __align__(16) unsigned char sm[];
-    {
-        const int4* src = reinterpret_cast<const int4*>(a.blob);
-        int4* dst = reinterpret_cast<int4*>(sm);
-        for (int t = threadIdx.x; t < a.smem_blob / 16; t += blockDim.x) dst[t] = src[t];
-    }
+    stage_blob(sm, a.blob, a.smem_blob);
     const int n_warps = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_acc = 2 * a.n_out;
     double* wacc = reinterpret_cast<double*>(sm + a.smem_acc);
@@ -346,11 +342,7 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
     qe_pair_kernel(FusedArgs<R> a, long long n_pairs, long long first_pair, uint32_t k0, uint32_t k1,
                    double* __restrict__ partial) {
     extern __shared__ __align__(16) unsigned char sm[];
-    {
-        const int4* src = reinterpret_cast<const int4*>(a.blob);
-        int4* dst = reinterpret_cast<int4*>(sm);
-        for (int t = threadIdx.x; t < a.smem_blob / 16; t += blockDim.x) dst[t] = src[t];
-    }
+    stage_blob(sm, a.blob, a.smem_blob);
     const int n_warps = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n_acc = 2 * a.n_out;
     double* wacc = reinterpret_cast<double*>(sm + a.smem_acc);
@@ -465,6 +457,128 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
     }
 }
 
+// One to three local-vol names with the two legs of a pair on neighbouring lanes (as in qe_pair_kernel), for launches
+// of few pairs: a warp then carries 16 pairs through half the instructions a step, and a launch that leaves the schedulers
+// a warp or two each lasts as long as one warp's walk (fused_legs_apart has the sizes). The lanes draw alternate batches of
+// Philox blocks and swap them. Each leg's arithmetic is fused_kernel's, so a pair's value is the same bit for bit.
+template <typename R, int N, int PRODUCT, int TM>
+__global__ void __launch_bounds__(512, 1)
+    fused_legs_kernel(FusedArgs<R> a, long long n_pairs, long long first_pair, uint32_t k0, uint32_t k1,
+                      double* __restrict__ partial) {
+    constexpr int G = 4 / gcd4(N), NB = N * G / 4, Z = N * G;  // steps, blocks and normals of one lane's batch
+    extern __shared__ __align__(16) unsigned char sm[];
+    stage_blob(sm, a.blob, a.smem_blob);
+    const int n_warps = blockDim.x >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n_acc = 2 * a.n_out;
+    double* wacc = reinterpret_cast<double*>(sm + a.smem_acc);
+    for (int t = threadIdx.x; t < n_warps * n_acc; t += blockDim.x) wacc[t] = 0.0;
+    __syncthreads();
+    const StepRec<R>* s_step = reinterpret_cast<const StepRec<R>*>(sm + a.off.step);
+    const NameStep<R>* s_ns = reinterpret_cast<const NameStep<R>*>(sm + a.off.name_step);
+    const R* s_root = reinterpret_cast<const R*>(sm + a.off.root);
+    const Pair2<R>* s_tab = TM == kTabStaged ? reinterpret_cast<const Pair2<R>*>(sm + a.off.table2) : a.tab;
+    const R* s_trig = reinterpret_cast<const R*>(sm + a.off.ln_trig);
+    const double* s_disc = reinterpret_cast<const double*>(sm + a.off.obs_disc);
+    const int* leg_type = reinterpret_cast<const int*>(sm + a.off.leg_type);
+    const R* leg_strike = reinterpret_cast<const R*>(sm + a.off.leg_strike);
+    const int* leg_barrier = reinterpret_cast<const int*>(sm + a.off.leg_barrier);
+    const R* ln_level = reinterpret_cast<const R*>(sm + a.off.ln_level);
+    const int S = a.n_steps, odd = lane & 1;
+    constexpr unsigned kFull = 0xffffffffu;
+    R rt[N * N];
+#pragma unroll
+    for (int k = 0; k < N * N; ++k) rt[k] = s_root[k];
+    const long long stride = (static_cast<long long>(gridDim.x) * blockDim.x) >> 1;
+    for (long long base = (static_cast<long long>(blockIdx.x) * blockDim.x + (threadIdx.x & ~31)) >> 1;
+         base < n_pairs; base += stride) {
+        const long long p = base + (lane >> 1);
+        const bool active = p < n_pairs;
+        const uint64_t pair = static_cast<uint64_t>(first_pair + (active ? p : n_pairs - 1));
+        R x[N], lp = R(0);
+#pragma unroll
+        for (int n = 0; n < N; ++n) x[n] = R(0);
+        Leg<R> l;
+        leg_init<R, PRODUCT>(l);
+        // The normals of the lanes' two batches (2 G steps). Each is drawn beside the steps of the one before, which do
+        // not wait for it: a warp alone on its scheduler fills the one chain's waits with the other.
+        R e[2 * Z];
+        auto draw = [&](int m) {
+            R z[Z];
+#pragma unroll
+            for (int k = 0; k < NB; ++k)
+                normals4<R>(pair, static_cast<uint64_t>(2 * m + odd) * NB + k, 0u, k0, k1, z[4 * k], z[4 * k + 1],
+                            z[4 * k + 2], z[4 * k + 3]);
+#pragma unroll
+            for (int k = 0; k < Z; ++k) {
+                const R o = __shfl_xor_sync(kFull, z[k], 1);
+                e[k] = odd ? o : z[k], e[Z + k] = odd ? z[k] : o;
+            }
+        };
+        // 2 G steps from step i0; only the tail (CHECK) may stop inside
+        auto run_batches = [&](int i0, int m, auto check, auto observe) {
+            constexpr bool CHECK = decltype(check)::value, OBS = decltype(observe)::value;
+            R c[2 * Z];
+#pragma unroll
+            for (int k = 0; k < 2 * Z; ++k) c[k] = e[k];
+            if (!CHECK) draw(m + 1);
+#pragma unroll
+            for (int g = 0; g < 2 * G; ++g) {
+                const int i = i0 + g;
+                if constexpr (CHECK) {
+                    if (i > S) break;
+                }
+                const StepRec<R> st = s_step[i - 1];
+                R w = R(0);
+#pragma unroll
+                for (int n = 0; n < N; ++n) {
+                    R acc = R(0);
+#pragma unroll
+                    for (int b = 0; b < N; ++b) acc += rt[n * N + b] * c[g * N + b];
+                    const NameStep<R> ns = s_ns[(i - 1) * N + n];
+                    int j;
+                    R f;
+                    table_cell(ns, a.top, x[n], j, f);
+                    const Pair2<R> y = TM == kTabGlobal ? ldg_pair(s_tab + ns.row + j) : s_tab[ns.row + j];
+                    const R zd = st.sdt * acc;  // sqrt(dt) z, the legs' +-
+                    x[n] = lv_advance(x[n], m_fma(f, y.b, y.a), st.hdt, odd ? -zd : zd);
+                    w = n == 0 ? x[n] + ns.lf : m_min(w, x[n] + ns.lf);
+                }
+                lp = w;
+                if (PRODUCT == OB_PRODUCT_LADDER) {
+                    l.hi = run_max(l.hi, lp), l.lo = run_min(l.lo, lp);
+                } else {
+                    l.lo = run_min(l.lo, lp);
+                    const int j = OBS ? st.obs : -1;
+                    if (j >= 0) leg_observe(a, s_trig, s_disc, l, lp, j);
+                }
+            }
+        };
+        draw(0);
+        int i0 = 1, m = 0;
+        for (; i0 + 2 * G - 1 <= S; i0 += 2 * G, ++m) {
+            // (a step without an observation holds minus the steps to the next one)
+            if (PRODUCT == OB_PRODUCT_LADDER || s_step[i0 - 1].obs <= -2 * G)
+                run_batches(i0, m, std::false_type{}, std::false_type{});
+            else
+                run_batches(i0, m, std::false_type{}, std::true_type{});
+        }
+        if (i0 <= S) run_batches(i0, m, std::true_type{}, std::true_type{});
+        for (int k = 0; k < a.n_out; ++k) {
+            const double mine = leg_output<R, PRODUCT>(a, leg_type, leg_strike, leg_barrier, ln_level, l, lp, k);
+            const double other = __shfl_xor_sync(kFull, mine, 1);
+            const double y = active && !odd ? 0.5 * (mine + other) : 0.0;
+            const double s1 = warp_sum(y), s2 = warp_sum(y * y);
+            if (lane == 0) wacc[warp * n_acc + k] += s1, wacc[warp * n_acc + a.n_out + k] += s2;
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < n_acc; t += blockDim.x) {
+        double s = 0.0;
+        for (int w = 0; w < n_warps; ++w) s += wacc[w * n_acc + t];
+        partial[static_cast<long long>(blockIdx.x) * n_acc + t] = s;
+    }
+}
+
 template <typename R>
 using FusedFn = void (*)(FusedArgs<R>, long long, long long, uint32_t, uint32_t, double*);
 
@@ -473,7 +587,7 @@ FusedFn<R> pick_n(int n) {
     if (n == 1) return fused_kernel<R, 1, KIND, PRODUCT, TM>;
     if (n == 2) return fused_kernel<R, 2, KIND, PRODUCT, TM>;
     if (n == 3) return fused_kernel<R, 3, KIND, PRODUCT, TM>;
-    if constexpr ((KIND == 1 || KIND == 0) && TM != kTabStreamed) {
+    if constexpr (KIND == 1 || KIND == 0) {
         if (n == 4) return fused_kernel<R, 4, KIND, PRODUCT, TM>;
         if (n == 5) return fused_kernel<R, 5, KIND, PRODUCT, TM>;
     }
@@ -492,13 +606,13 @@ FusedFn<R> pick_mix(int n) {
     }
 }
 
-// tm: where the kinds with a table (local vol, SLV) read it; rows are streamed for one to three local-vol names in
-// float (in double the arithmetic bounds the step, not the table's reads).
+// tm: where the kinds with a table (local vol, SLV) read it; rows are streamed for one local-vol name in float (in double
+// the arithmetic bounds the step, not the table's reads).
 template <typename R, int PRODUCT>
 FusedFn<R> pick_fused(int kind, int n, int tm, bool mix) {
     if (tm == kTabStreamed) {
         if constexpr (sizeof(R) == 4)
-            if (kind == 1 && !mix) return pick_n<R, 1, PRODUCT, kTabStreamed>(n);
+            if (kind == 1 && n == 1 && !mix) return fused_kernel<R, 1, 1, PRODUCT, kTabStreamed>;
         return nullptr;
     }
     const bool global = tm == kTabGlobal;
@@ -512,6 +626,23 @@ FusedFn<R> pick_fused(int kind, int n, int tm, bool mix) {
         case 4: return n == 1 ? qe_pair_kernel<R, PRODUCT> : nullptr;
         default: return nullptr;
     }
+}
+
+template <typename R, int PRODUCT, int TM>
+FusedFn<R> pick_legs_n(int n) {
+    if (n == 1) return fused_legs_kernel<R, 1, PRODUCT, TM>;
+    if (n == 2) return fused_legs_kernel<R, 2, PRODUCT, TM>;
+    if (n == 3) return fused_legs_kernel<R, 3, PRODUCT, TM>;
+    return nullptr;
+}
+
+// The kernel with a pair's legs on two lanes for the same stage, or null.
+template <typename R, int PRODUCT>
+FusedFn<R> pick_legs(int kind, int n, int tm, bool mix) {
+    if constexpr (sizeof(R) == 4)
+        if (kind == 1 && !mix)
+            return tm == kTabStaged ? pick_legs_n<R, PRODUCT, kTabStaged>(n) : pick_legs_n<R, PRODUCT, kTabGlobal>(n);
+    return nullptr;
 }
 
 struct Blob {
@@ -655,7 +786,7 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
         if (aligned() + cells * sizeof(Pair2<R>) + acc_bytes(block) > budget) {
             constexpr size_t kStreamBudget = 220u << 10;  // one block an SM
             const int G = batch_steps(n, kind, false);
-            tm = pick(kTabStreamed) && streams_rows(n, rq.n_pairs, plan.sms) &&
+            tm = pick(kTabStreamed) && streams_rows(rq.n_pairs, plan.sms, 12.0) &&
                          plan_row_stream<R>(a.rs, rq.n_x, n, G, aligned(), kStreamBudget - acc_bytes(1024))
                      ? kTabStreamed
                      : kTabGlobal;
@@ -681,6 +812,13 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
     const void* k = reinterpret_cast<const void*>(fn);
     allow_smem(k, smem);
     if (occupancy(k, block, smem) < 1) return false;
+    if (tm != kTabStreamed) {
+        plan.n_names = n;
+        plan.kernel_legs = reinterpret_cast<const void*>(rq.product == OB_PRODUCT_LADDER
+                                                             ? pick_legs<R, OB_PRODUCT_LADDER>(kind, n, tm, rq.mixer != 0)
+                                                             : pick_legs<R, OB_PRODUCT_AUTOCALL>(kind, n, tm, rq.mixer != 0));
+        if (plan.kernel_legs) allow_smem(plan.kernel_legs, smem);
+    }
     plan.fused = true;
     plan.threads_per_pair = kind == 4 ? 2 : 1;
     plan.kernel = k;
@@ -689,6 +827,14 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
     plan.n_out = a.n_out;
     plan.fused_args<R>() = a;
     return true;
+}
+
+// Whether a run of n_pairs on n names puts a pair's legs on two lanes: while an SM gets few warps of whole pairs.
+// Kernel times, whole pairs against legs apart, 504 steps: one name (staged) 2^9 pairs 57 / 50 us, 2^13 60 / 53, 2^14.5 71 /
+// 63, 2^15 72 / 71, 2^16 99 / 110; two names of 40 x 200 points 2^13 207 / 109, 2^15 194 / 135, 2^15.5 211 / 212; three
+// 250 / 137, 237 / 202, 269 / 317; three of 801-point rows 398 / 190, 394 / 252, 410 / 432.
+bool fused_legs_apart(int n, long long n_pairs, int sms) {
+    return static_cast<double>(n_pairs) / (32.0 * sms) < (n == 1 ? 5.5 : 7.5);
 }
 
 template bool fused_build<float>(McPlan&, const ob_mc_request&);

@@ -445,13 +445,15 @@ McPlan::~McPlan() {
 
 void McPlan::run(long long n_pairs, long long first_pair, unsigned long long seed, cudaStream_t st) {
     if (n_pairs < 1 || first_pair < 0) invalid("n_pairs must be >= 1 and first_pair >= 0");
-    const LaunchShape shape = launch_shape(kernel, smem_bytes, sms, n_pairs * threads_per_pair, block);
+    const bool apart = kernel_legs && fused_legs_apart(n_names, n_pairs, sms);
+    const LaunchShape shape = launch_shape(apart ? kernel_legs : kernel, smem_bytes, sms,
+                                           n_pairs * (apart ? 2 : threads_per_pair), block);
     const int grid = std::min(shape.grid, max_blocks), blk = shape.block;
     const uint32_t k0 = static_cast<uint32_t>(seed), k1 = static_cast<uint32_t>(seed >> 32);
     if (!timing) check_cuda(cudaEventRecord(e0, st), "cudaEventRecord"), timing = true;
     using FusedF = void (*)(FusedArgs<float>, long long, long long, uint32_t, uint32_t, double*);
     using FusedD = void (*)(FusedArgs<double>, long long, long long, uint32_t, uint32_t, double*);
-    void* fn = const_cast<void*>(kernel);
+    void* fn = const_cast<void*>(apart ? kernel_legs : kernel);
     if (fused && precision == OB_FP32)
         reinterpret_cast<FusedF>(fn)<<<grid, blk, smem_bytes, st>>>(fa_f, n_pairs, first_pair, k0, k1, d_partial);
     else if (fused)

@@ -38,11 +38,12 @@ struct McPlan {
     DeviceArena arena;
     int precision = OB_FP32;
     int n_out = 0, sms = 0, max_blocks = 0;
-    int block = 256;
+    int block = 256, n_names = 1;
     int threads_per_pair = 1;  // 2: the QE kernel runs the two legs of a pair on two lanes
     bool force_generic = false;  // tests: run the generic kernel even where the specialised one applies
     size_t smem_bytes = 0;
     const void* kernel = nullptr;
+    const void* kernel_legs = nullptr;  // the fused kernel with a pair's legs on two lanes, for runs of few pairs
     McArgs<float> args_f{};
     McArgs<double> args_d{};
     double* d_partial = nullptr;
@@ -79,6 +80,7 @@ inline FusedArgs<double>& McPlan::fused_args<double>() {
 
 template <typename R>
 bool fused_build(McPlan& plan, const ob_mc_request& rq);
+bool fused_legs_apart(int n, long long n_pairs, int sms);  // whether such a run puts the legs apart
 
 template <>
 inline McArgs<float>& McPlan::args<float>() {

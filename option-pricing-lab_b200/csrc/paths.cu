@@ -180,11 +180,7 @@ __global__ void __launch_bounds__(lv_block<N, TM>(), TM != kTabStreamed && N == 
     constexpr int G = paths_batch_steps(N, KIND, MIX);
     constexpr int NB = C * G / 4, NBA = CA * G / 4;
     extern __shared__ __align__(16) unsigned char sm[];
-    {
-        const int4* src = reinterpret_cast<const int4*>(a.blob);
-        int4* dst = reinterpret_cast<int4*>(sm);
-        for (int t = threadIdx.x; t < a.smem_blob / 16; t += blockDim.x) dst[t] = src[t];
-    }
+    stage_blob(sm, a.blob, a.smem_blob);
     __syncthreads();
     const StepRec<R>* s_step = reinterpret_cast<const StepRec<R>*>(sm + a.off.step);
     const NameStep<R>* s_ns = reinterpret_cast<const NameStep<R>*>(sm + a.off.name_step);
@@ -446,7 +442,7 @@ bool pack_paths_staged(const ob_paths_request& h, long long chunk, int sms, Devi
     a.tm = at + cells * sizeof(Pair2<R>) > (n == 1 ? budget : size_t(200) << 10) ? kTabGlobal : kTabStaged;
     if (a.tm == kTabGlobal) {
         const int G = paths_batch_steps(n, kind, false);
-        if (streams_paths<R>(n, kind, h.mixer != 0) && streams_rows(n, chunk, sms) &&
+        if (streams_paths<R>(n, kind, h.mixer != 0) && streams_rows(chunk, sms, 20.0) &&
             plan_row_stream<R>(a.rs, h.n_x, n, G, at, 220u << 10)) {
             a.tm = kTabStreamed;
             a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));

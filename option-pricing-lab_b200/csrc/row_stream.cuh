@@ -38,14 +38,16 @@ inline size_t row_stream_bytes(const RowStreamArgs& rs, int n, int G) {
     return 2 * static_cast<size_t>(rs.batches) * G * n * rs.chunks * 16;
 }
 
-// Whether a launch of n_pairs on n names streams its rows. Kernel times, table through L1 against streamed, 504 steps of
-// 801-point rows: one name 2^13 pairs 140 / 191 us, 2^14 138 / 133, 2^15 144 / 125, 2^16 194 / 157, 2^17 217 / 219, 2^19
-// 767 / 815; three names (756 steps of 40 x 200) 2^13 346 / 351, 2^14 390 / 287, 2^16 800 / 483, 2^17 886 / 772, 2^18
-// 1579 / 1521, 801-point rows 2^18 1305 / 1311. Below, a block's few warps share too little of each row's copy; above,
-// enough warps hide the lookups, and two unsynchronised blocks an SM do better than one in step.
-inline bool streams_rows(int n, long long n_pairs, int sms) {
-    const double warps = static_cast<double>(n_pairs) / (32.0 * sms);  // an SM
-    return warps >= 3.4 && warps < (n == 1 ? 24.0 : 40.0);
+// Whether a launch of n_pairs streams its rows: from kFirst warps an SM, where a block's warps share each row's copy, to
+// `most`, from where enough warps hide the lookups and two unsynchronised blocks an SM do better than one in step.
+// Kernel times through L1 against streamed, one name, 504 steps of 801-point rows: fused Phoenix 2^14 pairs 140 / 133
+// us, 2^15 141 / 124, 2^15.5 144 / 140, 2^16 149 / 157; path engine's columns 2^14 248 / 189, 2^15 252 / 176, 2^16 260 /
+// 207, 2^16.5 267 / 235, 2^17 297 / 296; Phoenix script 2^14 277 / 205, 2^15 280 / 215, 2^16 287 / 264, 2^16.5 293 /
+// 293. (Two and three names put their legs on two lanes at the sizes where streaming would serve: legs_apart.)
+inline bool streams_rows(long long n_pairs, int sms, double most) {
+    constexpr double kFirst = 3.4;
+    const double warps = static_cast<double>(n_pairs) / (32.0 * sms);
+    return warps >= kFirst && warps < most;
 }
 
 // One block's ring. Every thread of the block makes the same calls in the same order: first() once, then turn() before

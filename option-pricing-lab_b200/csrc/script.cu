@@ -468,11 +468,7 @@ __global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM != kTabStr
     constexpr int NB = C * G / 4;
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ double wacc[32][2];
-    {
-        const int4* src = reinterpret_cast<const int4*>(a.blob);
-        int4* dst = reinterpret_cast<int4*>(sm);
-        for (int t = threadIdx.x; t < a.smem_blob / 16; t += blockDim.x) dst[t] = src[t];
-    }
+    stage_blob(sm, a.blob, a.smem_blob);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     if (threadIdx.x < 64) (&wacc[0][0])[threadIdx.x] = 0.0;
     __syncthreads();
@@ -742,7 +738,7 @@ bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, int sm
     if (a.tm == kTabGlobal && (rq.branch || rq.n_calls > 0 || rq.n_windows > 2)) return false;
     if (a.tm == kTabGlobal) {
         constexpr int G = 8;  // (kLean)
-        if (streams_script<R>(n, rq.n_windows) && streams_rows(n, q.n_pairs, sms) &&
+        if (streams_script<R>(n, rq.n_windows) && streams_rows(q.n_pairs, sms, 20.0) &&
             plan_row_stream<R>(a.rs, q.n_x, n, G, at, 220u << 10)) {
             a.tm = kTabStreamed;
             a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));

@@ -1,6 +1,6 @@
-"""Streamed table rows (one launch's pairs in the range that streams) against the same pairs priced where rows are read
-from global memory: the kernels step alike, so columns and pair values agree bit for bit; sizes around the range's ends,
-steps around a stage, row lengths of odd and even interval counts, repeated rows, several passes a block."""
+"""Streamed table rows, and a pair's legs on two lanes, against the same pairs priced by the other kernels (rows read from
+global memory, whole pairs): they step alike, so columns and pair values agree bit for bit; sizes around the ranges'
+ends, steps around a stage, row lengths of odd and even interval counts, repeated rows, several passes a block."""
 
 import numpy as np
 import pytest
@@ -13,9 +13,9 @@ from optlab_b200.requests import mc_request, paths_request, result_arrays
 
 pytestmark = pytest.mark.gpu
 
-# 148 SMs stream from about 2^14 to 2^16.8 pairs (one name): the first and last streamed counts, ragged ones, none
-STREAMED = [16103, 30001, 113663]
-SMALL = 4096  # pairs read from global memory, to compare with
+# 148 SMs stream 16103 to 56831 pairs (one name; to 94719 in paths and scripts): the range's ends and a ragged count
+STREAMED = [16103, 30001, 56831]
+SMALL = 4096  # pairs read from global memory (prices: with a pair's legs on two lanes), to compare with
 
 
 def _model(names, steps, n_x, n_pairs, seed=31):
@@ -23,7 +23,7 @@ def _model(names, steps, n_x, n_pairs, seed=31):
     t0 = np.arange(steps) / 252.0
     rows = names * steps
     step_row = np.arange(rows).reshape(names, steps).copy()
-    step_row[:, 5:9] = step_row[:, 4:5]  # a row used by several steps
+    step_row[:, 2:5] = step_row[:, 1:2]  # a row used by several steps
     table = 0.04 * (1 + 0.2 * rng.random((rows, 1))) + 0.01 * np.linspace(1, -1, n_x)[None, :] ** 2
     corr = np.full((names, names), 0.4) + 0.6 * np.eye(names)
     return dict(dt=np.full(steps, 1 / 252), t0=t0, n_pairs=n_pairs, seed=seed, kind=[1] * names, cvar=np.zeros(names),
@@ -55,18 +55,18 @@ def test_streamed_columns_equal_those_of_rows_in_global_memory(n_pairs, steps, n
 
 @pytest.mark.parametrize("n_pairs", [*STREAMED, 3 * 65536])
 @pytest.mark.parametrize("names", [1, 2, 3])
-@pytest.mark.parametrize("steps,n_x", [(29, 801), (57, 400)])
-def test_streamed_prices_equal_those_of_the_pieces(names, n_pairs, steps, n_x):
+@pytest.mark.parametrize("steps,n_x", [(29, 801), (57, 400), (40, 60), (8, 60), (5, 2)])
+def test_prices_equal_those_of_the_pieces(names, n_pairs, steps, n_x):
     m = workloads.FlatMarket(100.0, 0.02, 0.01)
     args = _model(names, steps, n_x, n_pairs)
     t_end = np.concatenate([[0.0], args["t0"] + args["dt"]])
-    obs = np.array([8, 16, steps])
+    obs = np.unique([steps // 3, steps // 2, steps])
     fields = dict(model=OB_MODEL_PATHS, spot=np.full(names, 100.0), log_fwd=np.tile(m.log_fwd(t_end), (names, 1)),
-                  product=1, obs_step=obs, obs_discount=m.D(obs / 252), trigger=[1.0, 1.0, 0.0], coupon_barrier=0.95,
+                  product=1, obs_step=obs, obs_discount=m.D(obs / 252), trigger=[1.0] * (len(obs) - 1) + [0.0], coupon_barrier=0.95,
                   coupon=0.02, ki_barrier=0.9, put_strike=1.0, memory=1, ki_daily=1)
     whole, _ = result_arrays(engine.mc_price(mc_request(**args, **fields), "fp32"))
     total = np.zeros(4)
-    for at in range(0, n_pairs, SMALL):  # pieces below the range: rows in global memory
+    for at in range(0, n_pairs, SMALL):  # pieces below the range: legs on two lanes
         count = min(SMALL, n_pairs - at)
         piece = dict(args, n_pairs=max(count, 2), first_pair=at)
         r = engine.mc_price(mc_request(**piece, **fields), "fp32")
