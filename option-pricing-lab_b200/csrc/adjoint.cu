@@ -68,7 +68,8 @@ struct AdjArgs {
     unsigned char* ki_name;    // 2 x n_pairs
     double* partial;           // per block: price sum and square, then per name delta sum and square
     double* grad;              // kAdjBatches x n_rows x n_x
-    R* priv;                   // per backward block: (left, right) weights of each table interval, n_rows x (n_x - 1)
+    int n_copies;              // dense backward: copies of the gradient in priv, copy k for batch k % kAdjBatches
+    R* priv;                   // per copy (recomputing backward: per block): (left, right) weights of each table interval, n_rows x (n_x - 1)
                                // pairs, zeroed before each backward
     unsigned long long* batch_pairs;  // kAdjBatches
 };
@@ -512,23 +513,36 @@ __device__ __forceinline__ void dense_segment(const AdjArgs<R>& a, long long p, 
     }
 }
 
-// One leg a warp: warps 2k and 2k + 1 of a block take the two legs of the same 32 pairs (so a pair's gradient stays
-// in one block's batch). Half the state of a pair a thread, so more warps fit an SM to hide the states' loads.
-template <typename R, int N>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 1) adj_backward_dense(AdjArgs<R> a) {
-    using GT = R;
-    GT* sg = a.priv + 2 * static_cast<long long>(blockIdx.x) * a.n_rows * (a.n_x - 1);
+// One leg a warp: warps 2k and 2k + 1 of a block take the two legs of the same 32 pairs. Half the state of a pair a
+// thread, so more warps fit an SM to hide the states' loads; 128-thread blocks, each walking couples of chunks (64
+// pairs). Groups of 128 pairs take the gradient copies in turn, whatever block walks them, so the batches that give the
+// vegas' errors depend on the pair alone. BLOCKS an SM in float: six (80 registers), or seven (72) for a launch that
+// then ends in one round (AdjPlan::build). 3 names x 1008 steps: 2^16 pairs, 1.15 rounds at six, 1.76 -> 1.25 ms at seven;
+// 2^18 pairs, where the reductions' rate at L2 bounds the sweep, 4.60 ms at six and 4.84 at seven. Four names take five
+// (their states would spill).
+// Copies of the dense backward's gradient: one for each group of 128 pairs up to this many an SM (in float all of them
+// together stay in L2 for the benchmark's tables).
+template <typename R>
+constexpr int copies_per_sm(int n) {
+    return sizeof(R) == 4 ? 3 : n <= 2 ? 2 : 1;
+}
+
+template <typename R, int N, int BLOCKS>
+__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (N == 4 ? 5 : BLOCKS) : 2) adj_backward_dense(AdjArgs<R> a) {
     const Pair2<R>* tab = a.table;  // (staging it in shared memory measured no faster: the state loads bound it)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, leg = warp & 1;
-    const int chunks_per_block = blockDim.x >> 6;  // pairs of warps
     const long long P = a.n_pairs;
-    const long long n_chunks = (P + 31) / 32;
-    unsigned long long mine = 0;
-    for (long long c = static_cast<long long>(blockIdx.x) * chunks_per_block + (warp >> 1); c < n_chunks;
-         c += static_cast<long long>(gridDim.x) * chunks_per_block) {
-        const long long p = c * 32 + lane;
+    const long long n_couples = (P + 63) / 64;
+    for (long long couple = blockIdx.x; couple < n_couples; couple += gridDim.x) {
+        const long long p = (2 * couple + (warp >> 1)) * 32 + lane;
+        const int copy = static_cast<int>((couple >> 1) % a.n_copies);
+        if (leg == 0) {
+            const unsigned walked = __ballot_sync(0xffffffffu, p < P);
+            if (lane == 0 && walked)
+                atomicAdd(a.batch_pairs + copy % kAdjBatches, static_cast<unsigned long long>(__popc(walked)));
+        }
         if (p >= P) continue;  // no block-wide synchronisation below: inactive lanes may leave
-        if (leg == 0) ++mine;
+        R* sg = a.priv + 2 * static_cast<long long>(copy) * a.n_rows * (a.n_x - 1);
         const int kstep = __ldg(a.ki_step + leg * P + p);
         const int kname = __ldg(a.ki_name + leg * P + p);
         const R kd = __ldg(a.dki + leg * P + p);
@@ -576,7 +590,26 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 1) adj_backward_dens
                 for (int n = 0; n < N; ++n) cur[g][n] = nxt[g][n];
         }
     }
-    flush_gradient(a, sg, mine);
+}
+
+// The batches' gradients from the dense backward's copies: entry k of a row is the left weight of interval k plus the
+// right weight of interval k - 1, summed over the batch's copies in order. One batch a grid row.
+template <typename R>
+__global__ void adj_gather(AdjArgs<R> a) {
+    const int nx = a.n_x, tab_n = a.n_rows * nx, batch = blockIdx.y;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= tab_n) return;
+    const int row = t / nx, k = t - row * nx;
+    const long long cells = 2 * static_cast<long long>(a.n_rows) * (nx - 1);
+    const R* at = a.priv + 2 * static_cast<long long>(row) * (nx - 1);
+    double v = 0.0;
+#pragma unroll 7
+    for (int c = batch; c < a.n_copies; c += kAdjBatches) {
+        const R left = k < nx - 1 ? __ldcs(at + c * cells + 2 * k) : R(0);
+        const R right = k > 0 ? __ldcs(at + c * cells + 2 * k - 1) : R(0);
+        v += static_cast<double>(left), v += static_cast<double>(right);
+    }
+    a.grad[static_cast<long long>(batch) * tab_n + t] = v;
 }
 
 // (y_i, y_i+1 - y_i) pairs of the caller's FP64 table.
@@ -606,6 +639,7 @@ struct AdjPlan {
     bool backward = false;
     cudaStream_t last = nullptr;
     int tab_n = 0;
+    bool seven = false;  // the dense backward's blocks an SM: seven, else six
     bool dense = false;  // the forward stores every step's state and the backward recomputes nothing
     bool staged = false; // the table is staged in shared memory (float tables up to kStageBytes)
     int block_f = 256, block_b = 256;
@@ -615,6 +649,8 @@ struct AdjPlan {
     AdjArgs<R>& args();
     template <typename R>
     void build(const ob_adjoint_request& rq);
+    template <typename R>
+    void run_backward(cudaStream_t st);
     void run(const double* d_table, double* d_grad, cudaStream_t st);
     void result(ob_adjoint_result& res, long long* batch_pairs);
     ~AdjPlan() {
@@ -639,8 +675,9 @@ void pick_st(AdjPlan& p) {
     p.kf = reinterpret_cast<const void*>(adj_forward<R, N, false, kCk, ST>);
     p.kfs = p.dense ? reinterpret_cast<const void*>(adj_forward<R, N, true, 1, ST>)
                     : reinterpret_cast<const void*>(adj_forward<R, N, true, kCk, ST>);
-    p.kb = p.dense ? reinterpret_cast<const void*>(adj_backward_dense<R, N>)
-                   : reinterpret_cast<const void*>(adj_backward<R, N>);
+    p.kb = !p.dense        ? reinterpret_cast<const void*>(adj_backward<R, N>)
+           : p.seven ? reinterpret_cast<const void*>(adj_backward_dense<R, N, 7>)
+                     : reinterpret_cast<const void*>(adj_backward_dense<R, N, 6>);
 }
 
 // Staged tables for float only (double tables of the benchmark's size do not fit a block's shared memory).
@@ -723,6 +760,8 @@ void AdjPlan::build(const ob_adjoint_request& r) {
     const long long P = rq.n_pairs;
     const double dense_bytes = static_cast<double>(S) * n * 2 * P * sizeof(R);
     dense = r.checkpoint == 1 || (r.checkpoint == 0 && dense_bytes <= kDenseBudget);
+    const long long couples = (P + 63) / 64;
+    seven = sizeof(R) == 4 && n <= 3 && couples > 6LL * sms && couples <= 7LL * sms;  // (four names would spill)
     a.n_ck = dense ? S : a.n_seg - 1;
     a.ckpt = arena.alloc<R>(static_cast<size_t>(std::max(1, a.n_ck)) * n * 2 * P);
     a.dobs = arena.alloc<R>(static_cast<size_t>(rq.n_obs) * 2 * P);
@@ -741,7 +780,6 @@ void AdjPlan::build(const ob_adjoint_request& r) {
         case 3: pick<R, 3>(*this); break;
         default: pick<R, 4>(*this); break;
     }
-    const size_t smem_b = 0;
     if (staged) {
         check_cuda(cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
                    "cudaFuncSetAttribute");
@@ -749,22 +787,33 @@ void AdjPlan::build(const ob_adjoint_request& r) {
                    "cudaFuncSetAttribute");
     }
     tab_n = rq.n_rows * rq.n_x;
-    int per_b = 0;
-    check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_b, kb, block_b, smem_b), "occupancy");
+    if (dense) block_b = 128;
+    const int per_b = occupancy(kb, block_b, 0);
     const LaunchShape f = launch_shape(kfs, smem, sms, P, block_f);
     block_f = f.block, grid_f = f.grid;
     const long long pairs_b = dense ? block_b / 2 : block_b;  // the dense backward takes one leg a thread
     grid_b = static_cast<int>(std::max<long long>(
         1, std::min<long long>((P + pairs_b - 1) / pairs_b, static_cast<long long>(sms) * std::max(1, per_b))));
+    a.n_copies = dense ? static_cast<int>(std::min<long long>((P + 127) / 128, static_cast<long long>(sms) * copies_per_sm<R>(n)))
+                       : grid_b;
     a.partial = arena.alloc<double>(static_cast<size_t>(grid_f) * (2 + 2 * n));
     const size_t cells2 = 2 * static_cast<size_t>(rq.n_rows) * (rq.n_x - 1);
-    priv_bytes = static_cast<size_t>(grid_b) * cells2 * sizeof(R);
-    a.priv = arena.alloc<R>(static_cast<size_t>(grid_b) * cells2);
+    priv_bytes = static_cast<size_t>(a.n_copies) * cells2 * sizeof(R);
+    a.priv = arena.alloc<R>(static_cast<size_t>(a.n_copies) * cells2);
     for (int k = 0; k < n; ++k) spot[k] = rq.spot[k];
 }
 
 template void AdjPlan::build<float>(const ob_adjoint_request&);
 template void AdjPlan::build<double>(const ob_adjoint_request&);
+
+template <typename R>
+void AdjPlan::run_backward(cudaStream_t st) {
+    const AdjArgs<R>& a = args<R>();
+    check_cuda(cudaMemsetAsync(a.batch_pairs, 0, kAdjBatches * sizeof(unsigned long long), st), "memset");
+    check_cuda(cudaMemsetAsync(a.priv, 0, priv_bytes, st), "cudaMemsetAsync");
+    reinterpret_cast<void (*)(AdjArgs<R>)>(const_cast<void*>(kb))<<<grid_b, block_b, 0, st>>>(a);
+    if (dense) adj_gather<R><<<dim3((tab_n + 255) / 256, kAdjBatches), 256, 0, st>>>(a);
+}
 
 void AdjPlan::run(const double* d_table, double* d_grad, cudaStream_t st) {
     const bool grad = d_grad != nullptr;
@@ -792,18 +841,9 @@ void AdjPlan::run(const double* d_table, double* d_grad, cudaStream_t st) {
     check_cuda(cudaEventRecord(e1, st), "cudaEventRecord");
     if (grad) {
         const size_t gbytes = static_cast<size_t>(kAdjBatches) * tab_n * sizeof(double);
-        check_cuda(cudaMemsetAsync(d_grad, 0, gbytes, st), "cudaMemsetAsync");
-        if (precision == OB_FP32) {
-            check_cuda(cudaMemsetAsync(af.batch_pairs, 0, kAdjBatches * sizeof(unsigned long long), st), "memset");
-            check_cuda(cudaMemsetAsync(af.priv, 0, priv_bytes, st), "cudaMemsetAsync");
-            using B = void (*)(AdjArgs<float>);
-            reinterpret_cast<B>(const_cast<void*>(kb))<<<grid_b, block_b, 0, st>>>(af);
-        } else {
-            check_cuda(cudaMemsetAsync(ad.batch_pairs, 0, kAdjBatches * sizeof(unsigned long long), st), "memset");
-            check_cuda(cudaMemsetAsync(ad.priv, 0, priv_bytes, st), "cudaMemsetAsync");
-            using B = void (*)(AdjArgs<double>);
-            reinterpret_cast<B>(const_cast<void*>(kb))<<<grid_b, block_b, 0, st>>>(ad);
-        }
+        if (!dense) check_cuda(cudaMemsetAsync(d_grad, 0, gbytes, st), "cudaMemsetAsync");  // (else adj_gather writes it)
+        if (precision == OB_FP32) run_backward<float>(st);
+        else run_backward<double>(st);
         check_cuda(cudaGetLastError(), "adj_backward launch");
     }
     check_cuda(cudaEventRecord(e2, st), "cudaEventRecord");
