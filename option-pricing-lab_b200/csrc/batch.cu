@@ -43,6 +43,7 @@ struct BTrade {
     R lf_rate;  // (r - q): the log-forward at grid point i is lf_rate i dt
     QeConsts<R> qe;
     int has_coupon, memory, ki_daily;
+    int track;       // the payoff reads the path's extremes: a ladder with a barrier, an autocall with a daily knock-in
     R ln_cb, ln_ki;
     double coupon, put_strike, discount;
     int slot0;       // first partial slot of its base simulation
@@ -55,8 +56,7 @@ struct BDev {
     const BTrade<R>* trades;
     const Pair2<R>* tab;  // (1 + n_vol) x pool rows x (n_x - 1): (var_i, var_i+1 - var_i), base then each vol move
     long long tab_stride; // pool rows x (n_x - 1)
-    const R* row_org;     // the row's origin and 1 / dx in the cell form (cell_row)
-    const R* row_inv_dx;
+    const Pair2<R>* row_cell;  // the row's origin and 1 / dx in the cell form (cell_row)
     const int* row_of;    // step -> expiry row
     const R* root;
     const int* leg_type;
@@ -237,6 +237,12 @@ __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __res
             for (int k = threadIdx.x; k < N * N; k += blockDim.x) s_root[k] = d.root[root + k];
         }
         __syncthreads();
+        // the correlation root: in registers up to three names, read from shared memory for more (registers spill)
+        constexpr bool kRootRegs = !QE && N <= 3;
+        R rt[kRootRegs ? N * N : 1];
+#pragma unroll
+        for (int k = 0; k < (kRootRegs ? N * N : 0); ++k) rt[k] = s_root[k];
+        const bool track = QE || t.track;
         const Pair2<R>* tab = d.tab + (shocked ? sim : 0) * d.tab_stride;
         const long long p0 = static_cast<long long>(tile) * d.tile;
         const long long p1 = min(p0 + d.tile, t.n_pairs);
@@ -269,25 +275,31 @@ __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __res
                         lp0 = x0[0], lp1 = x1[0];
                     } else {
                         const int erow = d.row_of[i - 1];
-                        const R lf = t.lf_rate * (static_cast<R>(i) * d.dt);
-                        lp0 = R(1e30), lp1 = R(1e30);
 #pragma unroll
                         for (int n = 0; n < N; ++n) {
                             R zc = R(0);
 #pragma unroll
-                            for (int m = 0; m < N; ++m) zc += s_root[n * N + m] * z[g * C + m];
+                            for (int m = 0; m < N; ++m) zc += (kRootRegs ? rt[n * N + m] : s_root[n * N + m]) * z[g * C + m];
                             const int row = t.row0 + n * d.n_exp + erow;
-                            const R org = d.row_org[row], inv = d.row_inv_dx[row];
+                            const Pair2<R> cell = ldg_pair(d.row_cell + row);  // origin, 1 / dx
                             const Pair2<R>* trow = tab + static_cast<long long>(row) * (d.n_x - 1);
                             const R zd = d.sdt * zc;  // sqrt(dt) z, the legs' +-
                             R var0, var1;
-                            table_vars<kTabGlobal>(trow, nullptr, 0u, org, inv, 0, d.top, x0[n], x1[n], var0, var1);
+                            table_vars<kTabGlobal>(trow, nullptr, 0u, cell.a, cell.b, 0, d.top, x0[n], x1[n], var0, var1);
                             lv_advance_legs(x0[n], x1[n], var0, var1, d.hdt, zd);
-                            lp0 = m_min(lp0, x0[n] + lf), lp1 = m_min(lp1, x1[n] + lf);
                         }
                     }
+                    const bool observed = PRODUCT == OB_PRODUCT_AUTOCALL && obs_at == i;
+                    // a payoff without a barrier reads the path at its observations and its end alone
+                    if (!track && !observed && i < S) continue;
+                    if (!QE) {
+                        const R lf = t.lf_rate * (static_cast<R>(i) * d.dt);
+                        lp0 = x0[0] + lf, lp1 = x1[0] + lf;
+#pragma unroll
+                        for (int n = 1; n < N; ++n) lp0 = m_min(lp0, x0[n] + lf), lp1 = m_min(lp1, x1[n] + lf);
+                    }
                     int j = -1;
-                    if (PRODUCT == OB_PRODUCT_AUTOCALL && obs_at == i) {
+                    if (observed) {
                         j = next_obs++;
                         obs_at = next_obs < t.n_obs ? d.obs_step[t.obs0 + next_obs] : -1;
                     }
@@ -564,10 +576,9 @@ void Batch::build(const ob_batch_request& rq) {
                 for (int k = 0; k + 1 < nx; ++k) out[k] = {static_cast<R>(v[k]), static_cast<R>(v[k + 1] - v[k])};
             }
         d.tab = arena.put<Pair2<R>>(tab.data(), tab.size());
-        std::vector<R> org(max_row), inv(max_row);
-        for (int r = 0; r < max_row; ++r) cell_row(rq.row_lo[r], rq.row_inv_dx[r], d.top, org[r], inv[r]);
-        d.row_org = arena.put<R>(org.data(), org.size());
-        d.row_inv_dx = arena.put<R>(inv.data(), inv.size());
+        std::vector<Pair2<R>> cell(max_row);
+        for (int r = 0; r < max_row; ++r) cell_row(rq.row_lo[r], rq.row_inv_dx[r], d.top, cell[r].a, cell[r].b);
+        d.row_cell = arena.put<Pair2<R>>(cell.data(), cell.size());
         d.root = arena.put<R>(rq.root, max_root);
     }
     if (max_leg > 0) {
@@ -614,6 +625,9 @@ void Batch::build(const ob_batch_request& rq) {
         if (t.model == OB_MODEL_HESTON_QE) b.qe = make_qe_consts<R>(t.heston, t.r, t.q, rq.dt);
         b.has_coupon = t.coupon > 0.0 || t.coupon_barrier > 0.0;
         b.memory = t.memory, b.ki_daily = t.ki_daily;
+        b.track = t.product == OB_PRODUCT_AUTOCALL
+                      ? t.ki_daily != 0
+                      : std::any_of(rq.leg_barrier + t.leg0, rq.leg_barrier + t.leg0 + t.n_legs, [](int k) { return k != 0; });
         b.ln_cb = t.coupon_barrier > 0 ? static_cast<R>(std::log(t.coupon_barrier)) : R(-1e30);
         b.ln_ki = t.ki_barrier > 0 ? static_cast<R>(std::log(t.ki_barrier)) : R(-1e30);
         b.coupon = t.coupon, b.put_strike = t.put_strike, b.discount = t.discount;
