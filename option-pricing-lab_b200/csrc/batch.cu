@@ -209,6 +209,13 @@ __device__ __forceinline__ void rec_carry(Rec<R, OB_PRODUCT_AUTOCALL>& r, R lp, 
         if (c < nc) r.lowc[c] = run_min(r.lowc[c], lp + d.carry_dt[c] * fi);
 }
 
+// Four values of one shared-memory load (two in double).
+template <typename R>
+struct alignas(16) Quad {
+    R v[4];
+};
+constexpr int kRootPitch = 8;
+
 template <typename R, int N, bool QE, int PRODUCT>
 __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __restrict__ items, int n_items,
                                                     int* counter) {
@@ -217,7 +224,7 @@ __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __res
     constexpr int NB = C * G / 4;
     __shared__ int s_item;
     __shared__ double wacc[8][2 * kBatchMaxOut];
-    __shared__ R s_root[25];
+    __shared__ alignas(16) R s_root[N * kRootPitch];  // by columns: column m holds root[n][m] of every name n
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     for (;;) {
         if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
@@ -234,14 +241,14 @@ __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __res
         for (int k = threadIdx.x; k < 8 * 2 * kBatchMaxOut; k += blockDim.x) (&wacc[0][0])[k] = 0.0;
         if (!QE) {
             const int root = sim > d.n_vol ? t.corr_root0 + (sim - 1 - d.n_vol) * N * N : t.root0;
-            for (int k = threadIdx.x; k < N * N; k += blockDim.x) s_root[k] = d.root[root + k];
+            for (int k = threadIdx.x; k < N * N; k += blockDim.x) s_root[k % N * kRootPitch + k / N] = d.root[root + k];
         }
         __syncthreads();
         // the correlation root: in registers up to three names, read from shared memory for more (registers spill)
         constexpr bool kRootRegs = !QE && N <= 3;
         R rt[kRootRegs ? N * N : 1];
 #pragma unroll
-        for (int k = 0; k < (kRootRegs ? N * N : 0); ++k) rt[k] = s_root[k];
+        for (int k = 0; k < (kRootRegs ? N * N : 0); ++k) rt[k] = s_root[k % N * kRootPitch + k / N];
         const bool track = QE || t.track;
         const Pair2<R>* tab = d.tab + (shocked ? sim : 0) * d.tab_stride;
         const long long p0 = static_cast<long long>(tile) * d.tile;
@@ -275,11 +282,25 @@ __global__ void __launch_bounds__(256) batch_kernel(BDev<R> d, const int4* __res
                         lp0 = x0[0], lp1 = x1[0];
                     } else {
                         const int erow = d.row_of[i - 1];
+                        R zcs[N];
+#pragma unroll
+                        for (int n = 0; n < N; ++n) zcs[n] = R(0);
+#pragma unroll
+                        for (int m = 0; m < N; ++m) {
+                            if constexpr (kRootRegs) {
+#pragma unroll
+                                for (int n = 0; n < N; ++n) zcs[n] += rt[n * N + m] * z[g * C + m];
+                            } else {  // four names a load
+                                const Quad<R>* col = reinterpret_cast<const Quad<R>*>(s_root + m * kRootPitch);
+                                const Quad<R> q = col[0];
+                                const R last = N > 4 ? s_root[m * kRootPitch + 4] : R(0);
+#pragma unroll
+                                for (int n = 0; n < N; ++n) zcs[n] += (n < 4 ? q.v[n & 3] : last) * z[g * C + m];
+                            }
+                        }
 #pragma unroll
                         for (int n = 0; n < N; ++n) {
-                            R zc = R(0);
-#pragma unroll
-                            for (int m = 0; m < N; ++m) zc += (kRootRegs ? rt[n * N + m] : s_root[n * N + m]) * z[g * C + m];
+                            const R zc = zcs[n];
                             const int row = t.row0 + n * d.n_exp + erow;
                             const Pair2<R> cell = ldg_pair(d.row_cell + row);  // origin, 1 / dx
                             const Pair2<R>* trow = tab + static_cast<long long>(row) * (d.n_x - 1);

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM == kTabStr
     const double* s_disc = reinterpret_cast<const double*>(sm + a.off.obs_disc);
     const int S = a.n_steps;
     // the correlation root: in registers for one or two names, read from shared memory for more (registers spill)
-    constexpr bool kRootRegs = N <= 2;
+    constexpr bool kRootRegs = N <= 3;
     R rt[kRootRegs ? N * N : 1];
 #pragma unroll
     for (int k = 0; k < (kRootRegs ? N * N : 0); ++k) rt[k] = s_root[k];
