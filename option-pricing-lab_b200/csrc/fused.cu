@@ -94,12 +94,12 @@ constexpr int fused_min_blocks() {
     return MIX && N >= 4 ? 1 : min_blocks<R>();
 }
 
-// Steps per batch of whole Philox blocks. One local-vol name draws two blocks a batch (8 steps), whose two independent
-// multiply chains interleave (1.317 -> 1.300 ms for the 2^20-path Phoenix; one SLV name would draw four and spill in
-// FP64).
+// Steps per batch of whole Philox blocks. One or two local-vol names draw two blocks a batch (8 or 4 steps), whose two
+// independent multiply chains interleave (one name 1.317 -> 1.300 ms for the 2^20-path Phoenix, two 1150 -> 1045 us for
+// 500k paths x 756 steps; one SLV name would draw four and spill in FP64).
 constexpr int batch_steps(int n, int kind, bool mix) {
     const int c = kind == 4 ? 2 : kind == 2 ? 2 * n : n + (mix ? 1 : 0);
-    return c == 1 && kind == 1 ? 8 : 4 / gcd4(c);
+    return kind == 1 && c <= 2 ? 8 / c : 4 / gcd4(c);
 }
 
 // MIX (local vol, 2 to 5 names): the local-correlation mixer, one more normal a step after the names'.

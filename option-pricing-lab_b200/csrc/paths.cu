@@ -160,10 +160,11 @@ constexpr int lv_block() {
     return TM == kTabStreamed ? 1024 : N <= 2 ? 512 : 256;
 }
 
-// Steps per batch of whole Philox blocks.
+// Steps per batch of whole Philox blocks; one or two local-vol names draw two blocks a batch, as in the fused kernel (200k
+// paths x 756 steps: one name 385 -> 380 us, two 1476 -> 1433).
 constexpr int paths_batch_steps(int n, int kind, bool mix) {
     const int c = kind == 2 ? 2 * n : n + (mix ? 1 : 0);
-    return c % 4 == 0 ? 1 : (c % 2 == 0 ? 2 : 4);
+    return kind == 1 && c <= 2 ? 8 / c : c % 4 == 0 ? 1 : (c % 2 == 0 ? 2 : 4);
 }
 
 // KIND: 0 Black-Scholes (constant variance), 1 local vol (table), 2 Heston (Euler), 3 SLV (table x Heston, residuals
@@ -532,11 +533,12 @@ void run_paths(ob_paths_request& h) {
     }
     DeviceArena arena;
     arena.recycle = true;  // both streams are synchronised before the call returns
-    // Chunks of pairs, on two streams: the kernel of one chunk runs while the previous chunk's columns are copied to
-    // the host. A chunk's columns come back in the paths' own type (a float's double is the same value: half the bytes
-    // over the link) into the library's pinned staging (PinnedStage, at most a slot a chunk; host memory of this call
-    // where pinned memory cannot be had), and host threads widen and spread them into the caller's array while the
-    // next chunk runs. Large outputs go in four chunks at least. (The caller's array is not pinned: pinning 117 MB
+    // Chunks of pairs, on two streams. A chunk's columns go in the paths' own type (a float's double is the same value:
+    // half the bytes over the link) into the library's pinned staging, at most a slot a chunk: the kernel writes each
+    // there at its observation, across the link, while it steps (a copy after the kernel took 0.2 of the 1.46 ms of a call
+    // of 200k paths x 756 steps with 14 columns). Where pinned memory cannot be had, the kernel writes device memory,
+    // copied into host memory of this call. Host threads then widen and spread a chunk into the caller's array while the
+    // next one runs. Large outputs go in four chunks at least. (The caller's array is not pinned: pinning 117 MB
     // took 12.5 ms on a B200 host, longer than the pageable copy itself, 6.7 ms; pinned, 2.2 ms.)
     const long long cols = static_cast<long long>(n) * h.n_cols;
     const long long row_bytes = cols * 2 * static_cast<long long>(sizeof(R));  // one pair's output
@@ -582,18 +584,27 @@ void run_paths(ob_paths_request& h) {
         up.commit(arena);
     }
 
-    R* stage[2] = {nullptr, nullptr};
+    R* stage[2] = {nullptr, nullptr};  // the chunks' columns on the host
+    R* dbuf[2] = {nullptr, nullptr};   // where the kernels write them
     std::vector<R> own[2];
+    bool direct = false;
     if (cols > 0) {
         char* slot[2];
-        const bool pinned = PinnedStage::get().slots(static_cast<size_t>(row_bytes * chunk), slot);
-        for (int k = 0; k < 2; ++k) {
-            if (!pinned && (k == 0 || chunk < h.n_pairs)) own[k].resize(static_cast<size_t>(cols * 2 * chunk));
-            stage[k] = pinned ? reinterpret_cast<R*>(slot[k]) : own[k].data();
+        void *d0 = nullptr, *d1 = nullptr;
+        direct = PinnedStage::get().slots(static_cast<size_t>(row_bytes * chunk), slot) &&
+                 cudaHostGetDevicePointer(&d0, slot[0], 0) == cudaSuccess &&
+                 cudaHostGetDevicePointer(&d1, slot[1], 0) == cudaSuccess;
+        cudaGetLastError();
+        if (direct) {
+            for (int k = 0; k < 2; ++k) stage[k] = reinterpret_cast<R*>(slot[k]);
+            dbuf[0] = static_cast<R*>(d0), dbuf[1] = static_cast<R*>(d1);
         }
     }
-    R* dbuf[2] = {arena.alloc<R>(std::max<long long>(1, cols * 2 * chunk)),
-                  chunk < h.n_pairs ? arena.alloc<R>(std::max<long long>(1, cols * 2 * chunk)) : nullptr};
+    for (int k = 0; k < (chunk < h.n_pairs ? 2 : 1) && !direct; ++k) {
+        own[k].resize(static_cast<size_t>(cols * 2 * chunk));
+        stage[k] = own[k].data();
+        dbuf[k] = arena.alloc<R>(std::max<long long>(1, cols * 2 * chunk));
+    }
     const cudaStream_t sts[2] = {kept_stream(0), kept_stream(1)};
     std::vector<cudaEvent_t> evs;
     auto event = [&]() {
@@ -610,8 +621,12 @@ void run_paths(ob_paths_request& h) {
     } done{evs};
     const long long n_chunks = (h.n_pairs + chunk - 1) / chunk;
     std::vector<cudaEvent_t> k0(n_chunks), k1(n_chunks), staged(n_chunks);
-    // chunk c's columns into slot c % 2 on its stream (after its kernel) ...
+    // chunk c's columns are in slot c % 2 of the staging once its kernel, or the copy after it, has finished ...
     auto stage_chunk = [&](long long c) {
+        if (direct) {
+            staged[c] = k1[c];
+            return;
+        }
         const long long mcount = std::min(chunk, h.n_pairs - c * chunk);
         check_cuda(cudaMemcpyAsync(stage[c % 2], dbuf[c % 2], static_cast<size_t>(cols * 2 * mcount) * sizeof(R),
                                    cudaMemcpyDeviceToHost, sts[c % 2]),
