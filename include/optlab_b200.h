@@ -227,6 +227,16 @@ typedef struct {
     double forward_ms, backward_ms;
 } ob_adjoint_result;
 
+/* Tent bumps of the local volatility: device arrays of doubles, row-major. base: the local variances (n_rows x n_x) the
+   last run took, grad: the gradients it wrote; onehot (n_rows x n_names) and phi (n_rows x n_e) weigh a table row's name and expiry nodes, psi
+   (n_rows x n_x x n_k) its cells' log-strike nodes; work: n_rows x n_k x OB_ADJ_BATCHES doubles; out: the vegas, then
+   their standard errors (n_names x n_e x n_k each). */
+typedef struct {
+    const double *base, *grad, *onehot, *phi, *psi;
+    double *work, *out;
+    int n_names, n_e, n_k;
+} ob_adjoint_nodes;
+
 typedef struct ob_adjoint_plan ob_adjoint_plan;
 
 /* ---------------------------------------------------------------------------------------------- batched risk */
@@ -439,9 +449,12 @@ int ob_mc_plan_destroy(ob_mc_plan* plan);
    replacing the current one, NULL keeps it) and, with d_grad non-null, the backward pass, filling d_grad (device,
    OB_ADJ_BATCHES x n_rows x n_x doubles) with each batch's sum over its pairs of d(pair value)/d(table entry);
    result waits, returns price and deltas with standard errors, and the pairs of each batch (batch_pairs may be
-   NULL). Without d_grad, run is the smoothed revaluation of a bump-and-revalue. */
+   NULL). Without d_grad, run is the smoothed revaluation of a bump-and-revalue. node_vegas, after a run with a gradient
+   and on that run's stream, writes the node vegas of tent bumps and their batch-mean standard
+   errors. */
 int ob_adjoint_plan_create(const ob_adjoint_request* rq, int precision, ob_adjoint_plan** plan);
 int ob_adjoint_run(ob_adjoint_plan* plan, const double* d_table, double* d_grad, void* stream);
+int ob_adjoint_node_vegas(ob_adjoint_plan* plan, const ob_adjoint_nodes* nodes, void* stream);
 int ob_adjoint_result_get(ob_adjoint_plan* plan, ob_adjoint_result* res, long long* batch_pairs);
 int ob_adjoint_plan_destroy(ob_adjoint_plan* plan);
 

@@ -223,6 +223,11 @@ class ObAdjointRequest(C.Structure):
     _fields_ = [("base", ObMcRequest), ("smoothing", C.c_double), ("checkpoint", C.c_int)]
 
 
+class ObAdjointNodes(C.Structure):
+    _fields_ = [(k, C.c_void_p) for k in ("base", "grad", "onehot", "phi", "psi", "work", "out")] + [
+        (k, C.c_int) for k in ("n_names", "n_e", "n_k")]
+
+
 class ObAdjointResult(C.Structure):
     _fields_ = [
         ("price", C.c_double),
@@ -382,6 +387,7 @@ SIGNATURES = {
     "ob_mc_plan_destroy": (C.c_int, [C.c_void_p]),
     "ob_adjoint_plan_create": (C.c_int, [C.POINTER(ObAdjointRequest), C.c_int, C.POINTER(C.c_void_p)]),
     "ob_adjoint_run": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "ob_adjoint_node_vegas": (C.c_int, [C.c_void_p, C.POINTER(ObAdjointNodes), C.c_void_p]),
     "ob_adjoint_result_get": (C.c_int, [C.c_void_p, C.POINTER(ObAdjointResult), C.POINTER(C.c_longlong)]),
     "ob_adjoint_plan_destroy": (C.c_int, [C.c_void_p]),
     "ob_batch_create": (C.c_int, [C.POINTER(ObBatchRequest), C.c_int, C.POINTER(C.c_void_p)]),

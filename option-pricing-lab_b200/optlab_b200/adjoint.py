@@ -19,7 +19,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
-from ._abi import OB_ADJ_BATCHES, ObAdjointRequest, ObAdjointResult, check, load
+from ._abi import OB_ADJ_BATCHES, ObAdjointNodes, ObAdjointRequest, ObAdjointResult, check, load
 from .engine import precision_code
 
 
@@ -47,6 +47,11 @@ class AdjointPlan:
     def run(self, table: torch.Tensor | None = None, grad: bool = True, stream=None) -> ObAdjointResult:
         """One forward pass (and the backward pass with grad). table: CUDA (n_rows, n_x) local variance replacing the
         current one, or None. The result holds the price, its SE and the deltas."""
+        g, _table = self._launch(table, grad, stream)  # (held until the passes have read it)
+        return self._finish(g)
+
+    def _launch(self, table, grad, stream=None):
+        """The passes queued on the stream; the batches' gradients (None without grad) and the table they read."""
         lib = load()
         dev = torch.device("cuda", torch.cuda.current_device())
         t = None
@@ -64,13 +69,18 @@ class AdjointPlan:
                 C.c_void_p(st.cuda_stream),
             )
         )
+        return g, t
+
+    def _finish(self, g) -> ObAdjointResult:
+        """Waits for the passes; the result, and the gradients as attributes."""
+        lib = load()
         res = ObAdjointResult()
         bp = (C.c_longlong * OB_ADJ_BATCHES)()
         check(lib.ob_adjoint_result_get(self._p, C.byref(res), bp))
         self.last = res
         if g is not None:
             self.batch_grad = g
-            self.batch_pairs = torch.tensor(list(bp), dtype=torch.float64, device=dev)
+            self.batch_pairs = torch.tensor(list(bp), dtype=torch.float64, device=g.device)
             self.gradient = g.sum(0) / self.n_pairs
         return res
 
@@ -174,34 +184,75 @@ class VegaNodes:
         return torch.einsum("rn,re,brk->bnek", self.onehot, self.phi, per_row)
 
 
+def _node_kernels_take(nodes, plan, dev) -> bool:
+    """Whether the node kernels (ob_adjoint_node_vegas) read these nodes: VegaNodes as it builds itself, on the plan's
+    rows and the current device. Anything else (a subclass with its own table, tensors elsewhere or of another type, no
+    autograd) goes through torch."""
+    if type(nodes) is not VegaNodes or type(plan) is not AdjointPlan or not torch.is_grad_enabled():
+        return False
+    want = {"onehot": (plan.n_rows, nodes.shape[0]), "phi": (plan.n_rows, nodes.shape[1]),
+            "psi": (plan.n_rows, plan.n_x, nodes.shape[2])}
+    for k, shape in want.items():
+        t = getattr(nodes, k)
+        if t.device != dev or t.dtype != torch.float64 or tuple(t.shape) != shape or not t.is_contiguous() or t.requires_grad:
+            return False
+    return min(nodes.shape) > 0
+
+
+def _node_greeks(plan, nodes, table, dev):
+    """The passes on the table and the node kernels behind them on the same stream: (result, vegas, standard errors).
+    The table goes through its root, as VegaNodes.table's does at zero bumps."""
+    base = torch.tensor(table, dtype=torch.float64, device=dev)
+    n, e, k = nodes.shape
+    work = torch.empty(plan.n_rows * k * OB_ADJ_BATCHES, dtype=torch.float64, device=dev)
+    out = torch.empty((2, n, e, k), dtype=torch.float64, device=dev)
+    g, _ = plan._launch(torch.sqrt(base) ** 2, True)
+    q = ObAdjointNodes(base.data_ptr(), g.data_ptr(), nodes.onehot.data_ptr(), nodes.phi.data_ptr(),
+                       nodes.psi.data_ptr(), work.data_ptr(), out.data_ptr(), n, e, k)
+    check(load().ob_adjoint_node_vegas(plan._p, C.byref(q), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    res = plan._finish(g)
+    out = out.cpu().numpy()
+    return res, out[0], out[1]
+
+
+def _torch_greeks(plan, nodes, table, dev):
+    """(result, vegas, standard errors) through torch autograd."""
+    base = torch.tensor(table, dtype=torch.float64, device=dev)
+    bumps = torch.zeros(nodes.shape, dtype=torch.float64, device=dev, requires_grad=True)
+    price = AutocallPrice.apply(nodes.table(base, bumps), plan)
+    (vega,) = torch.autograd.grad(price, bumps)
+    res = plan.last
+    # batch means: each batch's vegas from its own gradient, all batches in one contraction
+    pairs = plan.batch_pairs
+    vb = nodes.contract_batches(plan.batch_grad / pairs.clamp(min=1.0)[:, None, None], base)
+    w = pairs / pairs.sum()
+    mean = (w[:, None, None, None] * vb).sum(0)
+    var = (w[:, None, None, None] * (vb - mean) ** 2).sum(0) * (len(pairs) / (len(pairs) - 1)) / len(pairs)
+    return res, vega.cpu().numpy(), torch.sqrt(var).cpu().numpy()
+
+
 def autocall_greeks(held, nodes: VegaNodes, smoothing: float = 0.005, precision="fp32", plan: AdjointPlan | None = None):
     """Price, deltas and node vegas (each with its standard error) of a local-vol autocall, by one forward and one
-    backward pass; the vegas go through torch autograd (AutocallPrice of VegaNodes.table)."""
+    backward pass. The vegas of a VegaNodes come from the node kernels; any other parameterisation of the table goes
+    through torch autograd (AutocallPrice of its table)."""
     own = plan is None
     plan = plan or AdjointPlan(held, smoothing, precision)
     try:
         s = held.struct
         dev = torch.device("cuda", torch.cuda.current_device())
         table = np.ctypeslib.as_array(s.table, shape=(s.n_rows * s.n_x,)).reshape(s.n_rows, s.n_x)
-        base = torch.tensor(table, dtype=torch.float64, device=dev)
-        bumps = torch.zeros(nodes.shape, dtype=torch.float64, device=dev, requires_grad=True)
-        price = AutocallPrice.apply(nodes.table(base, bumps), plan)
-        (vega,) = torch.autograd.grad(price, bumps)
-        res = plan.last
-        # batch means: each batch's vegas from its own gradient, all batches in one contraction
-        pairs = plan.batch_pairs
-        vb = nodes.contract_batches(plan.batch_grad / pairs.clamp(min=1.0)[:, None, None], base)
-        w = pairs / pairs.sum()
-        mean = (w[:, None, None, None] * vb).sum(0)
-        var = (w[:, None, None, None] * (vb - mean) ** 2).sum(0) * (len(pairs) / (len(pairs) - 1)) / len(pairs)
+        if _node_kernels_take(nodes, plan, dev) and table.shape == (plan.n_rows, plan.n_x):
+            res, vega, vega_se = _node_greeks(plan, nodes, table, dev)
+        else:
+            res, vega, vega_se = _torch_greeks(plan, nodes, table, dev)
         n = s.n_names
         return {
             "price": res.price,
             "price_se": res.price_se,
             "delta": np.array(res.delta[:n]),
             "delta_se": np.array(res.delta_se[:n]),
-            "vega": vega.cpu().numpy(),
-            "vega_se": torch.sqrt(var).cpu().numpy(),
+            "vega": vega,
+            "vega_se": vega_se,
             "forward_ms": res.forward_ms,
             "backward_ms": res.backward_ms,
         }
