@@ -19,12 +19,13 @@ inline int table_pitch(int n_x) {
 }
 
 // The ring for batches of G steps of n names beside `used` bytes of shared memory within `budget`: up to 16 steps a
-// stage; false when not even one batch a stage fits.
+// stage; false when not even one batch a stage fits, or for rows of a single word (2^32 / chunks must fit 32 bits).
 template <typename R>
 inline bool plan_row_stream(RowStreamArgs& rs, int n_x, int n, int G, size_t used, size_t budget) {
     rs.pitch = table_pitch<R>(n_x);
     const size_t row = static_cast<size_t>(rs.pitch) * sizeof(Pair2<R>);
     rs.chunks = static_cast<int>(row / 16);
+    if (rs.chunks < 2) return false;
     rs.inv = static_cast<unsigned>(((1ull << 32) + rs.chunks - 1) / rs.chunks);
     rs.off = static_cast<int>((used + 15) & ~static_cast<size_t>(15));
     for (rs.batches = std::max(1, 16 / G); rs.batches >= 1; --rs.batches) {

@@ -99,3 +99,17 @@ def test_a_streamed_script_equals_its_pair_values_in_pieces(n_pairs, window):
     part, w = values(SMALL, 0)
     assert np.array_equal(v[:SMALL], w)
     assert abs(whole.price / v.mean() - 1) < 1e-12
+
+
+@pytest.mark.parametrize("n_x", [2, 3, 4, 5])
+def test_short_rows_of_a_large_table_equal_those_of_a_staged_one(n_x):
+    # 20000 rows of one to four intervals do not fit the stage; the rows the steps read alone do
+    steps, n_pairs, spare = 40, 30001, 20000
+    args = _model(1, steps, n_x, n_pairs)
+    kw = dict(obs_step=[steps // 2, steps], heston=[0.0, 1, 1, 0, 0], same=1, fwd=np.full((1, 2), 100.0))
+    large = dict(args, step_row=args["step_row"] + spare, lo=np.full(spare + steps, -0.8),
+                 inv_dx=np.full(spare + steps, (n_x - 1) / 1.6),
+                 table=np.vstack([np.full((spare, n_x), 0.5), args["table"]]))
+    staged, streamed = paths_request(**args, **kw), paths_request(**large, **kw)
+    engine.paths(staged, "fp32"), engine.paths(streamed, "fp32")
+    assert np.array_equal(_out(staged), _out(streamed))
