@@ -400,9 +400,17 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
                 R z[4];
                 box_muller64(t, c[0], c[1], z[0], z[1]);
                 box_muller64(t, c[2], c[3], z[2], z[3]);
+                // the legs' tails add up to one: a lane takes those of its own block's two steps, of |z|, and swaps them
+                const double t0 = tail64(t, fabs(z[0])), t1 = tail64(t, fabs(z[2]));
+                const double o0 = __shfl_xor_sync(kFull, t0, 1), o1 = __shfl_xor_sync(kFull, t1, 1);
+                tail[0] = odd ? o0 : t0, tail[1] = odd ? o1 : t1;
+                tail[2] = odd ? t0 : o0, tail[3] = odd ? t1 : o1;
                 swap(z, e);
 #pragma unroll
-                for (int g = 0; g < 4; ++g) e[2 * g] *= sgn, e[2 * g + 1] *= sgn, tail[g] = tail64(t, e[2 * g]);
+                for (int g = 0; g < 4; ++g) {
+                    e[2 * g] *= sgn, e[2 * g + 1] *= sgn;
+                    tail[g] = e[2 * g] < 0.0 ? 1.0 - tail[g] : tail[g];
+                }
             };
             draw(0);
             int i = 1, m = 0;

@@ -20,9 +20,11 @@
 // Taylor sums; Phi(-z) is a Taylor sum of degree 11 about the nearest sixteenth (its derivatives are Hermite
 // polynomials times the density). All are within about an ulp (the tables in 80-bit arithmetic on the host).
 //
-// Measured (a 252-step ladder): 650 -> 270 warp instructions a step and leg (132 FP64); 2^16 paths 0.40 -> 0.28 ms of
-// kernel (FP64 pipe 48 % busy, 3.5 warps a scheduler: latency), 2^12 paths a call 323 -> 195 us; prices within 1e-14
-// of plain 64-bit arithmetic before and after.
+// Measured (a 252-step ladder): 650 -> 270 warp instructions a step and leg (132 FP64); 2^16 paths 0.40 -> 0.24 ms of
+// kernel, 2^12 paths a call 323 -> 183 us; prices within 1e-14 of plain 64-bit arithmetic before and after. Of the 2^16
+// paths' gain the last 37 us (306 -> 270 a call) came from the tails: taken once a pair (a leg's tail is one minus the
+// other's) from a table whose couples of coefficients lie cell by cell, they cost 26 shared-memory wavefronts a step and
+// warp where they took 79, more than a third of the SM's time at 14 warps.
 #pragma once
 
 #include <cmath>
@@ -31,11 +33,14 @@
 
 namespace ob {
 
-constexpr int kTailHalf = 109, kTailCells = 2 * kTailHalf + 1, kTailTerms = 12;  // |z| <= 6.77 for 32-bit uniforms
+constexpr int kTailCells = 110, kTailTerms = 12;  // |z| <= 6.77 for 32-bit uniforms
 constexpr int kLogCells = 128, kTurnCells = 256;
 
 struct alignas(16) Qe64Tables {
-    double tail[kTailCells][kTailTerms];  // Taylor coefficients of Phi(-z) about (cell - kTailHalf) / 16
+    // Taylor coefficients of Phi(-z) about cell / 16, two of a cell side by side and the cells of a couple in a row: the
+    // lanes' cells spread over all the banks (12 in a row a cell, 96 bytes, they meet in half of them: 13.2 wavefronts a
+    // 16-byte load of 32 lanes instead of 8.7)
+    double tail[kTailTerms / 2][kTailCells][2];
     double log[kLogCells][2];             // 1 / c and ln c, c in the interval of the mantissa's leading bits
     double turn[kTurnCells][2];           // cos and sin of 2 pi k / 256
 };
@@ -46,13 +51,13 @@ inline const Qe64Tables& qe64_tables() {
         auto* t = new Qe64Tables();
         const long double pi = 3.14159265358979323846264338327950288L;
         for (int k = 0; k < kTailCells; ++k) {
-            const long double c = static_cast<long double>(k - kTailHalf) / 16;
+            const long double c = static_cast<long double>(k) / 16;
             const long double density = std::exp(-c * c / 2) / std::sqrt(2 * pi);
-            t->tail[k][0] = static_cast<double>(std::erfc(c / std::sqrt(2.0L)) / 2);
+            t->tail[0][k][0] = static_cast<double>(std::erfc(c / std::sqrt(2.0L)) / 2);
             long double he0 = 1, he1 = c, sign = -1, fact = 1;  // He_0, He_1; d^n Phi(-z) = -(-1)^(n-1) He_(n-1) density
             for (int n = 1; n < kTailTerms; ++n) {
                 fact *= n;
-                t->tail[k][n] = static_cast<double>(sign * he0 * density / fact);
+                t->tail[n / 2][k][n % 2] = static_cast<double>(sign * he0 * density / fact);
                 const long double next = c * he1 - n * he0;
                 he0 = he1, he1 = next, sign = -sign;
             }
@@ -114,16 +119,18 @@ __device__ __forceinline__ double log1p64_small(double x) {
     const double low = fma(x2, b, a), mid = fma(x2, d, c), top = fma(x2, f, e);
     return fma(x2, fma(x4, fma(x4, top, mid), low), x);
 }
-__device__ __forceinline__ double tail64(const Qe64Tables& t, double z) {  // Phi(-z), |z| < 6.84
+__device__ __forceinline__ double tail64(const Qe64Tables& t, double z) {  // Phi(-z), 0 <= z < 6.84
     constexpr double kMagic = 6755399441055744.0;                            // 1.5 2^52: rounds to an integer
     const double w = fma(z, 16.0, kMagic);
-    const double* c = t.tail[__double2loint(w) + kTailHalf];
+    const int cell = __double2loint(w);
     const double d = fma(w - kMagic, -0.0625, z);
-    const double2* c2 = reinterpret_cast<const double2*>(c);
-    double2 k = c2[kTailTerms / 2 - 1];
+    double2 k = *reinterpret_cast<const double2*>(t.tail[kTailTerms / 2 - 1][cell]);
     double s = fma(k.y, d, k.x);
 #pragma unroll
-    for (int n = kTailTerms / 2 - 2; n >= 0; --n) k = c2[n], s = fma(fma(s, d, k.y), d, k.x);
+    for (int n = kTailTerms / 2 - 2; n >= 0; --n) {
+        k = *reinterpret_cast<const double2*>(t.tail[n][cell]);
+        s = fma(fma(s, d, k.y), d, k.x);
+    }
     return s;
 }
 // Box-Muller on two 32-bit draws (common.cuh's, in these functions).
