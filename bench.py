@@ -44,27 +44,27 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "sm_max_mhz": 1965.0
 # Executed warp instructions per path-step of the dominant kernel, measured by ncu (smsp__inst_executed.sum of one
 # launch divided by its path-steps) and recorded under profiles/. The issue roofline below multiplies it by the live
 # path-step rate. A launch's instruction count does not depend on timing, so a profiled launch gives it exactly.
-INST_PER_PATH_STEP = {"lv_phoenix": 1.0527, "heston_qe": 20.30, "script": 1.518,
-                      # the 11 class kernels of one revaluation of the 32-trade book: 326.2 G over 2.49e11 path-steps
-                      "batch": 1.310,
+INST_PER_PATH_STEP = {"lv_phoenix": 0.8648, "heston_qe": 8.344, "script": 1.356,
+                      # the 11 class kernels of one revaluation of the 32-trade book: 281.1 G over 2.49e11 path-steps
+                      "batch": 1.129,
                       # the drop-in path engine's local-vol kernel on the Phoenix model (12 columns + a daily window)
-                      "paths": 2.354}
+                      "paths": 2.283}
 # The ALGORITHM's lane instructions per path-step of the local-vol Phoenix (one name, both legs of a pair share each
 # normal), counted from the algorithm, not from the compiled code, so that extra instructions lower the fraction:
 #   Philox4x32-10, one call per 4 normals = 4 pair-steps = 8 path-steps: 10 rounds x (2 wide multiplies, 2 three-way
 #     xors, 2 key additions) + 4 to set the counter = 64, so 8 per path-step;
 #   Box-Muller, per 2 normals = 4 path-steps: 2 conversions and 2 multiply-adds to (0, 1), a logarithm (10 with its
 #     range reduction), a square root (2), sin and cos of 2 pi v (10), 2 products = 28, so 7 per path-step;
-#   the local-vol step, per path-step: the table coordinate (1 multiply-add), its integer part and back (2), the
-#     weight (1), the index clamp (2), the address (1), one 8-byte shared load of the interval (1), the interpolation
-#     (1 multiply-add); variance x dt (1), its square root (2), the drift and the diffusion (2 multiply-adds); the
-#     knock-in's running minimum (1): 14.
-# 29 lane instructions = 0.906 warp instructions per path-step. The observations (12 over 756 steps) add < 1 %.
-ALG_INST_PER_PATH_STEP = {"lv_phoenix": (8 + 7 + 14) / 32.0}
+#   the local-vol step, per path-step, the multiply-adds of a pair's two legs packed in one instruction where they can be:
+#     the table coordinate clamped by saturation (1), its integer part, back and the weight (3 packed: 1.5), the address
+#     (1), one 8-byte shared load of the interval (1), the interpolation (1 multiply-add), the variance's square root (2),
+#     the drift and the diffusion (2 packed: 1), the knock-in's running minimum (three inputs, two steps: 0.5): 9.
+# 24 lane instructions = 0.75 warp instructions per path-step. The observations (12 over 756 steps) add < 1 %.
+ALG_INST_PER_PATH_STEP = {"lv_phoenix": (8 + 7 + 9) / 32.0}
 
 # Warp instructions of one leverage calibration at 2^18 particles x 504 steps: one lev_persistent launch
 # (ncu smsp__inst_executed.sum).
-LEV_INST_PER_CALIBRATION = 2.2436e9
+LEV_INST_PER_CALIBRATION = 2.0013e9
 # One grid barrier of 148 blocks (arrival counter with a release, acquiring polls), measured alone on a B200: 1.27 us.
 # A leverage step needs three (the particles' range, the step's bins, the leverage row): 3.81 us a step is the floor
 # of any calibration that keeps this dependency structure.
@@ -974,9 +974,9 @@ def ctypes_sizeof_trade() -> int:
 def run_paths(args, world, rank):
     """The drop-in path engine (the reference's `run()`, `ob_paths`): the local-vol Phoenix's model, 2^20 paths x 756
     steps, its 12 quarterly spot columns and one daily window (lowest and highest spot) written for every path and
-    copied back to the host (2^20 x 14 doubles = 117 MB). `value`: path-steps per second of the kernel, timed by CUDA
-    events inside the engine (inputs on the device); `e2e`: the whole call from host arrays (upload, kernel, the
-    columns back), by the host clock. One rank: the call is one job."""
+    brought back to the host (2^20 x 14 doubles = 117 MB, half of that over the link as floats). `value`: path-steps per
+    second of the kernel, timed by CUDA events inside the engine (inputs on the device); `e2e`: the whole call from host
+    arrays (upload, kernel, the columns back), by the host clock. One rank: the call is one job."""
     import torch
 
     from optlab_b200 import engine
@@ -999,6 +999,7 @@ def run_paths(args, world, rank):
             kern.append(k_ms)
     t_k = statistics.median(kern) / 1e3
     out_bytes = 2 * s.n_pairs * s.n_names * s.n_cols * 8
+    link_bytes = out_bytes // 2  # the columns cross as the paths' floats and are widened on the host
     in_bytes = input_bytes(rq) - out_bytes
     cpu = None
     if not args.no_cpu_baseline and args.model == "lv":
@@ -1031,7 +1032,7 @@ def run_paths(args, world, rank):
                                    "instructions per path-step x live rate"),
         "cpu_baseline": cpu,
         "e2e": {"value": units / statistics.median(wall), "unit": "path-steps/s", "h2d_bytes_per_step": int(in_bytes),
-                "d2h_bytes_per_step": int(out_bytes)},
+                "d2h_bytes_per_step": int(link_bytes)},
         # outputs of 32 MB or more run in four chunks of pairs, one launch each
         "gpu_launches": args.steps * (4 if out_bytes >= 32 << 20 and s.n_pairs >= 4 else 1),
         "clocks": {"sm_mhz": clk["sm_mhz"], "sm_max_mhz": clk["sm_max_mhz"], "reasons": clk["reasons"]},
