@@ -171,11 +171,11 @@ void release_streams() {
     k.s.clear();
 }
 
-void upload_bytes(void* dst, const void* src, size_t n) {
+void upload_bytes(void* dst, const void* src, size_t n, cudaStream_t st) {
     const bool staged = staged_upload(static_cast<char*>(dst), n, [&](char* out, size_t at, size_t count) {
         std::memcpy(out, static_cast<const char*>(src) + at, count);
     });
-    if (!staged) check_cuda(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice), "cudaMemcpy (inputs)");
+    if (!staged) check_cuda(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync (inputs)");
 }
 
 namespace {

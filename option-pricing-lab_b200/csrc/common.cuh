@@ -100,10 +100,13 @@ constexpr int kKeptStreams = 3;
 cudaStream_t kept_stream(int which);
 void release_streams();  // (ob_release_buffers)
 
-// n bytes of pageable host memory to dst on the device; the copy has finished when it returns. From kStagedUpload the
-// bytes go through the pinned staging, spread over the host threads (staged_upload in host_copy.cuh).
+// n bytes of pageable host memory to dst on the device, ordered before the work queued on st from then on; src is free
+// when it returns. From kStagedUpload the bytes go through the pinned staging, spread over the host threads
+// (staged_upload in host_copy.cuh), and the copy has finished when it returns. Smaller ones are one pageable copy on st,
+// which returns once the source is staged: the bytes may still be on their way then, and a kernel on another
+// non-blocking stream does not wait for them.
 constexpr size_t kStagedUpload = size_t(512) << 10;
-void upload_bytes(void* dst, const void* src, size_t n);
+void upload_bytes(void* dst, const void* src, size_t n, cudaStream_t st);
 
 // Device buffers that finished calls handed back, for the next call of the process: a one-shot call's cudaMalloc and
 // cudaFree (a few hundred microseconds together, and cudaFree waits for the whole device) become a lookup. At most
@@ -243,7 +246,8 @@ struct DeviceArena {
 // A call's inputs gathered into one host buffer and copied to the device in one transfer by commit(): a call with
 // many small inputs pays one copy's driver work instead of one for each (a few microseconds apiece). add() converts
 // to T as DeviceArena::put does (null or empty gives a null pointer) and names the pointer that receives the device
-// address; the pointers hold their addresses once commit() has returned.
+// address; the pointers hold their addresses once commit() has returned, and the inputs are there for the work queued on
+// its stream from then on (upload_bytes).
 class Upload {
   public:
     template <typename T, typename S, typename P>
@@ -269,10 +273,10 @@ class Upload {
         bytes_.resize(off + count * sizeof(T), 0);
         fixes_.push_back({off, [&field](unsigned char* base) { field = reinterpret_cast<P*>(base); }});
     }
-    void commit(DeviceArena& arena) {
+    void commit(DeviceArena& arena, cudaStream_t st = nullptr) {
         if (bytes_.empty()) return;
         unsigned char* d = arena.alloc<unsigned char>(bytes_.size());
-        upload_bytes(d, bytes_.data(), bytes_.size());
+        upload_bytes(d, bytes_.data(), bytes_.size(), st);
         for (const Fix& f : fixes_) f.set(d + f.off);
     }
 

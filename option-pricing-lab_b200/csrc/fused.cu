@@ -799,7 +799,7 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
                      ? kTabStreamed
                      : kTabGlobal;
             if (tm == kTabStreamed) block = 1024, end = a.rs.off + row_stream_bytes(a.rs, n, G);
-            a.tab = upload_table<R>(plan.arena, rq.table, rq.n_rows, rq.n_x);
+            a.tab = upload_table<R>(plan.arena, rq.table, rq.n_rows, rq.n_x, nullptr);
         } else {
             a.off.table2 = blob.put<Pair2<R>>(nullptr, cells);
             pack_table<R>(rq.table, rq.n_x, rq.n_x - 1, 0, cells,

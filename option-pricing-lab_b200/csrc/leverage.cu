@@ -897,8 +897,9 @@ void run_leverage(ob_leverage_request& rq) {
     for (int i = 0; i < S; ++i)
         bw[i] = rq.bandwidth_scale * rq.atm_vol * std::sqrt(std::max(rq.t0[i], 0.15)) * std::pow(n_particles, -0.2);
     const size_t rows_n = static_cast<size_t>(S) * rq.n_lv;
+    const cudaStream_t st = kept_stream(0);
     double* rows = arena.alloc<double>(rows_n);
-    upload_bytes(rows, rq.lv_rows, rows_n * sizeof(double));
+    upload_bytes(rows, rq.lv_rows, rows_n * sizeof(double), st);
     d.lv_rows = rows;
     Upload up;  // the small inputs in one copy
     up.add<double>(d.dt, rq.dt, S);
@@ -906,8 +907,7 @@ void run_leverage(ob_leverage_request& rq) {
     up.add<double>(d.lv_lo, rq.lv_lo, S);
     up.add<double>(d.lv_inv_dx, rq.lv_inv_dx, S);
     up.add<double>(d.bw, bw.data(), S);
-    up.commit(arena);
-    const cudaStream_t st = kept_stream(0);
+    up.commit(arena, st);
     const int nb = rq.n_bins, nf = rq.n_fine, ll = rq.local_linear;
     d.nfp = (nf + kFinePad - 1) / kFinePad * kFinePad;
     d.nbq = (nb + 1 + 3) / 4 * 4;

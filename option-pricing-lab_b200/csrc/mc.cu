@@ -516,6 +516,8 @@ int ob_mc_plan_create(const ob_mc_request* rq, int precision, ob_mc_plan** plan)
         ob_mc_plan* p = new ob_mc_plan();
         try {
             p->impl.create(*rq, precision);
+            // the inputs' pageable copies may still be on their way: a plan may run on any stream
+            ob::check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize (inputs)");
         } catch (...) {
             delete p;
             throw;

@@ -448,7 +448,7 @@ bool pack_paths_staged(const ob_paths_request& h, long long chunk, int sms, Devi
             a.tm = kTabStreamed;
             a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
         }
-        a.tab = upload_table<R>(arena, h.table, h.n_rows, h.n_x);
+        a.tab = upload_table<R>(arena, h.table, h.n_rows, h.n_x, nullptr);
     } else if (cells) {
         a.off.table2 = put(nullptr, cells * sizeof(Pair2<R>));
         pack_table<R>(h.table, h.n_x, h.n_x - 1, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));
@@ -460,7 +460,7 @@ bool pack_paths_staged(const ob_paths_request& h, long long chunk, int sms, Devi
     }
     a.smem_blob = static_cast<int>(blob.size());
     if (a.tm != kTabStreamed) a.smem = a.smem_blob;
-    a.blob = arena.put<unsigned char>(blob.data(), blob.size());
+    a.blob = arena.put<unsigned char>(blob.data(), blob.size());  // (waits for the stream, so for the table's copy too)
     a.n_steps = S, a.n_obs = h.n_obs, a.n_cols = h.n_cols, a.n_keep = h.n_keep, a.n_win = h.n_windows;
     for (int w = 0; w < 2; ++w) {
         a.win_lo[w] = w < h.n_windows ? h.win_lo[w] : 0;
@@ -582,6 +582,7 @@ void run_paths(ob_paths_request& h) {
         up.add<int>(s.win_hi, h.win_hi, h.n_windows);
         up.add<R>(s.fwd, h.fwd, static_cast<size_t>(n) * h.n_obs);
         up.commit(arena);
+        check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize (inputs)");  // (the kernels run on streams of their own)
     }
 
     R* stage[2] = {nullptr, nullptr};  // the chunks' columns on the host

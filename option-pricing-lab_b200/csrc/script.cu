@@ -743,7 +743,7 @@ bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, int sm
             a.tm = kTabStreamed;
             a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
         }
-        a.tab = upload_table<R>(arena, q.table, q.n_rows, q.n_x);
+        a.tab = upload_table<R>(arena, q.table, q.n_rows, q.n_x, nullptr);
     } else {
         a.off.table2 = put(nullptr, cells * sizeof(Pair2<R>));
         pack_table<R>(q.table, q.n_x, q.n_x - 1, 0, cells, reinterpret_cast<Pair2<R>*>(blob.data() + a.off.table2));

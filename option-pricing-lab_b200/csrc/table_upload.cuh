@@ -25,9 +25,9 @@ inline void pack_table(const double* table, int n_x, int pitch, size_t first, si
     }
 }
 
-// The table in global memory, its rows table_pitch cells apart.
+// The table in global memory, its rows table_pitch cells apart, there for the work queued on st from then on.
 template <typename R>
-inline Pair2<R>* upload_table(DeviceArena& arena, const double* table, int n_rows, int n_x) {
+inline Pair2<R>* upload_table(DeviceArena& arena, const double* table, int n_rows, int n_x, cudaStream_t st) {
     const int pitch = table_pitch<R>(n_x);
     const size_t cells = static_cast<size_t>(n_rows) * static_cast<size_t>(pitch);
     Pair2<R>* d = arena.alloc<Pair2<R>>(cells);
@@ -39,7 +39,7 @@ inline Pair2<R>* upload_table(DeviceArena& arena, const double* table, int n_row
     if (!staged) {
         std::vector<Pair2<R>> tab(cells);
         pack_table<R>(table, n_x, pitch, 0, cells, tab.data());
-        check_cuda(cudaMemcpy(d, tab.data(), cells * sizeof(Pair2<R>), cudaMemcpyHostToDevice), "cudaMemcpy (table)");
+        upload_bytes(d, tab.data(), cells * sizeof(Pair2<R>), st);
     }
     return d;
 }
