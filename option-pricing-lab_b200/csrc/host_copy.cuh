@@ -88,15 +88,17 @@ class PinnedStage {
         std::lock_guard<std::mutex> lock(m_);
         const size_t want = need <= kSmallBytes ? kSmallBytes : kSlotBytes;
         if (need > kSlotBytes) return false;
-        if (size_ < want && !failed_) {
-            if (base_) cudaFreeHost(base_);
-            base_ = nullptr, size_ = want;
-            if (cudaHostAlloc(&base_, 2 * want, cudaHostAllocPortable) != cudaSuccess) {
+        if (size_ < want && want < refused_) {
+            void* more = nullptr;
+            if (cudaHostAlloc(&more, 2 * want, cudaHostAllocPortable) == cudaSuccess) {
+                if (base_) cudaFreeHost(base_);
+                base_ = more, size_ = want;
+            } else {
                 cudaGetLastError();
-                base_ = nullptr, size_ = 0, failed_ = true;
+                refused_ = want;  // a smaller pair, held or not, still serves
             }
         }
-        if (!base_ || size_ < want) return false;
+        if (size_ < want) return false;
         out[0] = static_cast<char*>(base_), out[1] = static_cast<char*>(base_) + size_;
         return true;
     }
@@ -104,14 +106,14 @@ class PinnedStage {
         std::lock_guard<std::mutex> lock(m_);
         if (base_) cudaFreeHost(base_);
         cudaGetLastError();
-        base_ = nullptr, size_ = 0, failed_ = false;
+        base_ = nullptr, size_ = 0, refused_ = ~size_t(0);
     }
 
   private:
     std::mutex m_;
     void* base_ = nullptr;
     size_t size_ = 0;
-    bool failed_ = false;
+    size_t refused_ = ~size_t(0);  // the smallest slots that could not be had
 };
 
 // Host threads for the copies out of the staging: the hardware threads less one, at most seven, started at the first

@@ -120,3 +120,34 @@ from optlab_b200.batch import Batch, sample_book
 Batch(sample_book(n_trades=4, seed=1, paths_log2=(8, 9), years=(1, 2)), "fp32")
 assert fake.fake_outstanding() == 0
 """)
+
+
+SMALL, LARGE = 2 * 4 * 2**20, 2 * 32 * 2**20  # bytes of the two pairs of pinned slots
+
+
+def test_a_pair_of_slots_that_cannot_grow_keeps_serving(on_the_stand_in):
+    # a 1.3 MB table goes through the small pair; the columns of 2^23 pairs ask for the large one
+    on_the_stand_in(f"""
+table = dict(steps=40, n_x=4001, n_obs=1)
+fake.fake_host_limit({SMALL})
+columns(**table)
+assert fake.fake_pinned_bytes() == {SMALL}
+columns(n_pairs=2**23, n_obs=1)
+columns(**table)
+assert fake.fake_pinned_bytes() == {SMALL}
+fake.fake_host_limit({LARGE})
+check(lib.ob_release_buffers())
+columns(**table)
+columns(n_pairs=2**23, n_obs=1)
+assert fake.fake_pinned_bytes() == {LARGE}
+""")
+
+
+def test_small_requests_after_a_refused_large_one_get_their_slots(on_the_stand_in):
+    on_the_stand_in(f"""
+fake.fake_host_limit({SMALL})
+columns(n_pairs=2**23, n_obs=1)
+assert fake.fake_pinned_bytes() == 0
+columns(steps=40, n_x=4001, n_obs=1)
+assert fake.fake_pinned_bytes() == {SMALL}
+""")
