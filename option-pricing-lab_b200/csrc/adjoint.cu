@@ -68,7 +68,8 @@ struct AdjArgs {
     unsigned char* ki_name;    // 2 x n_pairs
     double* partial;           // per block: price sum and square, then per name delta sum and square
     double* grad;              // kAdjBatches x n_rows x n_x
-    int n_copies;              // dense backward: copies of the gradient in priv, copy k for batch k % kAdjBatches
+    int n_copies;              // dense backward: copies of the gradient in priv, copy k for batch k % kAdjBatches;
+    int group;                 // groups of 2^group chunks of 32 pairs take them in turn
     R* priv;                   // per copy (recomputing backward: per block): (left, right) weights of each table interval, n_rows x (n_x - 1)
                                // pairs, zeroed before each backward
     unsigned long long* batch_pairs;  // kAdjBatches
@@ -516,11 +517,12 @@ __device__ __forceinline__ void dense_segment(const AdjArgs<R>& a, long long p, 
 // One leg a warp: warps 2k and 2k + 1 of a block take the two legs of the same 32 pairs. Half the state of a pair a
 // thread, so more warps fit an SM to hide the states' loads; 128-thread blocks, each walking couples of chunks (64
 // pairs). Groups of 128 pairs take the gradient copies in turn, whatever block walks them, so the batches that give the
-// vegas' errors depend on the pair alone. BLOCKS an SM in float: six (80 registers), or seven (72) for a launch that
+// vegas' errors depend on the pair alone; below 4096 pairs, where that leaves batches empty, groups of 64 or 32 pairs as
+// far as those fill them (AdjPlan::build). BLOCKS an SM in float: six (80 registers), or seven (72) for a launch that
 // then ends in one round (AdjPlan::build). 3 names x 1008 steps: 2^16 pairs, 1.15 rounds at six, 1.76 -> 1.25 ms at seven;
 // 2^18 pairs, where the reductions' rate at L2 bounds the sweep, 4.60 ms at six and 4.84 at seven. Four names take five
 // (their states would spill).
-// Copies of the dense backward's gradient: one for each group of 128 pairs up to this many an SM (in float all of them
+// Copies of the dense backward's gradient: one for each group of pairs up to this many an SM (in float all of them
 // together stay in L2 for the benchmark's tables).
 template <typename R>
 constexpr int copies_per_sm(int n) {
@@ -535,7 +537,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 4 ? (N == 4 ? 5 : BLOCKS) : 
     const long long n_couples = (P + 63) / 64;
     for (long long couple = blockIdx.x; couple < n_couples; couple += gridDim.x) {
         const long long p = (2 * couple + (warp >> 1)) * 32 + lane;
-        const int copy = static_cast<int>((couple >> 1) % a.n_copies);
+        const int copy = static_cast<int>((p >> (5 + a.group)) % a.n_copies);
         if (leg == 0) {
             const unsigned walked = __ballot_sync(0xffffffffu, p < P);
             if (lane == 0 && walked)
@@ -654,7 +656,7 @@ __global__ void __launch_bounds__(256) adj_node_rows(const double* __restrict__ 
 }
 
 // One warp a node: blockIdx.x = name * n_e + expiry, a warp of the block each strike. out: vegas, then their standard
-// errors (batch means weighted by the batches' pairs), n_names x n_e x n_k each.
+// errors (batch means weighted by the batches' pairs; zero from a single batch), n_names x n_e x n_k each.
 __global__ void __launch_bounds__(256) adj_node_sum(const double* __restrict__ h, const double* __restrict__ onehot,
                                                     const double* __restrict__ phi,
                                                     const unsigned long long* __restrict__ batch_pairs, double n_pairs,
@@ -677,7 +679,9 @@ __global__ void __launch_bounds__(256) adj_node_sum(const double* __restrict__ h
     const double pairs = static_cast<double>(batch_pairs[lane]);
     const double w = pairs / all(pairs), mean_b = c / fmax(pairs, 1.0);
     const double mean = all(w * mean_b), d = mean_b - mean;
-    const double var = all(w * (d * d)) * (kAdjBatches / (kAdjBatches - 1.0)) / kAdjBatches;
+    // the batches with pairs count: k means, each weighted by its pairs, estimate their mean's variance by sum w d^2 / (k - 1)
+    const int filled = __popc(__ballot_sync(0xffffffffu, pairs > 0.0));
+    const double var = all(w * (d * d)) / max(filled - 1, 1);
     const double total = all(c);
     if (lane == 0) {
         const long long at = static_cast<long long>(blockIdx.x) * n_k + k;
@@ -858,8 +862,10 @@ void AdjPlan::build(const ob_adjoint_request& r) {
     const long long pairs_b = dense ? block_b / 2 : block_b;  // the dense backward takes one leg a thread
     grid_b = static_cast<int>(std::max<long long>(
         1, std::min<long long>((P + pairs_b - 1) / pairs_b, static_cast<long long>(sms) * std::max(1, per_b))));
-    a.n_copies = dense ? static_cast<int>(std::min<long long>((P + 127) / 128, static_cast<long long>(sms) * copies_per_sm<R>(n)))
-                       : grid_b;
+    // the largest groups of 128, 64 or 32 pairs that fill every batch; of 128 where none does
+    a.group = P >= 4096 || P < 1024 ? 2 : P >= 2048 ? 1 : 0;
+    const long long groups = (P + (32LL << a.group) - 1) >> (5 + a.group);
+    a.n_copies = dense ? static_cast<int>(std::min<long long>(groups, static_cast<long long>(sms) * copies_per_sm<R>(n))) : grid_b;
     a.partial = arena.alloc<double>(static_cast<size_t>(grid_f) * (2 + 2 * n));
     const size_t cells2 = 2 * static_cast<size_t>(rq.n_rows) * (rq.n_x - 1);
     priv_bytes = static_cast<size_t>(a.n_copies) * cells2 * sizeof(R);

@@ -222,12 +222,13 @@ def _torch_greeks(plan, nodes, table, dev):
     price = AutocallPrice.apply(nodes.table(base, bumps), plan)
     (vega,) = torch.autograd.grad(price, bumps)
     res = plan.last
-    # batch means: each batch's vegas from its own gradient, all batches in one contraction
+    # batch means: each batch's vegas from its own gradient, all batches in one contraction; k batches with pairs,
+    # weighted by them, estimate their mean's variance by sum w d^2 / (k - 1) (zero from a single one)
     pairs = plan.batch_pairs
     vb = nodes.contract_batches(plan.batch_grad / pairs.clamp(min=1.0)[:, None, None], base)
     w = pairs / pairs.sum()
     mean = (w[:, None, None, None] * vb).sum(0)
-    var = (w[:, None, None, None] * (vb - mean) ** 2).sum(0) * (len(pairs) / (len(pairs) - 1)) / len(pairs)
+    var = (w[:, None, None, None] * (vb - mean) ** 2).sum(0) / (pairs > 0).sum().sub(1).clamp(min=1)
     return res, vega.cpu().numpy(), torch.sqrt(var).cpu().numpy()
 
 
