@@ -783,22 +783,15 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
         a.ln_ki = rq.ki_barrier > 0 ? static_cast<R>(std::log(rq.ki_barrier)) : R(-1e30);
         a.coupon = rq.coupon, a.put_strike = rq.put_strike, a.memory = rq.memory, a.ki_daily = rq.ki_daily;
     }
-    int block = 512;
+    const int block = 512;
     auto acc_bytes = [&](int b) { return static_cast<size_t>(b / 32) * 2 * a.n_out * sizeof(double); };
     const size_t budget = sizeof(R) == 4 ? (110u << 10) : (220u << 10);  // two blocks a SM in float, one in double
     auto aligned = [&] { return (blob.bytes.size() + 15) & ~static_cast<size_t>(15); };
     int tm = kTabStaged;
-    size_t end = 0;  // of the blob and the ring
     if (table) {
         const size_t cells = static_cast<size_t>(rq.n_rows) * (rq.n_x - 1);
         if (aligned() + cells * sizeof(Pair2<R>) + acc_bytes(block) > budget) {
-            constexpr size_t kStreamBudget = 220u << 10;  // one block an SM
-            const int G = batch_steps(n, kind, false);
-            tm = pick(kTabStreamed) && streams_rows(rq.n_pairs, plan.sms, 12.0) &&
-                         plan_row_stream<R>(a.rs, rq.n_x, n, G, aligned(), kStreamBudget - acc_bytes(1024))
-                     ? kTabStreamed
-                     : kTabGlobal;
-            if (tm == kTabStreamed) block = 1024, end = a.rs.off + row_stream_bytes(a.rs, n, G);
+            tm = kTabGlobal;
             a.tab = upload_table<R>(plan.arena, rq.table, rq.n_rows, rq.n_x, nullptr);
         } else {
             a.off.table2 = blob.put<Pair2<R>>(nullptr, cells);
@@ -809,23 +802,32 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
         for (size_t k = 0; k < static_cast<size_t>(S) * n; ++k)
             ns[k].row *= tm == kTabStaged ? rq.n_x - 1 : table_pitch<R>(rq.n_x);
     }
-    const FusedFn<R> fn = pick(tm);
-    a.smem_blob = static_cast<int>(aligned());
-    if (static_cast<size_t>(a.smem_blob) + acc_bytes(512) > budget) return false;
-    a.smem_acc = static_cast<int>(std::max(aligned(), end));
+    a.smem_blob = a.smem_acc = static_cast<int>(aligned());
     const size_t smem = a.smem_acc + acc_bytes(block);
+    if (smem > budget) return false;
     unsigned char* d = plan.arena.alloc<unsigned char>(std::max<size_t>(16, blob.bytes.size()));
     check_cuda(cudaMemcpy(d, blob.bytes.data(), blob.bytes.size(), cudaMemcpyHostToDevice), "copy blob");
     a.blob = d;
-    const void* k = reinterpret_cast<const void*>(fn);
+    const void* k = reinterpret_cast<const void*>(pick(tm));
     allow_smem(k, smem);
     if (occupancy(k, block, smem) < 1) return false;
-    if (tm != kTabStreamed) {
-        plan.n_names = n;
-        plan.kernel_legs = reinterpret_cast<const void*>(rq.product == OB_PRODUCT_LADDER
-                                                             ? pick_legs<R, OB_PRODUCT_LADDER>(kind, n, tm, rq.mixer != 0)
-                                                             : pick_legs<R, OB_PRODUCT_AUTOCALL>(kind, n, tm, rq.mixer != 0));
-        if (plan.kernel_legs) allow_smem(plan.kernel_legs, smem);
+    plan.n_names = n;
+    // beside the kernel for many pairs those for fewer (McPlan::run chooses by each run's count)
+    plan.kernel_legs = reinterpret_cast<const void*>(rq.product == OB_PRODUCT_LADDER
+                                                         ? pick_legs<R, OB_PRODUCT_LADDER>(kind, n, tm, rq.mixer != 0)
+                                                         : pick_legs<R, OB_PRODUCT_AUTOCALL>(kind, n, tm, rq.mixer != 0));
+    if (plan.kernel_legs) allow_smem(plan.kernel_legs, smem);
+    if (tm == kTabGlobal && pick(kTabStreamed)) {
+        constexpr size_t kStreamBudget = 220u << 10;  // one block an SM
+        const size_t acc = acc_bytes(kStreamedBlock);
+        const int G = batch_steps(n, kind, false);
+        if (plan_row_stream<R>(a.rs, rq.n_x, n, G, aligned(), kStreamBudget - acc)) {
+            plan.kernel_rows = reinterpret_cast<const void*>(pick(kTabStreamed));
+            plan.acc_rows = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
+            plan.smem_rows = plan.acc_rows + acc;
+            allow_smem(plan.kernel_rows, plan.smem_rows);
+            if (occupancy(plan.kernel_rows, kStreamedBlock, plan.smem_rows) < 1) plan.kernel_rows = nullptr;
+        }
     }
     plan.fused = true;
     plan.threads_per_pair = kind == 4 ? 2 : 1;
@@ -844,6 +846,9 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
 bool fused_legs_apart(int n, long long n_pairs, int sms) {
     return static_cast<double>(n_pairs) / (32.0 * sms) < (n == 1 ? 5.5 : 7.5);
 }
+
+// Whether a run of n_pairs streams its rows where the plan has that kernel (streams_rows has the times).
+bool fused_streams_rows(long long n_pairs, int sms) { return streams_rows(n_pairs, sms, 12.0); }
 
 template bool fused_build<float>(McPlan&, const ob_mc_request&);
 template bool fused_build<double>(McPlan&, const ob_mc_request&);

@@ -445,25 +445,29 @@ McPlan::~McPlan() {
 
 void McPlan::run(long long n_pairs, long long first_pair, unsigned long long seed, cudaStream_t st) {
     if (n_pairs < 1 || first_pair < 0) invalid("n_pairs must be >= 1 and first_pair >= 0");
-    const bool apart = kernel_legs && fused_legs_apart(n_names, n_pairs, sms);
-    const LaunchShape shape = launch_shape(apart ? kernel_legs : kernel, smem_bytes, sms,
-                                           n_pairs * (apart ? 2 : threads_per_pair), block);
+    // the kernel by this run's pairs, whatever count the plan was made for
+    const bool rows = kernel_rows && fused_streams_rows(n_pairs, sms);
+    const bool apart = !rows && kernel_legs && fused_legs_apart(n_names, n_pairs, sms);
+    void* fn = const_cast<void*>(rows ? kernel_rows : apart ? kernel_legs : kernel);
+    const size_t smem = rows ? smem_rows : smem_bytes;
+    const LaunchShape shape = launch_shape(fn, smem, sms, n_pairs * (apart ? 2 : threads_per_pair),
+                                           rows ? kStreamedBlock : block);
     const int grid = std::min(shape.grid, max_blocks), blk = shape.block;
     const uint32_t k0 = static_cast<uint32_t>(seed), k1 = static_cast<uint32_t>(seed >> 32);
     if (!timing) check_cuda(cudaEventRecord(e0, st), "cudaEventRecord"), timing = true;
     using FusedF = void (*)(FusedArgs<float>, long long, long long, uint32_t, uint32_t, double*);
     using FusedD = void (*)(FusedArgs<double>, long long, long long, uint32_t, uint32_t, double*);
-    void* fn = const_cast<void*>(apart ? kernel_legs : kernel);
-    if (fused && precision == OB_FP32)
-        reinterpret_cast<FusedF>(fn)<<<grid, blk, smem_bytes, st>>>(fa_f, n_pairs, first_pair, k0, k1, d_partial);
-    else if (fused)
-        reinterpret_cast<FusedD>(fn)<<<grid, blk, smem_bytes, st>>>(fa_d, n_pairs, first_pair, k0, k1, d_partial);
-    else if (precision == OB_FP32)
-        reinterpret_cast<KernelFn<float>>(fn)<<<grid, blk, smem_bytes, st>>>(args_f, n_pairs, first_pair, k0, k1,
-                                                                              d_partial);
-    else
-        reinterpret_cast<KernelFn<double>>(fn)<<<grid, blk, smem_bytes, st>>>(args_d, n_pairs, first_pair, k0, k1,
-                                                                               d_partial);
+    if (fused && precision == OB_FP32) {
+        FusedArgs<float> fa = fa_f;
+        if (rows) fa.smem_acc = acc_rows;
+        reinterpret_cast<FusedF>(fn)<<<grid, blk, smem, st>>>(fa, n_pairs, first_pair, k0, k1, d_partial);
+    } else if (fused) {
+        reinterpret_cast<FusedD>(fn)<<<grid, blk, smem, st>>>(fa_d, n_pairs, first_pair, k0, k1, d_partial);
+    } else if (precision == OB_FP32) {
+        reinterpret_cast<KernelFn<float>>(fn)<<<grid, blk, smem, st>>>(args_f, n_pairs, first_pair, k0, k1, d_partial);
+    } else {
+        reinterpret_cast<KernelFn<double>>(fn)<<<grid, blk, smem, st>>>(args_d, n_pairs, first_pair, k0, k1, d_partial);
+    }
     check_cuda(cudaGetLastError(), "mc_kernel launch");
     mc_finalize<<<1, 1024, 0, st>>>(d_partial, grid, 2 * n_out, d_sums, pairs_run > 0);
     check_cuda(cudaGetLastError(), "mc_finalize launch");

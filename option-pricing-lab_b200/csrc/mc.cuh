@@ -44,6 +44,9 @@ struct McPlan {
     size_t smem_bytes = 0;
     const void* kernel = nullptr;
     const void* kernel_legs = nullptr;  // the fused kernel with a pair's legs on two lanes, for runs of few pairs
+    const void* kernel_rows = nullptr;  // the fused kernel that streams its table's rows, for mid-sized runs
+    size_t smem_rows = 0;               // its shared memory at kStreamedBlock threads,
+    int acc_rows = 0;                   // and where the warps' sums are in it
     McArgs<float> args_f{};
     McArgs<double> args_d{};
     double* d_partial = nullptr;
@@ -81,6 +84,8 @@ inline FusedArgs<double>& McPlan::fused_args<double>() {
 template <typename R>
 bool fused_build(McPlan& plan, const ob_mc_request& rq);
 bool fused_legs_apart(int n, long long n_pairs, int sms);  // whether such a run puts the legs apart
+bool fused_streams_rows(long long n_pairs, int sms);       // whether such a run streams its rows
+constexpr int kStreamedBlock = 1024;
 
 template <>
 inline McArgs<float>& McPlan::args<float>() {

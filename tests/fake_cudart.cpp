@@ -2,7 +2,7 @@
 // memory is host memory, kernels do nothing, and every upload or clearing of device memory counts as outstanding on its
 // stream until the host waits for that stream. A launch on a stream that is not ordered behind an outstanding one (a
 // non-blocking stream and any other) is recorded. A pageable cudaMemcpy counts as outstanding too: it may return once
-// the source has been staged.
+// the source has been staged. The first kernel launched since fake_forget() is kept, to tell the routes of calls apart.
 #include <cstddef>
 #include <cstdint>
 #include <cstdlib>
@@ -22,7 +22,8 @@ std::map<void*, Stream> g_streams;
 std::map<void*, size_t> g_pinned;
 std::string g_unordered;
 size_t g_host_limit = ~size_t(0);
-int g_launches = 0;
+int g_launches = 0, g_first_block = 0;
+const void* g_first_kernel = nullptr;
 struct Config {
     Dim3 grid, block;
     size_t smem;
@@ -48,8 +49,8 @@ bool pinned(const void* p) {
         if (p >= e.first && p < static_cast<char*>(e.first) + e.second) return true;
     return false;
 }
-int launch(void* s) {
-    ++g_launches;
+int launch(const void* kernel, Dim3 block, void* s) {
+    if (g_launches++ == 0) g_first_kernel = kernel, g_first_block = static_cast<int>(block.x);
     stream(s);
     for (const auto& e : g_streams) {
         if (e.first == s || e.second.outstanding == 0) continue;
@@ -66,6 +67,8 @@ int launch(void* s) {
 extern "C" {
 const char* fake_unordered() { return g_unordered.c_str(); }
 int fake_launches() { return g_launches; }
+const void* fake_first_kernel() { return g_first_kernel; }
+int fake_first_block() { return g_first_block; }
 void fake_forget() { g_unordered.clear(), g_launches = 0; }
 int fake_outstanding() {
     int n = 0;
@@ -142,9 +145,9 @@ int cudaEventElapsedTime(float* ms, void*, void*) { return *ms = 0.0f, 0; }
 
 int cudaFuncSetAttribute(const void*, int, int) { return 0; }
 int cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t) { return *n = 1, 0; }
-int cudaLaunchKernel(const void*, Dim3, Dim3, void**, size_t, void* s) { return launch(s); }
-int cudaLaunchCooperativeKernel(const void*, Dim3, Dim3, void**, size_t, void* s) { return launch(s); }
-int cudaLaunchKernelExC(const Config* c, const void*, void**) { return launch(c->stream); }
+int cudaLaunchKernel(const void* f, Dim3, Dim3 b, void**, size_t, void* s) { return launch(f, b, s); }
+int cudaLaunchCooperativeKernel(const void* f, Dim3, Dim3 b, void**, size_t, void* s) { return launch(f, b, s); }
+int cudaLaunchKernelExC(const Config* c, const void* f, void**) { return launch(f, c->block, c->stream); }
 
 unsigned __cudaPushCallConfiguration(Dim3 grid, Dim3 block, size_t smem, void* s) {
     return g_config = {grid, block, smem, s}, 0u;
