@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
     double* wacc = reinterpret_cast<double*>(sm + a.smem_acc);
     for (int t = threadIdx.x; t < n_warps * n_acc; t += blockDim.x) wacc[t] = 0.0;
     __syncthreads();
-    const StepRec<R>* s_step = reinterpret_cast<const StepRec<R>*>(sm + a.off.step);
+    const int* s_obs = reinterpret_cast<const int*>(sm + a.off.step);  // the observation at each step's end, or negative
     const R* s_trig = reinterpret_cast<const R*>(sm + a.off.ln_trig);
     const double* s_disc = reinterpret_cast<const double*>(sm + a.off.obs_disc);
     const int* leg_type = reinterpret_cast<const int*>(sm + a.off.leg_type);
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(512, min_blocks<R>())
                 l.hi = run_max(l.hi, lp), l.lo = run_min(l.lo, lp);
             } else {
                 l.lo = run_min(l.lo, lp);
-                const int j = s_step[i - 1].obs;
+                const int j = s_obs[i - 1];
                 if (j >= 0) leg_observe(a, s_trig, s_disc, l, lp, j);
             }
         };
@@ -718,7 +718,13 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
             else steps[i - 1].obs = i - next;
         }
     }
-    a.off.step = blob.put(steps);
+    if (kind == 4) {  // (its steps are all alike: the kernel reads an autocall's observations alone)
+        std::vector<int> obs(rq.product == OB_PRODUCT_AUTOCALL ? S : 0);
+        for (size_t i = 0; i < obs.size(); ++i) obs[i] = steps[i].obs;
+        a.off.step = blob.put(obs);
+    } else {
+        a.off.step = blob.put(steps);
+    }
     const bool table = kind == 1 || kind == 3;
     if (kind == 4) {
         a.qe = make_qe_consts<R>(rq.heston, rq.r, rq.q, rq.dt[0]);

@@ -264,7 +264,8 @@ struct RowStreamArgs {
 
 // Byte offsets inside the staged blob.
 struct FusedOffsets {
-    int step, name_step, root, hes, table2, ln_trig, obs_disc, leg_type, leg_strike, leg_barrier, ln_level;
+    int step,  // StepRec a step; Heston QE: the observation of each step alone (an autocall's)
+        name_step, root, hes, table2, ln_trig, obs_disc, leg_type, leg_strike, leg_barrier, ln_level;
     int mix_den, low_root;  // local correlation: per step sigma sqrt(max(t0, 1/12)); the aligned low root
     int qe_tables;          // Heston QE in double: Qe64Tables
 };

@@ -1,5 +1,5 @@
 """A pricing plan chooses its kernel by the pairs of each run, not by the count it was made for (a rank prices its share
-of a plan's pairs, a quote refines on the plan of an indication): on the stand-in for the CUDA runtime, without a GPU."""
+of a plan's pairs, a quote refines on the plan of an indication), and long schedules keep the specialised kernel: on the stand-in for the CUDA runtime, without a GPU."""
 
 import pytest
 from test_upload_order import on_the_stand_in  # noqa: F401 (the fixture)
@@ -38,4 +38,29 @@ assert len(set(k for k, _ in own)) == {routes}, own
 for made_for in counts:
     p = plan(made_for)
     assert [route(p, c) for c in counts] == own, made_for
+""")
+
+
+@pytest.mark.parametrize("ladder", [False, True], ids=["autocall", "ladder"])
+def test_a_heston_qe_request_of_thousands_of_steps_keeps_its_kernel(on_the_stand_in, ladder):  # noqa: F811
+    # (27 years of daily steps: a double record of 32 bytes a step beside the step's tables passed the 220 KB stage)
+    on_the_stand_in(f"""
+from optlab_b200._abi import OB_MODEL_HESTON_QE
+from optlab_b200.requests import mc_request
+ladder = {ladder}
+fake.fake_first_kernel.restype = C.c_void_p
+
+def kernel(steps, precision):
+    product = dict(product=0, leg_type=[1], leg_strike=[100.0], leg_barrier=[0], leg_level=[0.0], discount=1.0) if ladder \\
+        else dict(product=1, obs_step=[steps], obs_discount=[1.0], trigger=[0.0], ki_barrier=0.6, put_strike=1.0)
+    held = mc_request(model=OB_MODEL_HESTON_QE, dt=np.full(steps, 1 / 252), t0=np.arange(steps) / 252, spot=[100.0],
+                      n_pairs=64, seed=1, heston=(0.04, 1.5, 0.04, 0.5, -0.7), r=0.02, q=0.0, **product)
+    p = C.c_void_p()
+    check(lib.ob_mc_plan_create(C.byref(held.struct), precision, C.byref(p)))
+    fake.fake_forget()
+    check(lib.ob_mc_run(p, C.c_longlong(64), C.c_longlong(0), C.c_ulonglong(1), None))
+    return fake.fake_first_kernel()
+
+for precision in (0, 1):
+    assert len(set(kernel(steps, precision) for steps in (252, 6300, 6500, 6804))) == 1
 """)
