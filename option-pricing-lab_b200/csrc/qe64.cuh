@@ -15,16 +15,19 @@
 // 2^12-path ladder is less than a warp an SM.
 //
 // Functions: reciprocals and roots start from the hardware approximations (rcp and rsqrt.approx.ftz.f64) and take one
-// third-order step of the binomial series; the logarithm is table-driven (Tang, ACM TOMS 16, 1990): 128 intervals,
-// ln x = k ln 2 - ln(1/c) + ln(1 + r); the angle's cosine and sine rotate a table of 256 directions by the remainder's
-// Taylor sums; Phi(-z) is a Taylor sum of degree 11 about the nearest sixteenth (its derivatives are Hermite
-// polynomials times the density). All are within about an ulp (the tables in 80-bit arithmetic on the host).
+// third-order step of the binomial series; the logarithm takes x = 2^k z with z in [3/4, 3/2), the tabulated reciprocal
+// c of the nearest of 129 centres, and ln x = k ln 2 - ln c + ln(1 + r) with r = c z - 1 by one multiply-add (the
+// reduction of Story and Tang, New algorithms for improved transcendental functions on IA-64, ARITH 14, 1999); the
+// angle's cosine and sine rotate a table of 256 directions by the remainder's Taylor sums; Phi(-z) is a Taylor sum of
+// degree 11 about the nearest sixteenth (its derivatives are Hermite polynomials times the density). All are within about
+// an ulp (the tables in 80-bit arithmetic on the host).
 //
 // Measured (a 252-step ladder): 650 -> 270 warp instructions a step and leg (132 FP64); 2^16 paths 0.40 -> 0.24 ms of
-// kernel, 2^12 paths a call 323 -> 183 us; prices within 1e-14 of plain 64-bit arithmetic before and after. Of the 2^16
-// paths' gain the last 37 us (306 -> 270 a call) came from the tails: taken once a pair (a leg's tail is one minus the
-// other's) from a table whose couples of coefficients lie cell by cell, they cost 26 shared-memory wavefronts a step and
-// warp where they took 79, more than a third of the SM's time at 14 warps.
+// kernel, 2^12 paths a call 323 -> 183 us. Against 80-bit arithmetic, over 60 ladders of 2^11 to 2^17 paths and 12 to 504
+// steps, the prices are off by 1.1e-15 (rms), those of the textbook form by 2.4e-15. Of the 2^16 paths' gain the last 37 us
+// (306 -> 270 a call) came from the tails: taken once a pair (a leg's tail is one minus the other's) from a table whose
+// couples of coefficients lie cell by cell, they cost 26 shared-memory wavefronts a step and warp where they took 79, more
+// than a third of the SM's time at 14 warps.
 #pragma once
 
 #include <cmath>
@@ -34,14 +37,14 @@
 namespace ob {
 
 constexpr int kTailCells = 110, kTailTerms = 12;  // |z| <= 6.77 for 32-bit uniforms
-constexpr int kLogCells = 128, kTurnCells = 256;
+constexpr int kLogCells = 129, kTurnCells = 256;
 
 struct alignas(16) Qe64Tables {
     // Taylor coefficients of Phi(-z) about cell / 16, two of a cell side by side and the cells of a couple in a row: the
     // lanes' cells spread over all the banks (12 in a row a cell, 96 bytes, they meet in half of them: 13.2 wavefronts a
     // 16-byte load of 32 lanes instead of 8.7)
     double tail[kTailTerms / 2][kTailCells][2];
-    double log[kLogCells][2];             // 1 / c and ln c, c in the interval of the mantissa's leading bits
+    double log[kLogCells][2];             // c and -ln c at the centres: seven fractional bits of a binade, 3/4 to 3/2
     double turn[kTurnCells][2];           // cos and sin of 2 pi k / 256
 };
 
@@ -63,15 +66,10 @@ inline const Qe64Tables& qe64_tables() {
             }
         }
         for (int j = 0; j < kLogCells; ++j) {
-            // the interval's mantissas: high words 0x3FE60000 + [j, j + 1) 2^13; those on both sides of 1 use c = 1
-            auto at = [](int jj) {
-                const long long bits = (0x3FE60000LL + (static_cast<long long>(jj) << 13)) << 32;
-                double d;
-                std::memcpy(&d, &bits, sizeof d);
-                return static_cast<long double>(d);
-            };
-            const double inv = j == 79 || j == 80 ? 1.0 : static_cast<double>(2 / (at(j) + at(j + 1)));
-            t->log[j][0] = inv, t->log[j][1] = static_cast<double>(-std::log(static_cast<long double>(inv)));
+            // c = 1 from 1 - 3/512, a cell below one's own: the sum would cancel there
+            const double centre = j < 64 ? (192 + j) / 256.0 : (64 + j) / 128.0;
+            const double c = j == 63 || j == 64 ? 1.0 : 1 / centre;
+            t->log[j][0] = c, t->log[j][1] = static_cast<double>(-std::log(static_cast<long double>(c)));
         }
         for (int k = 0; k < kTurnCells; ++k) {
             t->turn[k][0] = static_cast<double>(std::cos(2 * pi * k / kTurnCells));
@@ -98,18 +96,20 @@ __device__ __forceinline__ double sqrt64(double x, double& inv) {
     const double g = x * inv, e = fma(-g, inv, 1.0);  // sqrt(x) = g (1 - e)^(-1/2)
     return fma(g * e, fma(0.375, e, 0.5), g);
 }
-__device__ __forceinline__ double log64(const Qe64Tables& t, double x) {  // a normal x > 0
-    const int hi = __double2hiint(x), off = hi - 0x3FE60000, k = off >> 20;
-    const double z = __hiloint2double(hi - (k << 20), __double2loint(x));
-    const double2 c = *reinterpret_cast<const double2*>(t.log[(off >> 13) & (kLogCells - 1)]);
-    const double r = fma(z, c.x, -1.0);  // |r| < 2^-7
-    double s = fma(r, -1.0 / 8, 1.0 / 7);
-    s = fma(s, r, -1.0 / 6), s = fma(s, r, 1.0 / 5), s = fma(s, r, -1.0 / 4), s = fma(s, r, 1.0 / 3);
-    s = fma(s, r, -0.5);
-    const double kd = static_cast<double>(k);
-    // ln 2 as a sum, the first part exact times k
-    const double low = fma(kd, 5.497923018708371e-14, fma(r * r, s, r));
-    return fma(kd, 0.6931471805598903, c.y) + low;
+// 2^-127 < x < 1.5: within 2.2 2^-53 of ln x below one (the draws and the tails; 20 million of each).
+__device__ __forceinline__ double log64(const Qe64Tables& t, double x) {
+    const int hi = __double2hiint(x);
+    const int up = (hi + 0x80000) & 0x7FF00000;              // 2^k in place: a mantissa from 3/2 counts up
+    const int zh = hi - up + 0x3FF00000;                     // z, its high word
+    const int cell = (zh + 0x1000 - 0x3FE80000) >> 13;       // its nearest centre
+    const double2 c = *reinterpret_cast<const double2*>(t.log[cell]);
+    const double r = fma(__hiloint2double(zh, __double2loint(x)), c.x, -1.0);  // |r| < 1/160
+    double s = fma(r, 1.0 / 7, -1.0 / 6);
+    s = fma(s, r, 1.0 / 5), s = fma(s, r, -1.0 / 4), s = fma(s, r, 1.0 / 3), s = fma(s, r, -0.5);
+    const double kd = static_cast<double>((up >> 20) - 1023);
+    // ln 2 as a sum, the first part (46 bits) exact times k
+    const double low = fma(kd, -1.8641886737243033e-15, fma(r * r, s, r));
+    return fma(kd, 0.6931471805599472, c.y) + low;
 }
 // ln(1 + x), |x| <= 1/16.
 __device__ __forceinline__ double log1p64_small(double x) {
