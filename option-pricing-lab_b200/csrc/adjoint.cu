@@ -514,6 +514,13 @@ __device__ __forceinline__ void dense_segment(const AdjArgs<R>& a, long long p, 
     }
 }
 
+// Copies of the dense backward's gradient: one for each group of pairs up to this many an SM (in float all of them
+// together stay in L2 for the benchmark's tables).
+template <typename R>
+constexpr int copies_per_sm(int n) {
+    return sizeof(R) == 4 ? 3 : n <= 2 ? 2 : 1;
+}
+
 // One leg a warp: warps 2k and 2k + 1 of a block take the two legs of the same 32 pairs. Half the state of a pair a
 // thread, so more warps fit an SM to hide the states' loads; 128-thread blocks, each walking couples of chunks (64
 // pairs). Groups of 128 pairs take the gradient copies in turn, whatever block walks them, so the batches that give the
@@ -522,15 +529,8 @@ __device__ __forceinline__ void dense_segment(const AdjArgs<R>& a, long long p, 
 // then ends in one round (AdjPlan::build). 3 names x 1008 steps: 2^16 pairs, 1.15 rounds at six, 1.76 -> 1.25 ms at seven;
 // 2^18 pairs, where the reductions' rate at L2 bounds the sweep, 4.60 ms at six and 4.84 at seven. Four names take five
 // (their states would spill).
-// Copies of the dense backward's gradient: one for each group of pairs up to this many an SM (in float all of them
-// together stay in L2 for the benchmark's tables).
-template <typename R>
-constexpr int copies_per_sm(int n) {
-    return sizeof(R) == 4 ? 3 : n <= 2 ? 2 : 1;
-}
-
 template <typename R, int N, int BLOCKS>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? (N == 4 ? 5 : BLOCKS) : 2) adj_backward_dense(AdjArgs<R> a) {
+__global__ void __launch_bounds__(128, BLOCKS) adj_backward_dense(AdjArgs<R> a) {
     const Pair2<R>* tab = a.table;  // (staging it in shared memory measured no faster: the state loads bound it)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, leg = warp & 1;
     const long long P = a.n_pairs;
@@ -743,9 +743,11 @@ void pick_st(AdjPlan& p) {
     p.kf = reinterpret_cast<const void*>(adj_forward<R, N, false, kCk, ST>);
     p.kfs = p.dense ? reinterpret_cast<const void*>(adj_forward<R, N, true, 1, ST>)
                     : reinterpret_cast<const void*>(adj_forward<R, N, true, kCk, ST>);
-    p.kb = !p.dense        ? reinterpret_cast<const void*>(adj_backward<R, N>)
-           : p.seven ? reinterpret_cast<const void*>(adj_backward_dense<R, N, 7>)
-                     : reinterpret_cast<const void*>(adj_backward_dense<R, N, 6>);
+    constexpr int kBlocks = sizeof(R) == 8 ? 2 : N == 4 ? 5 : 6;
+    p.kb = reinterpret_cast<const void*>(adj_backward_dense<R, N, kBlocks>);
+    if constexpr (sizeof(R) == 4 && N <= 3)
+        if (p.seven) p.kb = reinterpret_cast<const void*>(adj_backward_dense<R, N, 7>);
+    if (!p.dense) p.kb = reinterpret_cast<const void*>(adj_backward<R, N>);
 }
 
 // Staged tables for float only (double tables of the benchmark's size do not fit a block's shared memory).

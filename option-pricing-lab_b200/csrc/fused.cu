@@ -130,12 +130,12 @@ __global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM == kTabStr
     const Pair2<R>* s_tab = TM == kTabStaged ? reinterpret_cast<const Pair2<R>*>(sm + a.off.table2) : a.tab;
     const uint32_t tab_s = TM == kTabStreamed ? static_cast<uint32_t>(a.rs.off)
                                               : shared_address<TABLE && TM == kTabStaged>(s_tab);
-    RowStream<R, N, G> rows(a.rs, a.tab, s_ns, sm, a.n_steps);
+    RowStream<R, G> rows(a.rs, a.tab, s_ns, sm, a.n_steps);
     if (TM == kTabStreamed) rows.first();
     const R* s_trig = reinterpret_cast<const R*>(sm + a.off.ln_trig);
     const double* s_disc = reinterpret_cast<const double*>(sm + a.off.obs_disc);
     const int S = a.n_steps;
-    // the correlation root: in registers for one or two names, read from shared memory for more (registers spill)
+    // the correlation root: in registers for up to three names, read from shared memory for more (registers spill)
     constexpr bool kRootRegs = N <= 3;
     R rt[kRootRegs ? N * N : 1];
 #pragma unroll
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM == kTabStr
                         if (VAR) vp0 = m_max(v0[n], R(0)), vp1 = m_max(v1[n], R(0));
                         if (TABLE) {
                             R t0, t1;
-                            table_vars<TM>(s_tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i, n) : ns.row,
+                            table_vars<TM>(s_tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i) : ns.row,
                                            a.top, x0[n], x1[n], t0, t1);
                             var0 = KIND == 1 ? t0 : t0 * vp0, var1 = KIND == 1 ? t1 : t1 * vp1;
                         } else if (VAR) {
@@ -827,9 +827,9 @@ bool fused_build(McPlan& plan, const ob_mc_request& rq) {
         constexpr size_t kStreamBudget = 220u << 10;  // one block an SM
         const size_t acc = acc_bytes(kStreamedBlock);
         const int G = batch_steps(n, kind, false);
-        if (plan_row_stream<R>(a.rs, rq.n_x, n, G, aligned(), kStreamBudget - acc)) {
+        if (plan_row_stream<R>(a.rs, rq.n_x, G, aligned(), kStreamBudget - acc)) {
             plan.kernel_rows = reinterpret_cast<const void*>(pick(kTabStreamed));
-            plan.acc_rows = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
+            plan.acc_rows = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, G));
             plan.smem_rows = plan.acc_rows + acc;
             allow_smem(plan.kernel_rows, plan.smem_rows);
             if (occupancy(plan.kernel_rows, kStreamedBlock, plan.smem_rows) < 1) plan.kernel_rows = nullptr;

@@ -203,13 +203,12 @@ __device__ __forceinline__ void table_vars(const Pair2<float>* tab, const unsign
     var0 = fmaf(f0, y0.b, y0.a), var1 = fmaf(f1, y1.b, y1.a);
 }
 template <int MODE>
-__device__ __forceinline__ void table_vars(const Pair2<double>* tab, const unsigned char* sm, uint32_t tab_s,
-                                           double org, double inv, int row, double top, double x0, double x1,
+__device__ __forceinline__ void table_vars(const Pair2<double>* tab, const unsigned char*, uint32_t, double org, double inv, int row, double top, double x0, double x1,
                                            double& var0, double& var1) {
+    static_assert(MODE != kTabStreamed, "rows are streamed in float");
     int j0, j1;
     double f0, f1;
     table_cell(org, inv, top, x0, j0, f0), table_cell(org, inv, top, x1, j1, f1);
-    if (MODE == kTabStreamed) tab = reinterpret_cast<const Pair2<double>*>(sm + tab_s);
     const Pair2<double> y0 = MODE == kTabGlobal ? ldg_pair(tab + row + j0) : tab[row + j0];
     const Pair2<double> y1 = MODE == kTabGlobal ? ldg_pair(tab + row + j1) : tab[row + j1];
     var0 = y0.a + f0 * y0.b, var1 = y1.a + f1 * y1.b;

@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(lv_block<N, TM>(), TM != kTabStreamed && N == 
     const Pair2<R>* tab = TM == kTabStaged ? reinterpret_cast<const Pair2<R>*>(sm + a.off.table2) : a.tab;
     const uint32_t tab_s = TM == kTabStreamed ? static_cast<uint32_t>(a.rs.off)
                                               : shared_address<TABLE && TM == kTabStaged>(tab);
-    RowStream<R, N, G> rows(a.rs, a.tab, s_ns, sm, a.n_steps);
+    RowStream<R, G> rows(a.rs, a.tab, s_ns, sm, a.n_steps);
     if (TM == kTabStreamed) rows.first();
     const int2* s_sched = reinterpret_cast<const int2*>(sm + a.off.sched);  // observations [x, y) at each step end
     const int* s_col = reinterpret_cast<const int*>(sm + a.off.col);
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(lv_block<N, TM>(), TM != kTabStreamed && N == 
                     if (VAR) vp0 = m_max(v0[n], R(0)), vp1 = m_max(v1[n], R(0));
                     if (TABLE) {
                         R t0, t1;
-                        table_vars<TM>(tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i, n) : ns.row,
+                        table_vars<TM>(tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i) : ns.row,
                                        a.top, x0[n], x1[n], t0, t1);
                         var0 = KIND == 1 ? t0 : t0 * vp0, var1 = KIND == 1 ? t1 : t1 * vp1;
                     } else if (VAR) {
@@ -444,9 +444,9 @@ bool pack_paths_staged(const ob_paths_request& h, long long chunk, int sms, Devi
     if (a.tm == kTabGlobal) {
         const int G = paths_batch_steps(n, kind, false);
         if (streams_paths<R>(n, kind, h.mixer != 0) && streams_rows(chunk, sms, 20.0) &&
-            plan_row_stream<R>(a.rs, h.n_x, n, G, at, 220u << 10)) {
+            plan_row_stream<R>(a.rs, h.n_x, G, at, 220u << 10)) {
             a.tm = kTabStreamed;
-            a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
+            a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, G));
         }
         a.tab = upload_table<R>(arena, h.table, h.n_rows, h.n_x, nullptr);
     } else if (cells) {

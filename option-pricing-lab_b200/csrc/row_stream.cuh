@@ -18,10 +18,10 @@ inline int table_pitch(int n_x) {
     return (n_x - 1 + per - 1) / per * per;
 }
 
-// The ring for batches of G steps of n names beside `used` bytes of shared memory within `budget`: up to 16 steps a
+// The ring for batches of G steps of one name beside `used` bytes of shared memory within `budget`: up to 16 steps a
 // stage; false when not even one batch a stage fits, or for rows of a single word (2^32 / chunks must fit 32 bits).
 template <typename R>
-inline bool plan_row_stream(RowStreamArgs& rs, int n_x, int n, int G, size_t used, size_t budget) {
+inline bool plan_row_stream(RowStreamArgs& rs, int n_x, int G, size_t used, size_t budget) {
     rs.pitch = table_pitch<R>(n_x);
     const size_t row = static_cast<size_t>(rs.pitch) * sizeof(Pair2<R>);
     rs.chunks = static_cast<int>(row / 16);
@@ -29,14 +29,14 @@ inline bool plan_row_stream(RowStreamArgs& rs, int n_x, int n, int G, size_t use
     rs.inv = static_cast<unsigned>(((1ull << 32) + rs.chunks - 1) / rs.chunks);
     rs.off = static_cast<int>((used + 15) & ~static_cast<size_t>(15));
     for (rs.batches = std::max(1, 16 / G); rs.batches >= 1; --rs.batches) {
-        const size_t rows = static_cast<size_t>(rs.batches) * G * n;
+        const size_t rows = static_cast<size_t>(rs.batches) * G;
         const unsigned long long words = static_cast<unsigned long long>(rows) * rs.chunks;
         if (rs.off + 2 * rows * row <= budget && words * rs.chunks < (1ull << 32)) return true;
     }
     return false;
 }
-inline size_t row_stream_bytes(const RowStreamArgs& rs, int n, int G) {
-    return 2 * static_cast<size_t>(rs.batches) * G * n * rs.chunks * 16;
+inline size_t row_stream_bytes(const RowStreamArgs& rs, int G) {
+    return 2 * static_cast<size_t>(rs.batches) * G * rs.chunks * 16;
 }
 
 // Whether a launch of n_pairs streams its rows: from kFirst warps an SM, where a block's warps share each row's copy, to
@@ -51,9 +51,9 @@ inline bool streams_rows(long long n_pairs, int sms, double most) {
     return warps >= kFirst && warps < most;
 }
 
-// One block's ring. Every thread of the block makes the same calls in the same order: first() once, then turn() before
+// One block's ring of one name's rows. Every thread of the block makes the same calls in the same order: first() once, then turn() before
 // each batch that opens a stage (opens()).
-template <typename R, int N, int G>
+template <typename R, int G>
 struct RowStream {
     const RowStreamArgs& rs;
     const Pair2<R>* tab;
@@ -66,12 +66,12 @@ struct RowStream {
         : rs(r), tab(t), ns(s), sm(shared), steps(S), n_batches((S + G - 1) / G), cur(1), row0(0) {}
 
     __device__ __forceinline__ void issue(int batch, int half) {
-        const int s0 = batch * G, rows = min(rs.batches * G, steps - s0) * N, n = rows * rs.chunks;
+        const int s0 = batch * G, rows = min(rs.batches * G, steps - s0), n = rows * rs.chunks;
         const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(sm + rs.off)) +
-                             static_cast<uint32_t>(half * rs.batches * G * N * rs.chunks) * 16u;
+                             static_cast<uint32_t>(half * rs.batches * G * rs.chunks) * 16u;
         for (int c = threadIdx.x; c < n; c += blockDim.x) {
             const int row = static_cast<int>(__umulhi(static_cast<unsigned>(c), rs.inv));
-            const char* src = reinterpret_cast<const char*>(tab + ns[s0 * N + row].row) + (c - row * rs.chunks) * 16;
+            const char* src = reinterpret_cast<const char*>(tab + ns[s0 + row].row) + (c - row * rs.chunks) * 16;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + static_cast<uint32_t>(c) * 16u), "l"(src)
                          : "memory");
         }
@@ -87,10 +87,10 @@ struct RowStream {
         cur ^= 1;
         const int next = batch + rs.batches < n_batches ? batch + rs.batches : more ? 0 : -1;
         if (next >= 0) issue(next, cur ^ 1);
-        row0 = (cur * rs.batches * G - batch * G) * N * rs.pitch;
+        row0 = (cur * rs.batches * G - batch * G) * rs.pitch;
     }
-    // The cell of step i's (1-based) row of name n, from the start of the ring.
-    __device__ __forceinline__ int row(int i, int n) const { return row0 + ((i - 1) * N + n) * rs.pitch; }
+    // The cell of step i's (1-based) row, from the start of the ring.
+    __device__ __forceinline__ int row(int i) const { return row0 + (i - 1) * rs.pitch; }
 };
 
 }  // namespace ob

@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM != kTabStr
     const R* s_root = reinterpret_cast<const R*>(sm + a.off.root);
     const Pair2<R>* s_tab = TM == kTabStaged ? reinterpret_cast<const Pair2<R>*>(sm + a.off.table2) : a.tab;
     const uint32_t tab_s = TM == kTabStreamed ? static_cast<uint32_t>(a.rs.off) : shared_address<TM == kTabStaged>(s_tab);
-    RowStream<R, N, G> rows(a.rs, a.tab, s_ns, sm, d.n_steps);
+    RowStream<R, G> rows(a.rs, a.tab, s_ns, sm, d.n_steps);
     if (TM == kTabStreamed) rows.first();
     const int2* s_sched = reinterpret_cast<const int2*>(sm + a.off.sched);  // (event, window mask) per step end
     const R* s_lf0 = reinterpret_cast<const R*>(sm + a.off.lf0);
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(TM == kTabStreamed ? 1024 : 512, TM != kTabStr
                 for (int n = 0; n < N; ++n) {
                     const NameStep<R> ns = s_ns[(i - 1) * N + n];
                     R v0, v1;
-                    table_vars<TM>(s_tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i, n) : ns.row,
+                    table_vars<TM>(s_tab, sm, tab_s, ns.org, ns.inv_dx, TM == kTabStreamed ? rows.row(i) : ns.row,
                                    a.top, x0[n], x1[n], v0, v1);
                     // sqrt(dt) z with the legs' signs (+1, -1 but before a branch), the step's multiply-adds written
                     // out: the same arithmetic in every instantiation, so a branch at step 0 is an ordinary run bit
@@ -739,9 +739,9 @@ bool pack_lv(const ob_script_request& rq, const std::vector<int2>& sched, int sm
     if (a.tm == kTabGlobal) {
         constexpr int G = 8;  // (kLean)
         if (streams_script<R>(n, rq.n_windows) && streams_rows(q.n_pairs, sms, 20.0) &&
-            plan_row_stream<R>(a.rs, q.n_x, n, G, at, 220u << 10)) {
+            plan_row_stream<R>(a.rs, q.n_x, G, at, 220u << 10)) {
             a.tm = kTabStreamed;
-            a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, n, G));
+            a.smem = static_cast<int>(a.rs.off + row_stream_bytes(a.rs, G));
         }
         a.tab = upload_table<R>(arena, q.table, q.n_rows, q.n_x, nullptr);
     } else {
