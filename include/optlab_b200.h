@@ -95,7 +95,7 @@ typedef struct {
     const int* win_lo;
     const int* win_hi;
     double* out;
-    double kernel_ms, total_ms;
+    double kernel_ms, total_ms; /* kernel_ms: the kernels', the columns' way over the link to the host included */
 } ob_paths_request;
 
 /* Same layout as optlab_device (requests.hpp:66-71). */
@@ -391,9 +391,9 @@ int ob_cpu_threads(void);
 int ob_device_info(int device, ob_device* out);
 /* No counterpart in the reference (it allocates and frees per call). The one-shot calls (ob_price, ob_mc_price,
    ob_paths, ob_script_price, ob_leverage, ob_philox_normals) keep their device buffers for the next call, at most
-   512 MB over all devices, with 64 MB of pinned host memory (at most) through which large inputs and outputs pass (the result
-   reads 16 KB more) and up to three streams a device; this frees them and forgets the kernels' occupancy answers and shared-memory limits the
-   plans cached. Call it before cudaDeviceReset or before destroying a context the library has used: cached buffers
+   512 MB over all devices, with 64 MB of pinned host memory (at most; 72 while its small pair of slots gives way to the
+   large one) through which large inputs and outputs pass (the result reads 16 KB more) and up to three streams a device;
+   this frees them and forgets the kernels' occupancy answers and shared-memory limits the plans cached. Call it before cudaDeviceReset or before destroying a context the library has used: cached buffers
    and attributes belong to the context that made them. */
 int ob_release_buffers(void);
 
@@ -450,8 +450,8 @@ int ob_mc_plan_destroy(ob_mc_plan* plan);
    OB_ADJ_BATCHES x n_rows x n_x doubles) with each batch's sum over its pairs of d(pair value)/d(table entry);
    result waits, returns price and deltas with standard errors, and the pairs of each batch (batch_pairs may be
    NULL). Without d_grad, run is the smoothed revaluation of a bump-and-revalue. node_vegas, after a run with a gradient
-   and on that run's stream, writes the node vegas of tent bumps and their batch-mean standard
-   errors. */
+   and on that run's stream, writes the node vegas of tent bumps and their standard errors, from the means of the batches
+   that hold pairs (0 from a single batch: up to 128 pairs, 256 in the recomputing backward). */
 int ob_adjoint_plan_create(const ob_adjoint_request* rq, int precision, ob_adjoint_plan** plan);
 int ob_adjoint_run(ob_adjoint_plan* plan, const double* d_table, double* d_grad, void* stream);
 int ob_adjoint_node_vegas(ob_adjoint_plan* plan, const ob_adjoint_nodes* nodes, void* stream);

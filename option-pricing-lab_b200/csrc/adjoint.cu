@@ -526,9 +526,10 @@ constexpr int copies_per_sm(int n) {
 // pairs). Groups of 128 pairs take the gradient copies in turn, whatever block walks them, so the batches that give the
 // vegas' errors depend on the pair alone; below 4096 pairs, where that leaves batches empty, groups of 64 or 32 pairs as
 // far as those fill them (AdjPlan::build). BLOCKS an SM in float: six (80 registers), or seven (72) for a launch that
-// then ends in one round (AdjPlan::build). 3 names x 1008 steps: 2^16 pairs, 1.15 rounds at six, 1.76 -> 1.25 ms at seven;
-// 2^18 pairs, where the reductions' rate at L2 bounds the sweep, 4.60 ms at six and 4.84 at seven. Four names take five
-// (their states would spill).
+// then ends in one round (AdjPlan::build). 3 names x 1008 steps, six against seven: 2^16 pairs, 1.15 rounds at six, 1.76 /
+// 1.25 ms; 66400, two rounds of either, 1.74 / 1.86; 100000 1.89 / 1.95; 2^17, where seven ends in two rounds and six does
+// not, 2.71 / 2.63; 2^18, where the reductions' rate at L2 bounds the sweep, 4.64 / 5.02. Four names take five (their
+// states would spill).
 template <typename R, int N, int BLOCKS>
 __global__ void __launch_bounds__(128, BLOCKS) adj_backward_dense(AdjArgs<R> a) {
     const Pair2<R>* tab = a.table;  // (staging it in shared memory measured no faster: the state loads bound it)
